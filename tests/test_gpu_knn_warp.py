@@ -1,0 +1,86 @@
+"""The warp-per-query kNN kernel (sorted rows, k <= 128) against the oracle, at the edges of
+its register lists (k around 32, 64 and 128), its scan units and its dispatch.  Ids and FP64
+distances are compared for equality: both sides round every product and sum separately."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import make_points
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # name, n, d, periodic, leaf, nq, k
+    ("uniform3d", 5000, 3, False, 16, 7, 1),
+    ("uniform3d_odd", 5001, 3, False, 16, 65, 31),
+    ("periodic3d", 5000, 3, True, 16, 65, 32),
+    ("periodic_clustered", 5000, 3, True, 8, 65, 33),
+    ("clustered_dup", 8000, 3, False, 16, 129, 64),
+    ("clustered_dup", 8000, 3, False, 1, 129, 65),
+    ("lattice_periodic", 8000, 3, True, 16, 64, 127),
+    ("lattice", 8000, 3, False, 40, 64, 128),
+    ("uniform3d", 5000, 3, False, 16, 64, 129),   # past the kernel's k: the packet kernel
+    ("tiny", 3, 3, True, 16, 4, 5),               # fewer points than k
+    ("tiny", 90, 2, False, 4, 4, 100),
+    ("d1", 2000, 1, True, 16, 33, 20),
+    ("d2", 2000, 2, False, 3, 33, 50),
+    ("d4", 3000, 4, True, 16, 33, 16),
+    ("d5", 3000, 5, False, 16, 33, 40),
+    ("d6_clustered", 6000, 6, False, 32, 33, 100),
+    ("d7", 3000, 7, True, 200, 17, 24),           # leaves of many scan units
+    ("d8", 3000, 8, False, 16, 17, 70),
+]
+
+
+@pytest.mark.parametrize("order", [1, 2], ids=["leaf_order", "caller_order"])
+@pytest.mark.parametrize("name,n,d,periodic,leaf,nq,k", CASES)
+def test_gpu_knn_warp_matches_oracle(gpu, oracle, name, n, d, periodic, leaf, nq, k, order):
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    P = make_points(name, n, d, periodic)
+    rng = np.random.default_rng(17)
+    Q = np.concatenate([P[rng.integers(0, n, nq // 2)],
+                        rng.random((nq - nq // 2, d)) - (0.5 if periodic else 0.0)])
+    if not periodic:
+        Q[-1] += 3.0  # outside the points
+    box = 1.0 if periodic else None
+    t = gpu.kdtree.build_kdtree(P, leaf=leaf, boxsize=box)
+    od, oi = oracle.OracleTree(P, leaf, box).knn(Q, k)
+    _lib.check(L.ckd_set_tuning(6, order))
+    try:
+        gd, gi = gpu.kdtree.knn_search(t, Q, k)
+    finally:
+        _lib.check(L.ckd_set_tuning(6, 0))
+    np.testing.assert_array_equal(gi, oi)
+    np.testing.assert_array_equal(gd, od)
+
+
+@pytest.mark.parametrize("k", [1, 33, 64])
+def test_gpu_knn_warp_forest(gpu, oracle, k):
+    rng = np.random.default_rng(23)
+    parts = [rng.random((n, 3)) - 0.5 for n in (1, 16, 17, 700, 4000)]
+    qs = [rng.random((m, 3)) - 0.5 for m in (2, 1, 3, 40, 1)]
+    f = gpu.build_forest(parts, leaf=16, boxsize=1.0)
+    qoff = np.cumsum([0] + [len(q) for q in qs])
+    d, i = f.knn(np.concatenate(qs), qoff, k)
+    for t, (P, q) in enumerate(zip(parts, qs)):
+        od, oi = oracle.OracleTree(P, 16, [1.0, 1.0, 1.0]).knn(q, k)
+        np.testing.assert_array_equal(i[qoff[t]:qoff[t + 1]].cpu().numpy(), oi)
+        np.testing.assert_array_equal(d[qoff[t]:qoff[t + 1]].cpu().numpy(), od)
+
+
+@pytest.mark.parametrize("nq", [32768 + 2200 * 16, 32768 + 2200 * 16 + 1])
+def test_gpu_knn_warp_at_its_dispatch_line(gpu, nq):
+    """Both sides of the rule that chooses the kernel give the rows of the per-lane kernel."""
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(29)
+    t = gpu.kdtree.build_kdtree(rng.random((30011, 3)))
+    q = rng.random((nq, 3))
+    d, i = gpu.kdtree.knn_search(t, q, 16)
+    _lib.check(L.ckd_set_knn_variant(8))
+    try:
+        ld, li = gpu.kdtree.knn_search(t, q, 16)
+    finally:
+        _lib.check(L.ckd_set_knn_variant(0))
+    np.testing.assert_array_equal(i, li)
+    np.testing.assert_array_equal(d, ld)
