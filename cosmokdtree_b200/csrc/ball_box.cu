@@ -292,7 +292,7 @@ constexpr int kHeavyStack = 128;
 // full the warp copies the subtree itself (same output).
 constexpr int32_t kTaskMin = 1024;
 constexpr int32_t kTaskChunk = 4096;
-constexpr unsigned kTaskCap = 1u << 20;
+constexpr unsigned kTaskCap = 1u << 20;  // at most: 64 a query, at least 2^16
 struct EmitTask {
   int64_t out;  // first output slot
   int32_t start, count, qi, pad;
@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(128) k_ball_fill_warp(TreeView tv, const doubl
                                                         double* __restrict__ odist, int want_d2,
                                                         EmitTask* __restrict__ tasks,
                                                         unsigned* __restrict__ n_tasks,
+                                                        unsigned task_cap,
                                                         const int32_t* __restrict__ qroot) {
   __shared__ int32_t sstk[4][kHeavyStack];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(128) k_ball_fill_warp(TreeView tv, const doubl
         unsigned tb = 0;
         if (lane == 0) tb = atomicAdd(n_tasks, nt);
         tb = __shfl_sync(0xffffffffu, tb, 0);
-        if (tb + nt <= kTaskCap) {
+        if (tb + nt <= task_cap) {
           for (unsigned c = lane; c < nt; c += 32) {
             EmitTask e;
             e.out = cur + (int64_t)c * kTaskChunk;
@@ -352,6 +353,8 @@ __global__ void __launch_bounds__(128) k_ball_fill_warp(TreeView tv, const doubl
           cur += m.count;
           continue;
         }
+        // the buffer is full: the slots left in it hold no work
+        for (unsigned c = lane; c < nt && tb + c < task_cap; c += 32) tasks[tb + c] = EmitTask{};
       }
       if (inside) {  // whole subtree: positions m.start .. m.start + count - 1 in order
         for (int32_t i = lane; i < m.count; i += 32) {
@@ -401,10 +404,11 @@ template <int D, bool PER>
 __global__ void __launch_bounds__(128) k_ball_emit(TreeView tv, const double* __restrict__ Q,
                                                    const EmitTask* __restrict__ tasks,
                                                    const unsigned* __restrict__ n_tasks,
+                                                   unsigned task_cap,
                                                    int64_t* __restrict__ oidx,
                                                    double* __restrict__ odist, int want_d2) {
   const int lane = threadIdx.x & 31;
-  const int64_t nt = min((int64_t)*n_tasks, (int64_t)kTaskCap);
+  const int64_t nt = min((int64_t)*n_tasks, (int64_t)task_cap);
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < nt;
        t += nwarps) {
@@ -856,17 +860,19 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
     const int hstack_len = std::max(kHeavyStack, t->depth + 4);
     if (hstack_len > kHeavyStack)
       CKD_CUDA(sc.alloc(&hstack, sizeof(int32_t) * hstack_len * hblocks * 4));
+    const unsigned task_cap =
+        (unsigned)std::min<int64_t>(kTaskCap, std::max<int64_t>(1 << 16, nq * 64));
     EmitTask* tasks = nullptr;
     unsigned* ntask = nullptr;
-    CKD_CUDA(sc.alloc(&tasks, sizeof(EmitTask) * kTaskCap));
+    CKD_CUDA(sc.alloc(&tasks, sizeof(EmitTask) * task_cap));
     CKD_CUDA(sc.alloc(&ntask, sizeof(unsigned)));
     CKD_CUDA(cudaMemsetAsync(ntask, 0, sizeof(unsigned), s));
     k_ball_fill_warp<D, PER><<<(unsigned)std::max<int64_t>(1, hblocks), 128, 0, s>>>(
         tv, q, heavy, cnt, r2, hstack, hstack_len, offsets, idx, dist, sorted ? 1 : 0, tasks,
-        ntask, qroot);
+        ntask, task_cap, qroot);
     CKD_LAUNCH_CHECK();
-    k_ball_emit<D, PER><<<(unsigned)sms * 8, 128, 0, s>>>(tv, q, tasks, ntask, idx, dist,
-                                                          sorted ? 1 : 0);
+    k_ball_emit<D, PER><<<(unsigned)sms * 8, 128, 0, s>>>(tv, q, tasks, ntask, task_cap, idx,
+                                                          dist, sorted ? 1 : 0);
     CKD_LAUNCH_CHECK();
   } else {
     if (qroot)
