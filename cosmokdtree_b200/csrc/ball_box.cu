@@ -16,8 +16,10 @@
 // union of the lanes' paths with a per-entry lane mask, left first, so every
 // row comes out in the reference's order.
 #include <algorithm>
+#include <cmath>
 
 #include "ckd_common.cuh"
+#include "ckd_knn.cuh"
 #include "ckd_traverse.cuh"
 
 namespace ckd {
@@ -35,7 +37,10 @@ __global__ void __launch_bounds__(128) k_ball(TreeView tv, const double* __restr
                                               const int64_t* __restrict__ offsets,
                                               int64_t* __restrict__ oidx,
                                               double* __restrict__ odist, int want_d2,
-                                              const int32_t* __restrict__ qroot) {
+                                              const int32_t* __restrict__ qroot,
+                                              int32_t* __restrict__ heavy = nullptr,
+                                              unsigned* __restrict__ n_heavy = nullptr,
+                                              int budget = 0) {
   // packet stack entries; with ROOTS (forests) each entry also carries the lanes
   // whose balls reached its parent, and the search starts one entry per distinct
   // root among the warp's queries
@@ -60,6 +65,7 @@ __global__ void __launch_bounds__(128) k_ball(TreeView tv, const double* __restr
   int64_t cur = (FILL && valid) ? offsets[qi] : 0;
   const int64_t cur_end = (FILL && valid) ? offsets[qi + 1] : 0;
   int32_t cov_lo = 0, cov_hi = 0;  // point range already counted whole (count pass)
+  int visited = 0;
   int top = 0;
   if (ROOTS) {
     const int32_t root = valid ? qroot[qi] : -1;
@@ -81,6 +87,14 @@ __global__ void __launch_bounds__(128) k_ball(TreeView tv, const double* __restr
     const unsigned em = ROOTS ? msk[top] : 0xffffffffu;
     --top;
     __syncwarp();
+    if (heavy && ++visited > budget) {  // left to the warp kernel, which starts again
+      const unsigned vm = __ballot_sync(0xffffffffu, valid);
+      unsigned base = 0;
+      if (lane == 0) base = atomicAdd(n_heavy, (unsigned)__popc(vm));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (valid) heavy[base + __popc(vm & ((1u << lane) - 1u))] = (int32_t)qi;
+      return;
+    }
     NodeMeta m = load_meta(tv.meta, node);
     bool need = ((em >> lane) & 1u) && box_mind2<D, PER>(tv, q, node) <= rr;
     if (!FILL && need && m.start >= cov_lo && m.start < cov_hi) need = false;
@@ -426,17 +440,332 @@ __global__ void __launch_bounds__(128) k_ball_emit(TreeView tv, const double* __
   }
 }
 
+// ------------------------------------------------------- ball, FP32 node tests
+// One query's ball against FP32 boxes.  The tests only decide what is surely
+// outside (pruned) or surely inside (taken whole); every other point is tested in FP64 with the reference arithmetic, so results are exact.  Query
+// coordinates beyond the FP32 range are clamped: the gaps of the clamped query
+// never exceed the true ones (tree coordinates are below 1e18 here), and such a
+// query takes nothing whole.
+template <int D, bool PER>
+struct BallQuery {
+  static constexpr int NV = (D + 3) / 4;
+  const TreeView& tv;
+  double q[D];
+  double rr;
+  QueryScreen<D, PER> qs;
+  float xl[D], xh[D];
+  float r2u, r2d;  // r^2 rounded up / down
+  bool wf;              // the ball cannot reach the periodic faces
+  bool whole_ok;
+
+  __device__ __forceinline__ BallQuery(const TreeView& t, const double* __restrict__ Q, int64_t qi,
+                                       double r2)
+      : tv(t), rr(r2) {
+    whole_ok = true;
+    r2u = __double2float_ru(r2);
+    r2d = __double2float_rd(r2);
+    const float r32 = sqrt_up(r2u);
+    wf = true;
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      q[j] = Q[qi * D + j];
+      const float x = __double2float_rn(q[j]);
+      whole_ok = whole_ok && fabsf(x) < 1e18f;
+      qs.q32[j] = fminf(fmaxf(x, -2e18f), 2e18f);
+      qs.dlt[j] = kTwoM21 * (fabsf(qs.q32[j]) + tv.slack[j]) * 1.0001f;
+      xl[j] = __fadd_ru(qs.q32[j], qs.dlt[j]);
+      xh[j] = __fsub_rd(qs.q32[j], qs.dlt[j]);
+      if (PER)
+        wf = wf && __fadd_ru(__fadd_ru(fabsf(qs.q32[j]), r32), qs.dlt[j]) < 0.5f * (float)tv.L[j];
+    }
+  }
+  // lower bound of the squared distance to any point of the box
+  __device__ __forceinline__ float lb(const float (&lo)[4 * NV], const float (&hi)[4 * NV]) const {
+    if (!PER || wf) {
+      float s2 = 0.0f;
+#pragma unroll
+      for (int j = 0; j < D; ++j) {
+        const float g = fmaxf(fmaxf(lo[j] - xl[j], xh[j] - hi[j]), 0.0f);
+        s2 = fmaf(g, g, s2);
+      }
+      return s2 * kShrink;
+    }
+    return box_mind_lb<D, PER>(tv, qs, lo, hi);
+  }
+  // whether every point of the box is surely within r: the direct differences,
+  // rounded up, bound every point's (the minimum image is the direct difference
+  // when that is at most half a side)
+  __device__ __forceinline__ bool holds(const float (&lo)[4 * NV], const float (&hi)[4 * NV]) const {
+    float s2 = 0.0f;
+    bool ok = whole_ok;
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      const float g = fmaxf(__fsub_ru(xl[j], lo[j]), __fsub_ru(hi[j], xh[j]));
+      if (PER) ok = ok && g <= 0.4999999f * (float)tv.L[j];
+      s2 = __fmaf_ru(g, g, s2);
+    }
+    return ok && __fmul_ru(s2, 1.000002f) <= r2d;
+  }
+  // Children of an internal node that the ball reaches, as entries {node, 0},
+  // {start, count} (to be tested point by point) or {start, -count} (whole);
+  // y == kNone: not reached.  Subtrees of at most `unit` points come as ranges.
+  static constexpr int32_t kNone = INT32_MIN;
+  __device__ __forceinline__ void expand(int32_t node, int32_t unit, int2& a, int2& b) const {
+    const float4* rec = tv.pair + (int64_t)node * pair_f4(D);
+    float v[4][4 * NV];
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int h = 0; h < NV; ++h) {
+        const float4 f = CKD_LDT(rec + s * NV + h);
+        v[s][4 * h] = f.x;
+        v[s][4 * h + 1] = f.y;
+        v[s][4 * h + 2] = f.z;
+        v[s][4 * h + 3] = f.w;
+      }
+    const int4 info = CKD_LDT(reinterpret_cast<const int4*>(rec + 4 * NV));
+    const int4 range = CKD_LDT(reinterpret_cast<const int4*>(rec + 4 * NV + 1));
+    const bool ra = info.z || range.y <= unit, rb = info.w || range.w <= unit;
+    a = make_int2(ra ? range.x : info.x, ra ? range.y : 0);
+    b = make_int2(rb ? range.z : info.y, rb ? range.w : 0);
+    if (!(lb(v[0], v[1]) <= r2u)) a.y = kNone;
+    else if (holds(v[0], v[1])) a = make_int2(range.x, -range.y);
+    if (!(lb(v[2], v[3]) <= r2u)) b.y = kNone;
+    else if (holds(v[2], v[3])) b = make_int2(range.z, -range.w);
+  }
+  // The subtree that holds the ball, from a root: while the split plane is further
+  // than r from the query, only its side of it can hold results.  The points left
+  // of a split lie at or below it, those on the right at or above it, and rounding
+  // is monotone, so a point on the far side has a computed squared distance of at
+  // least (split - q)^2, computed the same way.  Not for balls that may reach a
+  // periodic face.
+  __device__ __forceinline__ int2 root(int32_t node, int32_t unit) const {
+    NodeMeta m = load_meta(tv.meta, node);
+    while (m.left >= 0 && m.count > unit && (!PER || wf)) {
+      double qa = 0.0;
+#pragma unroll
+      for (int j = 0; j < D; ++j)
+        if (j == m.axis) qa = q[j];
+      const double g = dsub(m.split, qa);
+      if (!(dmul(g, g) > rr)) break;
+      node = g > 0.0 ? m.left : m.left + 1;
+      m = load_meta(tv.meta, node);
+    }
+    return m.left < 0 || m.count <= unit ? make_int2(m.start, m.count) : make_int2(node, 0);
+  }
+};
+
+// ------------------------------------------------------------ ball, warp per query
+// The warp keeps a stack of entries (BallQuery::expand) in depth-first order, the
+// next one on top.  Up to 32 entries are taken at once, a lane each: nodes are
+// replaced by their reached children (left on top), so the children of many nodes
+// are tested in parallel.
+//   count: ranges never enter the stack; whole ones are added up, the others listed
+//     and scanned over the lanes when enough wait;
+//   fill: the ranges above the topmost node are next in the row: they are emitted
+//     in order, flattened over the lanes, the others stay where they are.  A whole
+//     range of kTaskMin points on becomes emission tasks, which k_ball_emit spreads
+//     over the GPU.
+// A row is in leaf order, the order of the packet kernel and of k_ball_fill_warp.
+// The packet kernel walks the union of 32 balls with FP64 box tests, which is what
+// it was bound by; 4001 scattered queries on 2^22 clustered points, 20000 results
+// each: count 32.2 -> 0.45 ms, fill 8.8 -> 1.85 ms; 10^5 on 2^20 uniform points, 5
+// results each: 0.39 -> 0.26 and 0.44 -> 0.28 ms.  Now bound by issue: about 3000
+// warp instructions a query of the latter.  A lane per query (tried for small
+// balls, 100k queries) was no faster, waiting on its dependent loads.
+constexpr int kBallStack = 320;
+constexpr int kBallReserve = 130;  // room for one-at-a-time descents (tree depth < 127)
+constexpr int kBallList = 128;
+constexpr int kBallListRun = 16;   // ranges that wait before they are scanned (count)
+constexpr int32_t kBallUnit = 32;  // subtrees of at most this many points are scanned as a range
+constexpr int32_t kBallRoot = 64;  // and of this many where the descent from the root ends
+
+template <int D, bool PER, bool FILL>
+__global__ void __launch_bounds__(128) k_ball_warp(
+    TreeView tv, const double* __restrict__ Q, const int32_t* __restrict__ order, int64_t nq,
+    double r2, int64_t* __restrict__ counts,
+    const int64_t* __restrict__ offsets, int64_t* __restrict__ oidx, double* __restrict__ odist,
+    int want_d2, EmitTask* __restrict__ tasks, unsigned* __restrict__ n_tasks, unsigned task_cap,
+    const int32_t* __restrict__ qroot, const unsigned* __restrict__ n_rows = nullptr) {
+  constexpr unsigned FULL = 0xffffffffu;
+  using BQ = BallQuery<D, PER>;
+  __shared__ int2 s_stk[4][kBallStack];
+  __shared__ int2 s_list[4][FILL ? 1 : kBallList];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  int2* stk = s_stk[w];
+  int2* list = s_list[w];
+  const int64_t nr = n_rows ? (int64_t)*n_rows : nq;
+  for (int64_t r = (int64_t)blockIdx.x * 4 + w; r < nr; r += (int64_t)gridDim.x * 4) {
+    const int64_t qi = order ? (int64_t)order[r] : r;
+    int64_t cur = FILL ? offsets[qi] : 0;
+    const int64_t cur_end = FILL ? offsets[qi + 1] : 0;
+    if (FILL && cur == cur_end) continue;
+    const BQ bq(tv, Q, qi, r2);
+    int64_t cnt = 0;  // per lane
+    int top = 1, nl = 0;
+    if (lane == 0) stk[0] = bq.root(qroot ? qroot[qi] : 0, kBallRoot);
+    __syncwarp();
+    while (top > 0) {
+      if (FILL && cur >= cur_end) break;  // all of the row's results are found
+      const int n = min(min(top, 32), max(1, kBallStack - kBallReserve - top));
+      int2 e = make_int2(0, BQ::kNone);
+      if (lane < n) e = stk[top - 1 - lane];
+      __syncwarp();
+      top -= n;
+      // lanes below `lead` hold the ranges that come next (fill)
+      int lead = 0;
+      if (FILL) {
+        const unsigned nm = __ballot_sync(FULL, lane >= n || e.y == 0);
+        lead = nm ? __ffs(nm) - 1 : 32;
+        const unsigned big = __ballot_sync(FULL, lane < lead && e.y <= -kTaskMin);
+        if (big & 1u) lead = 1;
+        else if (big) lead = __ffs(big) - 1;
+      }
+      int2 a = make_int2(0, BQ::kNone), b = make_int2(0, BQ::kNone);
+      if (lane < n && lane >= lead) {
+        if (e.y == 0) bq.expand(e.x, kBallUnit, a, b);
+        else a = e;
+      }
+      if (!FILL) {
+        if (a.y < 0 && a.y != BQ::kNone) {
+          cnt -= a.y;
+          a.y = BQ::kNone;
+        }
+        if (b.y < 0 && b.y != BQ::kNone) {
+          cnt -= b.y;
+          b.y = BQ::kNone;
+        }
+        const unsigned ga = __ballot_sync(FULL, a.y > 0), gb = __ballot_sync(FULL, b.y > 0);
+        const int o = nl + __popc(ga & lt) + __popc(gb & lt);
+        if (a.y > 0) list[o] = a;
+        if (b.y > 0) list[o + (a.y > 0 ? 1 : 0)] = b;
+        nl += __popc(ga) + __popc(gb);
+        if (a.y > 0) a.y = BQ::kNone;
+        if (b.y > 0) b.y = BQ::kNone;
+      }
+      // back onto the stack, the first lane's entries on top, left above right
+      const unsigned ma = __ballot_sync(FULL, a.y != BQ::kNone);
+      const unsigned mb = __ballot_sync(FULL, b.y != BQ::kNone);
+      const int total = __popc(ma) + __popc(mb);
+      const int above = __popc(ma & lt) + __popc(mb & lt);
+      if (a.y != BQ::kNone) stk[top + total - 1 - above] = a;
+      if (b.y != BQ::kNone) stk[top + total - 1 - above - (a.y != BQ::kNone ? 1 : 0)] = b;
+      top += total;
+      __syncwarp();
+      if (!FILL) {
+        if (nl < kBallListRun && top > 0) continue;
+#pragma unroll 1
+        for (int u0 = 0; u0 < nl; u0 += 32) {
+          const int2 x = u0 + lane < nl ? list[u0 + lane] : make_int2(0, 0);
+          int32_t inc = x.y;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int32_t v = __shfl_up_sync(FULL, inc, o);
+            if (lane >= o) inc += v;
+          }
+          const int32_t tot = __shfl_sync(FULL, inc, 31);
+          const int32_t delta = x.x - (inc - x.y);
+#pragma unroll 2
+          for (int32_t t = lane; t - lane < tot; t += 32) {
+            int j = 0;  // the range holding t: the first with inc > t
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+              const int32_t v = __shfl_sync(FULL, inc, j + o - 1);
+              if (v <= t) j += o;
+            }
+            const int32_t p = __shfl_sync(FULL, delta, j) + t;
+            if (t < tot && point_d2_rec<D, PER>(tv, bq.q, p) <= r2) ++cnt;
+          }
+        }
+        nl = 0;
+        __syncwarp();
+      } else if (lead > 0) {
+        if (lead == 1) {  // a large whole range: tasks, unless their buffer is full
+          const int32_t st = __shfl_sync(FULL, e.x, 0), ct = -__shfl_sync(FULL, e.y, 0);
+          if (ct >= kTaskMin && cur < cur_end) {
+            const int64_t len = min((int64_t)ct, cur_end - cur);
+            const unsigned nt = (unsigned)((len + kTaskChunk - 1) / kTaskChunk);
+            unsigned tb = 0;
+            if (lane == 0) tb = atomicAdd(n_tasks, nt);
+            tb = __shfl_sync(FULL, tb, 0);
+            if (tb + nt <= task_cap) {
+              for (unsigned c = lane; c < nt; c += 32) {
+                EmitTask x;
+                x.out = cur + (int64_t)c * kTaskChunk;
+                x.start = st + (int32_t)c * kTaskChunk;
+                x.count = (int32_t)min((int64_t)kTaskChunk, len - (int64_t)c * kTaskChunk);
+                x.qi = (int32_t)qi;
+                x.pad = 0;
+                tasks[tb + c] = x;
+              }
+              cur += ct;
+              continue;
+            }
+            // the buffer is full: the slots left in it hold no work
+            for (unsigned c = lane; c < nt && tb + c < task_cap; c += 32)
+              tasks[tb + c] = EmitTask{};
+          }
+        }
+        const int32_t ct = lane < lead ? abs(e.y) : 0;
+        int32_t inc = ct;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int32_t v = __shfl_up_sync(FULL, inc, o);
+          if (lane >= o) inc += v;
+        }
+        const int32_t tot = __shfl_sync(FULL, inc, 31);
+        const int32_t delta = e.x - (inc - ct);
+        const unsigned wholes = __ballot_sync(FULL, lane < lead && e.y < 0);
+#pragma unroll 2
+        for (int32_t t = lane; t - lane < tot; t += 32) {
+          int j = 0;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            const int32_t v = __shfl_sync(FULL, inc, j + o - 1);
+            if (v <= t) j += o;
+          }
+          const int32_t p = __shfl_sync(FULL, delta, j) + t;
+          bool hit = t < tot;
+          double d2 = 0.0;
+          int32_t id = 0;
+          if (hit) {
+            d2 = point_d2_rec<D, PER>(tv, bq.q, p);
+            id = CKD_LDT(&tv.ids[p]);
+            hit = d2 <= r2 || ((wholes >> (j & 31)) & 1u);
+          }
+          const unsigned hm = __ballot_sync(FULL, hit);
+          if (hit) {
+            const int64_t o = cur + __popc(hm & lt);
+            if (o < cur_end) {
+              oidx[o] = id;
+              odist[o] = want_d2 ? d2 : sqrt(d2);
+            }
+          }
+          cur += __popc(hm);
+        }
+      }
+    }
+    if (!FILL) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(FULL, cnt, o);
+      if (lane == 0) counts[qi] = cnt;
+    }
+    __syncwarp();
+  }
+}
+
 // rows of the fill split by length: heavy ones (>= kHeavyRow) to `heavy`, the rest
 // to `light`, both in the processing order (`order`, the leaf order when given)
 __global__ void k_split_rows(const int64_t* __restrict__ offsets, const int32_t* __restrict__ order,
-                             int64_t nq, int32_t* __restrict__ heavy,
+                             int64_t nq, int64_t heavy_row, int32_t* __restrict__ heavy,
                              unsigned* __restrict__ n_heavy, int32_t* __restrict__ light,
                              unsigned* __restrict__ n_light) {
   const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool valid = slot < nq;
   const int64_t i = valid ? (order ? (int64_t)order[slot] : slot) : 0;
-  const bool h = valid && offsets[i + 1] - offsets[i] >= kHeavyRow;
+  const bool h = valid && offsets[i + 1] - offsets[i] >= heavy_row;
   const unsigned hm = __ballot_sync(0xffffffffu, h);
   const unsigned lm = __ballot_sync(0xffffffffu, valid && !h);
   unsigned hb = 0, lb = 0;
@@ -818,6 +1147,28 @@ __global__ void __launch_bounds__(128) k_box(TreeView tv, const double* __restri
   if (!FILL && valid) counts[bi] = cnt;
 }
 
+// Batches up to which every query takes a warp of its own.  Beyond, the packet
+// kernel goes first: 32 queries adjacent in leaf order share their nodes, which is
+// faster while the balls are small against their spacing (10^6 queries on 2^20
+// uniform points, 5 results each: count 1.05 against 2.29 ms) and far slower
+// where density is uneven (3 x 10^5 queries on 2^22 clustered points, 1290 results
+// each: 12.1 against 2.1 ms).  There a packet that has visited kPacketBudget nodes
+// hands its queries over, unless they lie denser than half the points (2^22
+// clustered points, 950 results each, count with / without handing over: 2^20
+// queries 8.3 / 12.4 ms, 2^22 queries 27.4 / 23.4 ms); on an even tree it shares
+// enough to go on (10^6 queries on 2^20 uniform points, 2700 results each: 13.3
+// against 16.5 ms).  The fill gives it
+// rows of fewer than kPacketRow results only (3 x 10^5 rows of 287 results: 13.4 ms
+// as packets, 2.2 as warps; of 30 results: 1.09 and 1.05).
+constexpr int64_t kBallWarpMax = 200000;
+constexpr int kPacketBudget = 512;
+constexpr int64_t kPacketRow = 64;
+bool ball_warp_ok(const ckd_tree* t) { return t->screen_ok && t->depth < kBallReserve - 3; }
+// uneven density: a tree much deeper than its leaf count needs
+bool uneven(const ckd_tree* t) {
+  return t->depth > 1.5 * std::log2((double)t->n / t->leaf + 2.0);
+}
+
 template <int D, bool PER>
 ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
                        double r, bool fill, int sorted, int64_t* counts, const int64_t* offsets,
@@ -830,59 +1181,79 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
   int stack_len = std::max(kStack, t->depth + 4 + (qroot ? 32 : 0));
   Scratch sc(s);
   int32_t* gstack = nullptr;
-  if (stack_len > kStack)
+  if (stack_len > kStack && !ball_warp_ok(t))
     CKD_CUDA(sc.alloc(&gstack, sizeof(int32_t) * 2 * stack_len * (int64_t)blocks * nw));
   double r2 = r * r;  // radius**2 (cosmokdtree.f90:1112)
-  if (fill) {
-    // heavy rows: a warp per query; light rows: the per-lane kernel over a list
-    int32_t *heavy = nullptr, *light = nullptr, *hstack = nullptr;
-    unsigned* cnt = nullptr;
-    CKD_CUDA(sc.alloc(&heavy, sizeof(int32_t) * nq));
-    CKD_CUDA(sc.alloc(&light, sizeof(int32_t) * nq));
-    CKD_CUDA(sc.alloc(&cnt, 2 * sizeof(unsigned)));
-    CKD_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), s));
-    k_split_rows<<<(unsigned)cdiv(nq, 256), 256, 0, s>>>(offsets, order, nq, heavy, cnt, light,
-                                                         cnt + 1);
-    CKD_LAUNCH_CHECK();
-    if (qroot)
-      k_ball<D, PER, true, true><<<blocks, threads, 0, s>>>(tv, q, light, nq, cnt + 1, r2, gstack,
-                                                            stack_len, nullptr, offsets, idx,
-                                                            dist, sorted ? 1 : 0, qroot);
+  int dev = 0, sms = 148;
+  CKD_CUDA(cudaGetDevice(&dev));
+  CKD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // rows of the warp kernel (null: all, in processing order), and the packet
+  // kernel's rows before it for large batches and for trees that the warp kernel
+  // does not take
+  const bool warp = ball_warp_ok(t), packet = !warp || nq > kBallWarpMax;
+  int32_t *heavy = nullptr, *light = nullptr;
+  unsigned* cnt = nullptr;  // heavy rows, light rows, emission tasks
+  CKD_CUDA(sc.alloc(&cnt, 3 * sizeof(unsigned)));
+  if (packet || fill) CKD_CUDA(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), s));
+  if (packet) {
+    if (warp || fill) CKD_CUDA(sc.alloc(&heavy, sizeof(int32_t) * nq));
+    if (fill) {
+      CKD_CUDA(sc.alloc(&light, sizeof(int32_t) * nq));
+      k_split_rows<<<(unsigned)cdiv(nq, 256), 256, 0, s>>>(
+          offsets, order, nq, warp ? kPacketRow : kHeavyRow, heavy, cnt, light, cnt + 1);
+      CKD_LAUNCH_CHECK();
+    }
+    int32_t* bail = warp && uneven(t) && nq * 2 <= t->n ? heavy : nullptr;
+    const int w2 = sorted ? 1 : 0;
+    if (fill && qroot)
+      k_ball<D, PER, true, true><<<blocks, threads, 0, s>>>(
+          tv, q, light, nq, cnt + 1, r2, gstack, stack_len, nullptr, offsets, idx, dist, w2, qroot,
+          bail, cnt, kPacketBudget);
+    else if (fill)
+      k_ball<D, PER, true><<<blocks, threads, 0, s>>>(
+          tv, q, light, nq, cnt + 1, r2, gstack, stack_len, nullptr, offsets, idx, dist, w2,
+          nullptr, bail, cnt, kPacketBudget);
+    else if (qroot)
+      k_ball<D, PER, false, true><<<blocks, threads, 0, s>>>(
+          tv, q, order, nq, nullptr, r2, gstack, stack_len, counts, nullptr, nullptr, nullptr, 0,
+          qroot, bail, cnt, kPacketBudget);
     else
-      k_ball<D, PER, true><<<blocks, threads, 0, s>>>(tv, q, light, nq, cnt + 1, r2, gstack,
-                                                       stack_len, nullptr, offsets, idx, dist,
-                                                       sorted ? 1 : 0, nullptr);
+      k_ball<D, PER, false><<<blocks, threads, 0, s>>>(
+          tv, q, order, nq, nullptr, r2, gstack, stack_len, counts, nullptr, nullptr, nullptr, 0,
+          nullptr, bail, cnt, kPacketBudget);
     CKD_LAUNCH_CHECK();
-    int dev = 0, sms = 148;
-    CKD_CUDA(cudaGetDevice(&dev));
-    CKD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  const unsigned task_cap =
+      (unsigned)std::min<int64_t>(kTaskCap, std::max<int64_t>(1 << 16, nq * 64));
+  EmitTask* tasks = nullptr;
+  if (fill) CKD_CUDA(sc.alloc(&tasks, sizeof(EmitTask) * task_cap));
+  if (warp) {
+    const unsigned g = (unsigned)std::min<int64_t>(cdiv(nq, nw), (int64_t)sms * 16);
+    const int32_t* rows = packet ? heavy : order;
+    const unsigned* n_rows = packet ? cnt : nullptr;
+    if (fill)
+      k_ball_warp<D, PER, true><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, nullptr, offsets, idx,
+                                                      dist, sorted ? 1 : 0, tasks, cnt + 2,
+                                                      task_cap, qroot, n_rows);
+    else
+      k_ball_warp<D, PER, false><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, counts, nullptr,
+                                                       nullptr, nullptr, 0, nullptr, nullptr, 0,
+                                                       qroot, n_rows);
+    CKD_LAUNCH_CHECK();
+  } else if (fill) {
     const int64_t hblocks = std::min<int64_t>(cdiv(nq, 4), (int64_t)sms * 8);
     const int hstack_len = std::max(kHeavyStack, t->depth + 4);
+    int32_t* hstack = nullptr;
     if (hstack_len > kHeavyStack)
       CKD_CUDA(sc.alloc(&hstack, sizeof(int32_t) * hstack_len * hblocks * 4));
-    const unsigned task_cap =
-        (unsigned)std::min<int64_t>(kTaskCap, std::max<int64_t>(1 << 16, nq * 64));
-    EmitTask* tasks = nullptr;
-    unsigned* ntask = nullptr;
-    CKD_CUDA(sc.alloc(&tasks, sizeof(EmitTask) * task_cap));
-    CKD_CUDA(sc.alloc(&ntask, sizeof(unsigned)));
-    CKD_CUDA(cudaMemsetAsync(ntask, 0, sizeof(unsigned), s));
     k_ball_fill_warp<D, PER><<<(unsigned)std::max<int64_t>(1, hblocks), 128, 0, s>>>(
         tv, q, heavy, cnt, r2, hstack, hstack_len, offsets, idx, dist, sorted ? 1 : 0, tasks,
-        ntask, task_cap, qroot);
+        cnt + 2, task_cap, qroot);
     CKD_LAUNCH_CHECK();
-    k_ball_emit<D, PER><<<(unsigned)sms * 8, 128, 0, s>>>(tv, q, tasks, ntask, task_cap, idx,
+  }
+  if (fill) {
+    k_ball_emit<D, PER><<<(unsigned)sms * 8, 128, 0, s>>>(tv, q, tasks, cnt + 2, task_cap, idx,
                                                           dist, sorted ? 1 : 0);
-    CKD_LAUNCH_CHECK();
-  } else {
-    if (qroot)
-      k_ball<D, PER, false, true><<<blocks, threads, 0, s>>>(tv, q, order, nq, nullptr, r2,
-                                                             gstack, stack_len, counts, nullptr,
-                                                             nullptr, nullptr, 0, qroot);
-    else
-      k_ball<D, PER, false><<<blocks, threads, 0, s>>>(tv, q, order, nq, nullptr, r2, gstack,
-                                                        stack_len, counts, nullptr, nullptr,
-                                                        nullptr, 0, nullptr);
     CKD_LAUNCH_CHECK();
   }
   if (fill && sorted) {
@@ -905,9 +1276,6 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
         CKD_CUDA(sc.alloc(&tidx, sizeof(int64_t) * hs[1]));
         CKD_CUDA(sc.alloc(&tdist, sizeof(double) * hs[1]));
       }
-      int dev = 0, sms = 148;
-      CKD_CUDA(cudaGetDevice(&dev));
-      CKD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       const unsigned g = (unsigned)std::min<unsigned long long>(hs[0], (unsigned long long)sms * 8);
       k_sort_big<<<g, 256, 0, s>>>(offsets, big, sel, toff, idx, dist, tidx, tdist);
       CKD_LAUNCH_CHECK();
@@ -964,12 +1332,21 @@ bool want_order(const ckd_tree* t, int64_t nq);
 ckd_status query_order_roots(const ckd_tree* t, const double* q, int64_t nq, int32_t* order,
                              const int32_t* qroot, cudaStream_t s);
 
+// Leaf order of a ball search's queries.  A warp per query gains from it only
+// through the caches, where density is uneven and rows are long (10^5 queries on 2^22 clustered points, 218 results
+// each: count + fill 1473 ordered, 1920 us in the caller's order; on 2^20 uniform
+// points 611 against 533, the ordering included).
+bool want_ball_order(const ckd_tree* t, int64_t nq) {
+  if (query_order_mode() != 0 || nq > kBallWarpMax || !ball_warp_ok(t)) return want_order(t, nq);
+  return nq >= 50000 && uneven(t) && want_order(t, nq);
+}
+
 ckd_status ball_run(const ckd_tree* t, const double* q, int64_t nq, double r, bool fill, int sorted,
                     int64_t* counts, const int64_t* offsets, int64_t* idx, double* dist,
                     cudaStream_t s, const int32_t* qroot) {
   int32_t* order = nullptr;
   Scratch sc(s);
-  if (want_order(t, nq)) {
+  if (want_ball_order(t, nq)) {
     CKD_CUDA(sc.alloc(&order, sizeof(int32_t) * nq));
     CKD_TRY(query_order_roots(t, q, nq, order, qroot, s));
   }

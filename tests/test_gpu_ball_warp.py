@@ -1,0 +1,76 @@
+"""The warp-per-query ball kernel against the oracle at the edges of its scan units, its batch
+rule and its hand-overs.  Counts, ids and FP64 distances are compared for equality (separately
+rounded arithmetic on both sides); unsorted periodic rows hold the reference's points in leaf
+order, so they are compared sorted."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import make_points
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # name, n, d, periodic, leaf, nq, r
+    ("tiny", 5, 3, False, 16, 3, 0.4),
+    ("uniform3d", 65, 3, False, 16, 9, 0.3),            # one scan unit past the root's
+    ("uniform3d", 6000, 3, False, 16, 33, 0.05),
+    ("periodic3d", 6000, 3, True, 8, 33, 0.2),          # balls across the faces
+    ("periodic_clustered", 20000, 3, True, 16, 64, 0.45),
+    ("clustered_dup", 20000, 3, False, 40, 64, 0.02),   # leaves longer than a unit
+    ("lattice", 8000, 3, False, 1, 40, 0.125),          # distances equal to the radius
+    ("lattice_periodic", 8000, 3, True, 16, 40, 0.25),
+    ("d1", 3000, 1, True, 16, 17, 0.01),
+    ("d2", 3000, 2, False, 3, 17, 0.1),
+    ("d5", 3000, 5, False, 16, 17, 0.4),
+    ("d8", 3000, 8, True, 16, 17, 0.6),
+]
+
+
+@pytest.mark.parametrize("sorted_", [False, True])
+@pytest.mark.parametrize("name,n,d,periodic,leaf,nq,r", CASES)
+def test_gpu_ball_warp_matches_oracle(gpu, oracle, name, n, d, periodic, leaf, nq, r, sorted_):
+    P = make_points(name, n, d, periodic)
+    rng = np.random.default_rng(41)
+    Q = np.concatenate([P[rng.integers(0, n, nq // 2)],
+                        rng.random((nq - nq // 2, d)) - (0.5 if periodic else 0.0)])
+    if not periodic:
+        Q[-1] = 1e30  # far beyond FP32 squares
+    box = 1.0 if periodic else None
+    t = gpu.kdtree.build_kdtree(P, leaf=leaf, boxsize=box)
+    ooff, oidx, odist = oracle.OracleTree(P, leaf, box).ball_csr(Q, r, sorted=sorted_)
+    off, idx, dist = (x.cpu().numpy() for x in
+                      gpu.kdtree.ball_search_csr(t, Q, r, sorted=sorted_))
+    np.testing.assert_array_equal(off, ooff)
+    if sorted_ or not periodic:
+        np.testing.assert_array_equal(idx, oidx)
+        np.testing.assert_array_equal(dist, odist)
+    else:
+        for a, b in zip(off[:-1], off[1:]):
+            np.testing.assert_array_equal(np.sort(idx[a:b]), np.sort(oidx[a:b]))
+            np.testing.assert_array_equal(np.sort(dist[a:b]), np.sort(odist[a:b]))
+
+
+@pytest.mark.parametrize("name,r", [("uniform3d", 0.01), ("clustered_deep", 0.004)])
+def test_gpu_ball_batches_past_the_warp_rule(gpu, name, r):
+    """A batch past the rule (packets first, heavy ones handed over on an uneven tree) gives
+    the rows of the same queries in small batches."""
+    rng = np.random.default_rng(43)
+    n, nq = 410000, 200001
+    P = rng.random((n, 3))
+    if name == "clustered_deep":  # most points in a few very dense clumps
+        c = rng.random((6, 3))
+        P[: n - 20000] = c[rng.integers(0, 6, n - 20000)] + \
+            rng.standard_normal((n - 20000, 3)) * 10.0 ** rng.uniform(-6, -2, (n - 20000, 1))
+    t = gpu.kdtree.build_kdtree(P)
+    Q = P[rng.integers(0, n, nq)]
+    if name == "clustered_deep":
+        Q[: nq - 2000] = rng.random((nq - 2000, 3)) * 3.0  # mostly empty rows, some very long
+    off, idx, dist = gpu.kdtree.ball_search_csr(t, Q, r)
+    ids = rng.integers(0, nq, 3000)
+    ids[:500] = nq - 1 - np.arange(500)
+    soff, sidx, sdist = gpu.kdtree.ball_search_csr(t, Q[ids], r)
+    off, soff = off.cpu().numpy(), soff.cpu().numpy()
+    np.testing.assert_array_equal(np.diff(off)[ids], np.diff(soff))
+    take = np.concatenate([np.arange(off[i], off[i + 1]) for i in ids])
+    np.testing.assert_array_equal(idx.cpu().numpy()[take], sidx.cpu().numpy())
+    np.testing.assert_array_equal(dist.cpu().numpy()[take], sdist.cpu().numpy())
