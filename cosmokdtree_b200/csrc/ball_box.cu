@@ -448,7 +448,9 @@ __global__ void __launch_bounds__(128) k_ball_emit(TreeView tv, const double* __
 // query takes nothing whole.
 template <int D, bool PER>
 struct BallQuery {
+  static constexpr int kD = D;
   static constexpr int NV = (D + 3) / 4;
+  static constexpr bool kDist = true;
   const TreeView& tv;
   double q[D];
   double rr;
@@ -506,32 +508,13 @@ struct BallQuery {
     }
     return ok && __fmul_ru(s2, 1.000002f) <= r2d;
   }
-  // Children of an internal node that the ball reaches, as entries {node, 0},
-  // {start, count} (to be tested point by point) or {start, -count} (whole);
-  // y == kNone: not reached.  Subtrees of at most `unit` points come as ranges.
-  static constexpr int32_t kNone = INT32_MIN;
-  __device__ __forceinline__ void expand(int32_t node, int32_t unit, int2& a, int2& b) const {
-    const float4* rec = tv.pair + (int64_t)node * pair_f4(D);
-    float v[4][4 * NV];
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int h = 0; h < NV; ++h) {
-        const float4 f = CKD_LDT(rec + s * NV + h);
-        v[s][4 * h] = f.x;
-        v[s][4 * h + 1] = f.y;
-        v[s][4 * h + 2] = f.z;
-        v[s][4 * h + 3] = f.w;
-      }
-    const int4 info = CKD_LDT(reinterpret_cast<const int4*>(rec + 4 * NV));
-    const int4 range = CKD_LDT(reinterpret_cast<const int4*>(rec + 4 * NV + 1));
-    const bool ra = info.z || range.y <= unit, rb = info.w || range.w <= unit;
-    a = make_int2(ra ? range.x : info.x, ra ? range.y : 0);
-    b = make_int2(rb ? range.z : info.y, rb ? range.w : 0);
-    if (!(lb(v[0], v[1]) <= r2u)) a.y = kNone;
-    else if (holds(v[0], v[1])) a = make_int2(range.x, -range.y);
-    if (!(lb(v[2], v[3]) <= r2u)) b.y = kNone;
-    else if (holds(v[2], v[3])) b = make_int2(range.z, -range.w);
+  __device__ __forceinline__ bool reaches(const float (&lo)[4 * NV],
+                                          const float (&hi)[4 * NV]) const {
+    return lb(lo, hi) <= r2u;
+  }
+  __device__ __forceinline__ bool hit(int32_t p, bool whole, double& d2) const {
+    d2 = point_d2_rec<D, PER>(tv, q, p);
+    return whole || d2 <= rr;
   }
   // The subtree that holds the ball, from a root: while the split plane is further
   // than r from the query, only its side of it can hold results.  The points left
@@ -539,7 +522,7 @@ struct BallQuery {
   // is monotone, so a point on the far side has a computed squared distance of at
   // least (split - q)^2, computed the same way.  Not for balls that may reach a
   // periodic face.
-  __device__ __forceinline__ int2 root(int32_t node, int32_t unit) const {
+  __device__ __forceinline__ int2 root(int32_t node, int32_t unit) {
     NodeMeta m = load_meta(tv.meta, node);
     while (m.left >= 0 && m.count > unit && (!PER || wf)) {
       double qa = 0.0;
@@ -555,8 +538,145 @@ struct BallQuery {
   }
 };
 
-// ------------------------------------------------------------ ball, warp per query
-// The warp keeps a stack of entries (BallQuery::expand) in depth-first order, the
+// -------------------------------------------------------- box, FP32 node tests
+// One query box against the tree.  What the reference returns is the points of the
+// closed box that its strict descent reaches (left iff lo < split, right iff
+// hi > split, :1296-1300).  The points left of a split lie at or below it and those
+// on the right at or above it, so a point strictly inside the box is reached at
+// every split above it: subtrees whose tight box lies strictly inside are taken
+// whole, subtrees whose tight box misses the closed box hold nothing, and only a
+// point on a face of the box needs its path checked (also what a NaN bound leaves).
+template <int D>
+struct BoxQuery {
+  static constexpr int kD = D;
+  static constexpr int NV = (D + 3) / 4;
+  static constexpr bool kDist = false;
+  const TreeView& tv;
+  double lo[D], hi[D];
+  float lod[D], lou[D], hid[D], hiu[D];  // the bounds rounded down / up
+  int32_t top;                           // node that the root descent reached
+
+  __device__ __forceinline__ BoxQuery(const TreeView& t, const double* __restrict__ boxes,
+                                      int64_t bi, double)
+      : tv(t) {
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      lo[j] = boxes[bi * 2 * D + 2 * j];
+      hi[j] = boxes[bi * 2 * D + 2 * j + 1];
+      lod[j] = __double2float_rd(lo[j]);
+      lou[j] = __double2float_ru(lo[j]);
+      hid[j] = __double2float_rd(hi[j]);
+      hiu[j] = __double2float_ru(hi[j]);
+    }
+  }
+  __device__ __forceinline__ bool reaches(const float (&blo)[4 * NV],
+                                          const float (&bhi)[4 * NV]) const {
+    bool out = false;
+#pragma unroll
+    for (int j = 0; j < D; ++j) out = out || bhi[j] < lod[j] || blo[j] > hiu[j];
+    return !out;
+  }
+  __device__ __forceinline__ bool holds(const float (&blo)[4 * NV],
+                                        const float (&bhi)[4 * NV]) const {
+    bool in = true;
+#pragma unroll
+    for (int j = 0; j < D; ++j) in = in && lou[j] < blo[j] && bhi[j] < hid[j];
+    return in;
+  }
+  // which sides of a node's split the strict descent visits (:1296, :1300)
+  __device__ __forceinline__ void sides(const NodeMeta& m, bool& gl, bool& gr) const {
+    double bl = 0.0, bh = 0.0;
+#pragma unroll
+    for (int j = 0; j < D; ++j)
+      if (j == m.axis) {
+        bl = lo[j];
+        bh = hi[j];
+      }
+    gl = bl < m.split;
+    gr = bh > m.split;
+  }
+  __device__ __forceinline__ int2 root(int32_t node, int32_t unit) {
+    NodeMeta m = load_meta(tv.meta, node);
+    while (m.left >= 0 && m.count > unit) {
+      bool gl, gr;
+      sides(m, gl, gr);
+      if (!gl && !gr) return make_int2(0, INT32_MIN);
+      if (gl && gr) break;
+      node = gl ? m.left : m.left + 1;
+      m = load_meta(tv.meta, node);
+    }
+    top = node;
+    return m.left < 0 || m.count <= unit ? make_int2(m.start, m.count) : make_int2(node, 0);
+  }
+  __device__ __forceinline__ bool hit(int32_t p, bool whole, double&) const {
+    if (whole) return true;
+    double v[4 * NV];
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+      const double2* r = reinterpret_cast<const double2*>(tv.pts64 + (int64_t)p * NV + h);
+      const double2 a = CKD_LDT(r), b = CKD_LDT(r + 1);
+      v[4 * h] = a.x;
+      v[4 * h + 1] = a.y;
+      v[4 * h + 2] = b.x;
+      v[4 * h + 3] = b.y;
+    }
+    bool in = true, inner = true;
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      in = in && !(v[j] < lo[j] || v[j] > hi[j]);  // :1319
+      inner = inner && lo[j] < v[j] && v[j] < hi[j];
+    }
+    if (!in || inner) return in;
+    // on a face: reached iff every split on its path is passed on its side
+    NodeMeta m = load_meta(tv.meta, top);
+    while (m.left >= 0) {
+      bool gl, gr;
+      sides(m, gl, gr);
+      const NodeMeta l = load_meta(tv.meta, m.left);
+      if (p < l.start + l.count) {
+        if (!gl) return false;
+        m = l;
+      } else {
+        if (!gr) return false;
+        m = load_meta(tv.meta, m.left + 1);
+      }
+    }
+    return true;
+  }
+};
+
+// Children of an internal node that the query reaches, as entries {node, 0},
+// {start, count} (to be tested point by point) or {start, -count} (whole);
+// y == kNone: not reached.  Subtrees of at most `unit` points come as ranges.
+constexpr int32_t kNone = INT32_MIN;
+template <class QT>
+__device__ __forceinline__ void expand(const QT& qt, int32_t node, int32_t unit, int2& a, int2& b) {
+  constexpr int NV = QT::NV;
+  const float4* rec = qt.tv.pair + (int64_t)node * pair_f4(QT::kD);
+  float v[4][4 * NV];
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+      const float4 f = CKD_LDT(rec + s * NV + h);
+      v[s][4 * h] = f.x;
+      v[s][4 * h + 1] = f.y;
+      v[s][4 * h + 2] = f.z;
+      v[s][4 * h + 3] = f.w;
+    }
+  const int4 info = CKD_LDT(reinterpret_cast<const int4*>(rec + 4 * NV));
+  const int4 range = CKD_LDT(reinterpret_cast<const int4*>(rec + 4 * NV + 1));
+  const bool ra = info.z || range.y <= unit, rb = info.w || range.w <= unit;
+  a = make_int2(ra ? range.x : info.x, ra ? range.y : 0);
+  b = make_int2(rb ? range.z : info.y, rb ? range.w : 0);
+  if (!qt.reaches(v[0], v[1])) a.y = kNone;
+  else if (qt.holds(v[0], v[1])) a = make_int2(range.x, -range.y);
+  if (!qt.reaches(v[2], v[3])) b.y = kNone;
+  else if (qt.holds(v[2], v[3])) b = make_int2(range.z, -range.w);
+}
+
+// ------------------------------------------------- ball and box, warp per query
+// The warp keeps a stack of entries (expand) in depth-first order, the
 // next one on top.  Up to 32 entries are taken at once, a lane each: nodes are
 // replaced by their reached children (left on top), so the children of many nodes
 // are tested in parallel.
@@ -580,15 +700,14 @@ constexpr int kBallListRun = 16;   // ranges that wait before they are scanned (
 constexpr int32_t kBallUnit = 32;  // subtrees of at most this many points are scanned as a range
 constexpr int32_t kBallRoot = 64;  // and of this many where the descent from the root ends
 
-template <int D, bool PER, bool FILL>
-__global__ void __launch_bounds__(128) k_ball_warp(
+template <class QT, bool FILL>
+__global__ void __launch_bounds__(128) k_range_warp(
     TreeView tv, const double* __restrict__ Q, const int32_t* __restrict__ order, int64_t nq,
     double r2, int64_t* __restrict__ counts,
     const int64_t* __restrict__ offsets, int64_t* __restrict__ oidx, double* __restrict__ odist,
     int want_d2, EmitTask* __restrict__ tasks, unsigned* __restrict__ n_tasks, unsigned task_cap,
     const int32_t* __restrict__ qroot, const unsigned* __restrict__ n_rows = nullptr) {
   constexpr unsigned FULL = 0xffffffffu;
-  using BQ = BallQuery<D, PER>;
   __shared__ int2 s_stk[4][kBallStack];
   __shared__ int2 s_list[4][FILL ? 1 : kBallList];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -601,15 +720,17 @@ __global__ void __launch_bounds__(128) k_ball_warp(
     int64_t cur = FILL ? offsets[qi] : 0;
     const int64_t cur_end = FILL ? offsets[qi + 1] : 0;
     if (FILL && cur == cur_end) continue;
-    const BQ bq(tv, Q, qi, r2);
+    QT bq(tv, Q, qi, r2);
     int64_t cnt = 0;  // per lane
     int top = 1, nl = 0;
-    if (lane == 0) stk[0] = bq.root(qroot ? qroot[qi] : 0, kBallRoot);
+    const int2 first = bq.root(qroot ? qroot[qi] : 0, kBallRoot);
+    if (first.y == kNone) top = 0;
+    if (lane == 0) stk[0] = first;
     __syncwarp();
     while (top > 0) {
       if (FILL && cur >= cur_end) break;  // all of the row's results are found
       const int n = min(min(top, 32), max(1, kBallStack - kBallReserve - top));
-      int2 e = make_int2(0, BQ::kNone);
+      int2 e = make_int2(0, kNone);
       if (lane < n) e = stk[top - 1 - lane];
       __syncwarp();
       top -= n;
@@ -622,35 +743,35 @@ __global__ void __launch_bounds__(128) k_ball_warp(
         if (big & 1u) lead = 1;
         else if (big) lead = __ffs(big) - 1;
       }
-      int2 a = make_int2(0, BQ::kNone), b = make_int2(0, BQ::kNone);
+      int2 a = make_int2(0, kNone), b = make_int2(0, kNone);
       if (lane < n && lane >= lead) {
-        if (e.y == 0) bq.expand(e.x, kBallUnit, a, b);
+        if (e.y == 0) expand(bq, e.x, kBallUnit, a, b);
         else a = e;
       }
       if (!FILL) {
-        if (a.y < 0 && a.y != BQ::kNone) {
+        if (a.y < 0 && a.y != kNone) {
           cnt -= a.y;
-          a.y = BQ::kNone;
+          a.y = kNone;
         }
-        if (b.y < 0 && b.y != BQ::kNone) {
+        if (b.y < 0 && b.y != kNone) {
           cnt -= b.y;
-          b.y = BQ::kNone;
+          b.y = kNone;
         }
         const unsigned ga = __ballot_sync(FULL, a.y > 0), gb = __ballot_sync(FULL, b.y > 0);
         const int o = nl + __popc(ga & lt) + __popc(gb & lt);
         if (a.y > 0) list[o] = a;
         if (b.y > 0) list[o + (a.y > 0 ? 1 : 0)] = b;
         nl += __popc(ga) + __popc(gb);
-        if (a.y > 0) a.y = BQ::kNone;
-        if (b.y > 0) b.y = BQ::kNone;
+        if (a.y > 0) a.y = kNone;
+        if (b.y > 0) b.y = kNone;
       }
       // back onto the stack, the first lane's entries on top, left above right
-      const unsigned ma = __ballot_sync(FULL, a.y != BQ::kNone);
-      const unsigned mb = __ballot_sync(FULL, b.y != BQ::kNone);
+      const unsigned ma = __ballot_sync(FULL, a.y != kNone);
+      const unsigned mb = __ballot_sync(FULL, b.y != kNone);
       const int total = __popc(ma) + __popc(mb);
       const int above = __popc(ma & lt) + __popc(mb & lt);
-      if (a.y != BQ::kNone) stk[top + total - 1 - above] = a;
-      if (b.y != BQ::kNone) stk[top + total - 1 - above - (a.y != BQ::kNone ? 1 : 0)] = b;
+      if (a.y != kNone) stk[top + total - 1 - above] = a;
+      if (b.y != kNone) stk[top + total - 1 - above - (a.y != kNone ? 1 : 0)] = b;
       top += total;
       __syncwarp();
       if (!FILL) {
@@ -675,7 +796,8 @@ __global__ void __launch_bounds__(128) k_ball_warp(
               if (v <= t) j += o;
             }
             const int32_t p = __shfl_sync(FULL, delta, j) + t;
-            if (t < tot && point_d2_rec<D, PER>(tv, bq.q, p) <= r2) ++cnt;
+            double d2;
+            if (t < tot && bq.hit(p, false, d2)) ++cnt;
           }
         }
         nl = 0;
@@ -730,16 +852,15 @@ __global__ void __launch_bounds__(128) k_ball_warp(
           double d2 = 0.0;
           int32_t id = 0;
           if (hit) {
-            d2 = point_d2_rec<D, PER>(tv, bq.q, p);
             id = CKD_LDT(&tv.ids[p]);
-            hit = d2 <= r2 || ((wholes >> (j & 31)) & 1u);
+            hit = bq.hit(p, (wholes >> (j & 31)) & 1u, d2);
           }
           const unsigned hm = __ballot_sync(FULL, hit);
           if (hit) {
             const int64_t o = cur + __popc(hm & lt);
             if (o < cur_end) {
               oidx[o] = id;
-              odist[o] = want_d2 ? d2 : sqrt(d2);
+              if (QT::kDist) odist[o] = want_d2 ? d2 : sqrt(d2);
             }
           }
           cur += __popc(hm);
@@ -868,184 +989,20 @@ __global__ void __launch_bounds__(128) k_box_lane(TreeView tv, const double* __r
   if (!FILL) counts[bi] = cnt;
 }
 
-// Warp-per-box search for small batches, where one lane per box would leave most
-// of the GPU idle and each box would pay one dependent load per visited node.
-// The warp expands the frontier of visited nodes one level at a time (every lane
-// tests one frontier node with the descent rule of :1296-1300, so a level costs
-// one dependent load), keeping the frontier in leaf order: children replace
-// their parent, left first, and leaves stay in place (stored as ~id).  The final
-// frontier lists the visited leaves in the order of the left-first depth-first
-// walk, so every row comes out in the reference's order.  A frontier that
-// outgrows its buffer falls back to a depth-first walk with a warp stack.
-constexpr int kBoxFront = 256;
-// Boxes per call up to which the warp kernel is used on a single tree; beyond, a lane
-// per box is faster for evenly filled boxes (2^20 boxes of side 0.005 on 2^20 uniform
-// points: 0.80 vs 4.8 ms).  Forest boxes always take the warp kernel: their trees are
-// clusters whose central boxes hold most of the points, and a lane per box leaves the
-// whole search waiting on the heaviest lanes (128k boxes on 2000 NFW trees: 25.4 vs
-// 40.8 ms, and 11.8 ms with the whole-subtree ranges above).
-constexpr int64_t kBoxWarpMax = 32768;
-
-template <int D, bool FILL>
-__global__ void __launch_bounds__(128) k_box_warp(TreeView tv, const double* __restrict__ boxes,
-                                                  int64_t nb, int64_t* __restrict__ counts,
-                                                  const int64_t* __restrict__ offsets,
-                                                  int64_t* __restrict__ oidx,
-                                                  const int32_t* __restrict__ broot) {
-  constexpr unsigned FULL = 0xffffffffu;
-  __shared__ int32_t front[4][2][kBoxFront];
-  __shared__ int32_t stk[4][kBoxLaneStack];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  const int64_t bi = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
-  if (bi >= nb) return;  // the whole warp leaves together
-  double lo[D], hi[D];
-#pragma unroll
-  for (int j = 0; j < D; ++j) {
-    lo[j] = boxes[bi * 2 * D + 2 * j];
-    hi[j] = boxes[bi * 2 * D + 2 * j + 1];
+// Copies of the recorded whole-subtree chunks of box rows, a warp per chunk.
+__global__ void __launch_bounds__(128) k_box_emit(const int32_t* __restrict__ ids,
+                                                  const EmitTask* __restrict__ tasks,
+                                                  const unsigned* __restrict__ n_tasks,
+                                                  unsigned task_cap, int64_t* __restrict__ oidx) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nt = min((int64_t)*n_tasks, (int64_t)task_cap);
+  const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < nt;
+       t += nwarps) {
+    const EmitTask e = tasks[t];
+#pragma unroll 8
+    for (int32_t i = lane; i < e.count; i += 32) oidx[e.out + i] = __ldg(&ids[e.start + i]);
   }
-  int64_t cnt = 0;
-  int64_t cur = FILL ? offsets[bi] : 0;
-  const int64_t cur_end = FILL ? offsets[bi + 1] : 0;
-  const int32_t root = broot ? broot[bi] : 0;
-  // points of one leaf, tested by the lanes and emitted in position order; a
-  // subtree inside the box (whole) is counted or emitted without the tests
-  auto scan_leaf = [&](int32_t st, int32_t ct, bool whole) {
-    if (!FILL && whole) {
-      cnt += ct;
-      return;
-    }
-    for (int32_t b = 0; b < ct; b += 32) {
-      const int32_t p = st + b + lane;
-      bool in = b + lane < ct;
-      if (in && !whole) {
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-          const double x = __ldg(&tv.pts[(int64_t)j * tv.n + p]);
-          in = in && !(x < lo[j] || x > hi[j]);  // :1319
-        }
-      }
-      const unsigned hm = __ballot_sync(FULL, in);
-      if (FILL) {
-        if (in) {
-          const int64_t o = cur + __popc(hm & lt);
-          if (o < cur_end) oidx[o] = __ldg(&tv.ids[p]);
-        }
-        cur += __popc(hm);
-      } else {
-        cnt += __popc(hm);
-      }
-    }
-  };
-  int nf = 1, fb = 0;
-  if (lane == 0) front[w][0][0] = root;
-  __syncwarp();
-  bool overflow = false;
-  for (;;) {
-    bool any = false;
-    for (int c = lane; c < nf; c += 32) any = any || front[w][fb][c] >= 0;
-    if (!__any_sync(FULL, any)) break;
-    int nn = 0;
-    for (int c0 = 0; c0 < nf; c0 += 32) {
-      const int c = c0 + lane;
-      int32_t o0 = 0, o1 = 0;
-      int kout = 0;
-      if (c < nf) {
-        const int32_t e = front[w][fb][c];
-        if (e < 0) {
-          o0 = e;
-          kout = 1;
-        } else {
-          const NodeMeta m = load_meta(tv.meta, e);
-          if (m.left < 0) {
-            o0 = ~e;
-            kout = 1;
-          } else {
-            double bl = 0.0, bh = 0.0;
-#pragma unroll
-            for (int j = 0; j < D; ++j)
-              if (j == m.axis) {
-                bl = lo[j];
-                bh = hi[j];
-              }
-            const bool gl = bl < m.split, gr = bh > m.split;  // :1296, :1300
-            if (gl && gr && m.count >= kBoxWholeMin && box_holds_node<D>(tv, e, lo, hi)) {
-              o0 = ~e;  // a subtree inside the box: scanned as one range, like a leaf
-              kout = 1;
-            } else {
-              o0 = gl ? m.left : m.left + 1;
-              o1 = m.left + 1;
-              kout = (gl ? 1 : 0) + (gr ? 1 : 0);
-            }
-          }
-        }
-      }
-      const unsigned b1 = __ballot_sync(FULL, kout >= 1), b2 = __ballot_sync(FULL, kout == 2);
-      const int pre = __popc(b1 & lt) + __popc(b2 & lt);
-      const int tot = __popc(b1) + __popc(b2);
-      if (nn + tot <= kBoxFront) {
-        if (kout >= 1) front[w][1 - fb][nn + pre] = o0;
-        if (kout == 2) front[w][1 - fb][nn + pre + 1] = o1;
-      }
-      nn += tot;
-    }
-    __syncwarp();
-    if (nn > kBoxFront) {
-      overflow = true;
-      break;
-    }
-    nf = nn;
-    fb = 1 - fb;
-  }
-  if (!overflow) {
-    for (int c0 = 0; c0 < nf; c0 += 32) {
-      int32_t st_l = 0, ct_l = 0, wh_l = 0;
-      if (c0 + lane < nf) {
-        const NodeMeta m = load_meta(tv.meta, ~front[w][fb][c0 + lane]);
-        st_l = m.start;
-        ct_l = m.count;
-        wh_l = m.left >= 0;  // an internal node in the frontier lies inside the box
-      }
-      const int nl = min(32, nf - c0);
-      for (int i = 0; i < nl; ++i)
-        scan_leaf(__shfl_sync(FULL, st_l, i), __shfl_sync(FULL, ct_l, i),
-                  __shfl_sync(FULL, wh_l, i) != 0);
-    }
-  } else {  // depth-first walk, left child first (stack depth <= tree depth + 2)
-    int top = 0;
-    if (lane == 0) stk[w][0] = root;
-    __syncwarp();
-    while (top >= 0) {
-      const int32_t node = stk[w][top];
-      --top;
-      __syncwarp();
-      const NodeMeta m = load_meta(tv.meta, node);
-      if (m.left < 0) {
-        scan_leaf(m.start, m.count, false);
-      } else {
-        double bl = 0.0, bh = 0.0;
-#pragma unroll
-        for (int j = 0; j < D; ++j)
-          if (j == m.axis) {
-            bl = lo[j];
-            bh = hi[j];
-          }
-        const bool gr = bh > m.split, gl = bl < m.split;
-        if (gl && gr && m.count >= kBoxWholeMin && box_holds_node<D>(tv, node, lo, hi)) {
-          scan_leaf(m.start, m.count, true);
-          continue;
-        }
-        if (lane == 0) {
-          if (gr) stk[w][top + 1] = m.left + 1;
-          if (gl) stk[w][top + 1 + (gr ? 1 : 0)] = m.left;
-        }
-        top += (gr ? 1 : 0) + (gl ? 1 : 0);
-        __syncwarp();
-      }
-    }
-  }
-  if (!FILL && lane == 0) counts[bi] = cnt;
 }
 
 template <int D, bool FILL>
@@ -1232,11 +1189,11 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
     const int32_t* rows = packet ? heavy : order;
     const unsigned* n_rows = packet ? cnt : nullptr;
     if (fill)
-      k_ball_warp<D, PER, true><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, nullptr, offsets, idx,
+      k_range_warp<BallQuery<D, PER>, true><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, nullptr, offsets, idx,
                                                       dist, sorted ? 1 : 0, tasks, cnt + 2,
                                                       task_cap, qroot, n_rows);
     else
-      k_ball_warp<D, PER, false><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, counts, nullptr,
+      k_range_warp<BallQuery<D, PER>, false><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, counts, nullptr,
                                                        nullptr, nullptr, 0, nullptr, nullptr, 0,
                                                        qroot, n_rows);
     CKD_LAUNCH_CHECK();
@@ -1284,18 +1241,41 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
   return CKD_OK;
 }
 
+// Boxes per call up to which the warp kernel is used on a single tree; beyond, a lane
+// per box is faster for evenly filled boxes.  Forest boxes always take the warp
+// kernel: their trees are clusters whose central boxes hold most of the points.
+constexpr int64_t kBoxWarpMax = 32768;
+
 template <int D>
 ckd_status box_launch(const ckd_tree* t, const double* boxes, int64_t nb, bool fill,
                       int64_t* counts, const int64_t* offsets, int64_t* idx, cudaStream_t s,
                       const int32_t* broot) {
   TreeView tv = t->view();
   const int threads = 128, nw = threads / 32;
-  if (t->depth < kBoxLaneStack - 2 && (nb <= kBoxWarpMax || broot) && box_warp_enabled()) {
-    const unsigned wb = (unsigned)cdiv(nb, nw);
-    if (fill)
-      k_box_warp<D, true><<<wb, threads, 0, s>>>(tv, boxes, nb, nullptr, offsets, idx, broot);
-    else
-      k_box_warp<D, false><<<wb, threads, 0, s>>>(tv, boxes, nb, counts, nullptr, nullptr, broot);
+  if (t->depth < kBallReserve - 3 && (nb <= kBoxWarpMax || broot) && box_warp_enabled()) {
+    int dev = 0, sms = 148;
+    CKD_CUDA(cudaGetDevice(&dev));
+    CKD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const unsigned wb = (unsigned)std::min<int64_t>(cdiv(nb, nw), (int64_t)sms * 16);
+    if (!fill) {
+      k_range_warp<BoxQuery<D>, false><<<wb, threads, 0, s>>>(tv, boxes, nullptr, nb, 0.0, counts,
+                                                              nullptr, nullptr, nullptr, 0, nullptr,
+                                                              nullptr, 0, broot);
+      CKD_LAUNCH_CHECK();
+      return CKD_OK;
+    }
+    Scratch sc(s);
+    const unsigned task_cap =
+        (unsigned)std::min<int64_t>(kTaskCap, std::max<int64_t>(1 << 16, nb * 64));
+    EmitTask* tasks = nullptr;  // and their counter behind them
+    CKD_CUDA(sc.alloc(&tasks, sizeof(EmitTask) * (task_cap + 1)));
+    unsigned* ntask = reinterpret_cast<unsigned*>(tasks + task_cap);
+    CKD_CUDA(cudaMemsetAsync(ntask, 0, sizeof(unsigned), s));
+    k_range_warp<BoxQuery<D>, true><<<wb, threads, 0, s>>>(tv, boxes, nullptr, nb, 0.0, nullptr,
+                                                           offsets, idx, nullptr, 0, tasks, ntask,
+                                                           task_cap, broot);
+    CKD_LAUNCH_CHECK();
+    k_box_emit<<<(unsigned)sms * 8, 128, 0, s>>>(tv.ids, tasks, ntask, task_cap, idx);
     CKD_LAUNCH_CHECK();
     return CKD_OK;
   }

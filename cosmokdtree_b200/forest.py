@@ -138,7 +138,9 @@ class Forest:
             b, bo = self._grouped(boxes, box_offsets, "boxes", 2 * self.d)
             nb = b.shape[0]
             counts = torch.empty(nb, dtype=torch.int64, device=b.device)
-            offsets = torch.zeros(nb + 1, dtype=torch.int64, device=b.device)
+            # the scan writes every entry
+            offsets = (torch.empty if nb > 0 else torch.zeros)(nb + 1, dtype=torch.int64,
+                                                                device=b.device)
             if nb > 0:
                 check(L.ckd_forest_box_count(self.handle, _ptr(b), _ptr(bo), nb, _ptr(counts),
                                              _stream()))
@@ -162,7 +164,9 @@ class Forest:
             q, qo = self._grouped(queries, query_offsets, "queries", self.d)
             nq = q.shape[0]
             counts = torch.empty(nq, dtype=torch.int64, device=q.device)
-            offsets = torch.zeros(nq + 1, dtype=torch.int64, device=q.device)
+            # the scan writes every entry
+            offsets = (torch.empty if nq > 0 else torch.zeros)(nq + 1, dtype=torch.int64,
+                                                                device=q.device)
             if nq > 0:
                 check(L.ckd_forest_ball_count(self.handle, _ptr(q), _ptr(qo), nq, radius,
                                               _ptr(counts), _stream()))

@@ -368,7 +368,9 @@ def ball_search_csr(tree: KDTree, target, radius, sorted=False):
         q, _ = _queries(tree, target)
         nq = q.shape[0]
         counts = torch.empty(nq, dtype=torch.int64, device=q.device)
-        offsets = torch.zeros(nq + 1, dtype=torch.int64, device=q.device)
+        # the scan writes every entry
+        offsets = (torch.empty if nq > 0 else torch.zeros)(nq + 1, dtype=torch.int64,
+                                                            device=q.device)
         if nq > 0:
             check(L.ckd_ball_count(tree.handle, _ptr(q), nq, radius, _ptr(counts), _stream()))
             check(L.ckd_exclusive_scan(_ptr(counts), _ptr(offsets), nq, _stream()))
@@ -409,7 +411,9 @@ def box_search_csr(tree: KDTree, boxes):
         b = b.to(f"cuda:{tree.device}").contiguous()
         nb = b.shape[0]
         counts = torch.empty(nb, dtype=torch.int64, device=b.device)
-        offsets = torch.zeros(nb + 1, dtype=torch.int64, device=b.device)
+        # the scan writes every entry
+        offsets = (torch.empty if nb > 0 else torch.zeros)(nb + 1, dtype=torch.int64,
+                                                            device=b.device)
         if nb > 0:
             check(L.ckd_box_count(tree.handle, _ptr(b), nb, _ptr(counts), _stream()))
             check(L.ckd_exclusive_scan(_ptr(counts), _ptr(offsets), nb, _stream()))
