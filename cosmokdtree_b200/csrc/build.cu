@@ -11,7 +11,12 @@
 //   scan          tile offsets
 //   k_children    n_left per node, child pairs, child cells, next open list
 //   k_scatter     stable out-of-place partition into the other buffer; points of
-//                 new leaves also land in the final leaf-ordered arrays
+//                 closed children land in the final leaf-ordered arrays
+//   k_finish      (after the levels) every closed node of more than `leaf` points:
+//                 its whole subtree by one block in shared memory
+//
+// The levels close a node at finish_max(D) points (or at `leaf`, when that is more),
+// which is what "leaf" means in their kernels.
 //
 // The working set of a level holds only the points of open nodes (more than
 // `leaf` points), compacted into SoA ping-pong buffers X[2][d][n] (stride n):
@@ -56,11 +61,13 @@ struct BuildBufs {
   double* X[2] = {nullptr, nullptr};
   int32_t* I[2] = {nullptr, nullptr};
   int32_t* NID[2] = {nullptr, nullptr};
-  // per node (capacity cap)
-  int64_t cap = 0;
+  // per node of the finished tree (capacity tcap)
+  int64_t tcap = 0;
   NodeMeta* meta = nullptr;
   double* cell = nullptr;
   double* box = nullptr;
+  // per node of the level passes (capacity cap)
+  int64_t cap = 0;
   unsigned long long* keys = nullptr;  // [cap][2d] ordered min/max keys
   int32_t* ext = nullptr;              // slide point position
   int32_t* mode = nullptr;             // 0 midpoint, 1 slide left, 2 slide right
@@ -309,6 +316,42 @@ __global__ void __launch_bounds__(kBT, 5) k_seg_box(const double* __restrict__ X
   }
 }
 
+// The split of a node with tight box [lo, hi] and cell [clo, chi]
+// (cosmokdtree.f90:347-410): axis, splitting value and mode (0 midpoint, 1 slide
+// left, 2 slide right).
+template <int D>
+__device__ __forceinline__ void split_rule(const double (&lo)[D], const double (&hi)[D],
+                                           const double (&clo)[D], const double (&chi)[D],
+                                           int& axis, double& mid, int& md) {
+  // longest cell side; exact ties go to the larger data spread (:355-365)
+  double maxside = dsub(chi[0], clo[0]);
+  double spread = dsub(hi[0], lo[0]);
+  double cl = clo[0], ch = chi[0], minx = lo[0], maxx = hi[0];
+  axis = 0;
+#pragma unroll
+  for (int j = 1; j < D; ++j) {
+    const double side = dsub(chi[j], clo[j]), sp = dsub(hi[j], lo[j]);
+    if (side > maxside || (side == maxside && sp > spread)) {
+      maxside = side;
+      spread = sp;
+      axis = j;
+      cl = clo[j];
+      ch = chi[j];
+      minx = lo[j];
+      maxx = hi[j];
+    }
+  }
+  mid = dmul(0.5, dadd(cl, ch));  // :367
+  md = 0;
+  if (minx >= mid) {  // :376
+    mid = minx;
+    md = 1;
+  } else if (maxx < mid) {  // :391
+    mid = maxx;
+    md = 2;
+  }
+}
+
 // Split decision per open node (cosmokdtree.f90:347-410).
 template <int D>
 __global__ void k_decide(const int32_t* __restrict__ act, const int4* __restrict__ st,
@@ -333,36 +376,9 @@ __global__ void k_decide(const int32_t* __restrict__ act, const int4* __restrict
     clo[j] = cell[(int64_t)a * 2 * D + 2 * j];
     chi[j] = cell[(int64_t)a * 2 * D + 2 * j + 1];
   }
-  // longest cell side; exact ties go to the larger data spread (:355-365)
-  double maxside = dsub(chi[0], clo[0]);
-  int axis = 0;
-#pragma unroll
-  for (int j = 1; j < D; ++j) {
-    double side = dsub(chi[j], clo[j]);
-    if (side > maxside) {
-      maxside = side;
-      axis = j;
-    }
-    if (side == maxside && dsub(hi[j], lo[j]) > dsub(hi[axis], lo[axis])) axis = j;
-  }
-  double cl = 0.0, ch = 0.0, minx = 0.0, maxx = 0.0;
-#pragma unroll
-  for (int j = 0; j < D; ++j)
-    if (j == axis) {
-      cl = clo[j];
-      ch = chi[j];
-      minx = lo[j];
-      maxx = hi[j];
-    }
-  double mid = dmul(0.5, dadd(cl, ch));  // :367
-  int md = 0;
-  if (minx >= mid) {  // :376
-    mid = minx;
-    md = 1;
-  } else if (maxx < mid) {  // :391
-    mid = maxx;
-    md = 2;
-  }
+  int axis, md;
+  double mid;
+  split_rule<D>(lo, hi, clo, chi, axis, mid, md);
   meta[a].split = mid;
   meta[a].axis = axis;
   mode[a] = md;
@@ -740,6 +756,327 @@ __global__ void __launch_bounds__(kBT) k_scatter(
   }
 }
 
+// ------------------------------------------------------ subtrees in shared memory
+// A node of at most finish_max(D) points leaves the level passes: its points go to
+// its range of the leaf-ordered arrays, and one block builds the rest of its subtree
+// in shared memory, with the level passes' rules (split_rule, the stable
+// partition, the first point at the extreme for a slide).  The points stay where
+// they were loaded, as ordered keys; a 16-bit permutation is partitioned, ping-pong,
+// level by level, and the points of a new leaf are written to their final place.  Nodes of more than
+// kFinBlock points are split by the whole block, the others by a warp each.  A
+// level's children take their ids from one atomic add on the node count, so
+// children follow their parents and a pair stays adjacent, but the numbering
+// below finish_max depends on the order of the blocks.
+// A level pass costs ~45 us of launches and, at 2^24 points, 104 bytes a point; this
+// replaces the last ten or so.  Whole builds before / after (us): 1000 points 559 /
+// 286, 20011 clustered 1376 / 658, 2^20 uniform 1460 / 990, 2^24 clustered 14214 /
+// 12664 (2.6 ms of it here).  Bound by issue and by waiting at the levels' barriers
+// (24 warps an SM, 47 % of issue slots): about 950 warp instructions a split node,
+// most nodes holding fewer than 40 points.  Not faster: 1024 or 512 points a block,
+// 128 or 512 threads, small subtrees queued for warps that need no barrier.
+constexpr int kFinT = 256;
+constexpr int kFinBlock = 512;
+__host__ __device__ constexpr int finish_max(int d) { return d <= 3 ? 2048 : 1024; }
+__host__ __device__ constexpr int finish_open(int m, int leaf) { return m / (leaf + 1) + 1; }
+__host__ __device__ constexpr size_t finish_smem(int d, int leaf) {
+  const size_t m = finish_max(d);
+  return m * (8 * d + 4 + 2 * 2) + 2 * (size_t)finish_open((int)m, leaf) * 8;
+}
+
+// minimum of a 64-bit key over the warp
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+  const unsigned hi = (unsigned)(k >> 32);
+  const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? (unsigned)k : 0xffffffffu);
+  return ((unsigned long long)mh << 32) | ml;
+}
+
+// nodes the level passes left: leaves of the list so far with more than `leaf` points
+__global__ void k_finish_list(const NodeMeta* __restrict__ meta, int32_t n_nodes, int leaf,
+                              int32_t* __restrict__ list, int32_t* __restrict__ n_list) {
+  const int32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= n_nodes) return;
+  if (meta[a].left < 0 && meta[a].count > leaf) list[atomicAdd(n_list, 1)] = a;
+}
+
+// ctr: {node count, deepest level + 1, error (1 node capacity, 2 depth), next list entry}
+template <int D>
+__global__ void __launch_bounds__(kFinT) k_finish(const int32_t* __restrict__ list,
+                                                  const int32_t* __restrict__ n_list,
+                                                  NodeMeta* meta, double* cell, double* box,
+                                                  double* Pf, int32_t* If, int64_t n, int leaf,
+                                                  int32_t node_cap, int32_t max_levels,
+                                                  int32_t* ctr) {
+  constexpr int M = finish_max(D), W = kFinT / 32, NP = M / kFinT;
+  static_assert(NP * W <= 64, "one warp scans the chunk counts");
+  extern __shared__ __align__(16) unsigned char fsm[];
+  unsigned long long* X = reinterpret_cast<unsigned long long*>(fsm);    // [D][M] keys
+  int32_t* I = reinterpret_cast<int32_t*>(X + (size_t)D * M);            // [M]
+  uint16_t* perm0 = reinterpret_cast<uint16_t*>(I + M);                  // [2][M]
+  const int lcap = finish_open(M, leaf);
+  int2* open = reinterpret_cast<int2*>(perm0 + 2 * M);                   // [2][lcap] {node, start | count << 16}
+  __shared__ unsigned long long red[W][2 * D];
+  __shared__ int32_t cpre[65];
+  __shared__ int32_t s_job, s_base, s_next, s_ext;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const int32_t jobs = *n_list;
+  int deepest = 0;
+  for (;;) {
+    if (tid == 0) s_job = atomicAdd(&ctr[3], 1);
+    __syncthreads();
+    const int32_t job = s_job;
+    if (job >= jobs) break;
+    const int32_t root = list[job];
+    const int32_t g0 = meta[root].start, c0 = meta[root].count;
+    int depth = meta[root].depth;
+    for (int i = tid; i < c0; i += kFinT) {
+#pragma unroll
+      for (int j = 0; j < D; ++j) X[j * M + i] = dkey(Pf[(int64_t)j * n + g0 + i]);
+      I[i] = If[g0 + i];
+      perm0[i] = (uint16_t)i;
+    }
+    if (tid == 0) open[0] = make_int2(root, c0 << 16);
+    int m = 1, cur = 0;
+    bool ok = true;
+    while (m > 0) {
+      const uint16_t* pa = perm0 + (cur ? M : 0);
+      uint16_t* pb = perm0 + (cur ? 0 : M);
+      const int2* oa = open + (cur ? lcap : 0);
+      int2* ob = open + (cur ? 0 : lcap);
+      if (tid == 0) {
+        s_base = atomicAdd(&ctr[0], 2 * m);
+        s_next = 0;
+      }
+      __syncthreads();  // also: the points, the open list and the permutation are in place
+      const int32_t base = s_base;
+      if (depth >= max_levels || base > node_cap - 2 * m) {
+        if (tid == 0) atomicMax(&ctr[2], depth >= max_levels ? 2 : 1);
+        ok = false;
+        break;  // the same for the whole block
+      }
+      // the children of open node e (node a, local start s, count c), split as told,
+      // with nl points on the left: records and the next open list
+      auto children = [&](int e, int32_t a, int s, int c, int nl, int axis, double mid,
+                          const double (&lo)[D], const double (&hi)[D], int ln) {
+        const int32_t l = base + 2 * e;
+        if (ln < 2 * D) {
+          double v = lo[0];
+#pragma unroll
+          for (int j = 0; j < D; ++j) {
+            if (ln == 2 * j) v = lo[j];
+            if (ln == 2 * j + 1) v = hi[j];
+          }
+          box[(int64_t)a * 2 * D + ln] = v;
+          double cl = cell[(int64_t)a * 2 * D + ln];
+          const bool ax = (ln >> 1) == axis;
+          cell[(int64_t)l * 2 * D + ln] = ax && (ln & 1) ? mid : cl;         // :419-422
+          cell[(int64_t)(l + 1) * 2 * D + ln] = ax && !(ln & 1) ? mid : cl;
+        }
+        if (ln < 2) {
+          NodeMeta cm;
+          cm.split = 0.0;
+          cm.left = -1;
+          cm.axis = -1;
+          cm.start = g0 + s + (ln ? nl : 0);
+          cm.count = ln ? c - nl : nl;
+          cm.depth = depth + 1;
+          cm.parent = a;
+          meta[l + ln] = cm;
+          if (cm.count > leaf) {
+            const int o = atomicAdd(&s_next, 1);
+            ob[o] = make_int2(l + ln, (s + (ln ? nl : 0)) | (cm.count << 16));
+          }
+        }
+        if (ln == 2) {
+          meta[a].split = mid;
+          meta[a].left = l;
+          meta[a].axis = axis;
+        }
+      };
+      // a point's place: in the child's segment of the other permutation, or, when
+      // the child is a leaf, in the leaf-ordered arrays
+      auto place = [&](uint16_t ix, int pos, int ccount) {
+        if (ccount > leaf) {
+          pb[pos] = ix;
+        } else {
+#pragma unroll
+          for (int j = 0; j < D; ++j) Pf[(int64_t)j * n + g0 + pos] = dkey_inv(X[j * M + ix]);
+          If[g0 + pos] = I[ix];
+        }
+      };
+      // ---- large nodes, the whole block each
+      for (int e = 0; e < m; ++e) {
+        const int32_t a = oa[e].x;
+        const int s = oa[e].y & 0xffff, c = (unsigned)oa[e].y >> 16;
+        if (c <= kFinBlock) continue;
+        unsigned long long kmn[D], kmx[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) kmn[j] = kmx[j] = ~0ull;
+        for (int i = tid; i < c; i += kFinT) {
+          const int ix = pa[s + i];
+#pragma unroll
+          for (int j = 0; j < D; ++j) {
+            const unsigned long long k = X[j * M + ix];
+            kmn[j] = k < kmn[j] ? k : kmn[j];
+            kmx[j] = ~k < kmx[j] ? ~k : kmx[j];
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          kmn[j] = warp_min_key(kmn[j]);
+          kmx[j] = warp_min_key(kmx[j]);
+          if (lane == 0) {
+            red[w][2 * j] = kmn[j];
+            red[w][2 * j + 1] = kmx[j];
+          }
+        }
+        if (tid == 0) s_ext = 0x7fffffff;
+        __syncthreads();
+        double lo[D], hi[D], clo[D], chi[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          unsigned long long a0 = red[0][2 * j], a1 = red[0][2 * j + 1];
+#pragma unroll
+          for (int x = 1; x < W; ++x) {
+            a0 = red[x][2 * j] < a0 ? red[x][2 * j] : a0;
+            a1 = red[x][2 * j + 1] < a1 ? red[x][2 * j + 1] : a1;
+          }
+          lo[j] = dkey_inv(a0);
+          hi[j] = dkey_inv(~a1);
+          clo[j] = cell[(int64_t)a * 2 * D + 2 * j];
+          chi[j] = cell[(int64_t)a * 2 * D + 2 * j + 1];
+        }
+        int axis, md;
+        double mid;
+        split_rule<D>(lo, hi, clo, chi, axis, mid, md);
+        const unsigned long long* xa = X + axis * M;
+        // the FP64 comparisons as key comparisons (the two zeros are equal)
+        const unsigned long long km = dkey(mid == 0.0 ? -0.0 : mid), wide = mid == 0.0 ? 1 : 0;
+        unsigned msk[NP];
+#pragma unroll
+        for (int it = 0; it < NP; ++it) {
+          const int i = it * kFinT + tid;
+          bool f = false;
+          if (i < c) {
+            const unsigned long long k = xa[pa[s + i]];
+            f = md == 0 ? k < km : k - km <= wide;
+            if (md != 0 && f) atomicMin(&s_ext, i);
+          }
+          msk[it] = __ballot_sync(0xffffffffu, f);
+          if (lane == 0) cpre[it * W + w] = __popc(msk[it]);
+        }
+        __syncthreads();
+        if (w == 0) {
+          const int x0 = 2 * lane < NP * W ? cpre[2 * lane] : 0;
+          const int x1 = 2 * lane + 1 < NP * W ? cpre[2 * lane + 1] : 0;
+          const int inc = warp_inclusive_scan(x0 + x1);
+          cpre[2 * lane] = inc - x0 - x1;
+          cpre[2 * lane + 1] = inc - x1;
+          if (lane == 31) cpre[64] = inc;
+        }
+        __syncthreads();
+        const int ext = s_ext;
+        const int nl = md == 0 ? cpre[64] : md == 1 ? 1 : c - 1;
+#pragma unroll
+        for (int it = 0; it < NP; ++it) {
+          const int i = it * kFinT + tid;
+          if (i >= c) continue;
+          bool f;
+          int r;  // rank in the child
+          if (md == 0) {
+            f = (msk[it] >> lane) & 1u;
+            const int lp = cpre[it * W + w] + __popc(msk[it] & lt);
+            r = f ? lp : i - lp;
+          } else {  // the slide point alone on one side, the others keep their order
+            f = (i == ext) == (md == 1);
+            r = i == ext ? 0 : i - (i > ext ? 1 : 0);
+          }
+          place(pa[s + i], s + (f ? r : nl + r), f ? nl : c - nl);
+        }
+        children(e, a, s, c, nl, axis, mid, lo, hi, tid);
+        __syncthreads();  // red, cpre and s_ext serve the next large node
+      }
+      // ---- the others, a warp each
+      for (int e = w; e < m; e += W) {
+        const int32_t a = oa[e].x;
+        const int s = oa[e].y & 0xffff, c = (unsigned)oa[e].y >> 16;
+        if (c > kFinBlock) continue;
+        double lo[D], hi[D], clo[D], chi[D];
+        {
+          unsigned long long kmn[D], kmx[D];
+#pragma unroll
+          for (int j = 0; j < D; ++j) kmn[j] = kmx[j] = ~0ull;
+          for (int i = lane; i < c; i += 32) {
+            const int ix = pa[s + i];
+#pragma unroll
+            for (int j = 0; j < D; ++j) {
+              const unsigned long long k = X[j * M + ix];
+              kmn[j] = k < kmn[j] ? k : kmn[j];
+              kmx[j] = ~k < kmx[j] ? ~k : kmx[j];
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < D; ++j) {
+            lo[j] = dkey_inv(warp_min_key(kmn[j]));
+            hi[j] = dkey_inv(~warp_min_key(kmx[j]));
+            clo[j] = cell[(int64_t)a * 2 * D + 2 * j];
+            chi[j] = cell[(int64_t)a * 2 * D + 2 * j + 1];
+          }
+        }
+        int axis, md;
+        double mid;
+        split_rule<D>(lo, hi, clo, chi, axis, mid, md);
+        const unsigned long long* xa = X + axis * M;
+        // the FP64 comparisons as key comparisons (the two zeros are equal)
+        const unsigned long long km = dkey(mid == 0.0 ? -0.0 : mid), wide = mid == 0.0 ? 1 : 0;
+        int nl = 0, ext = -1;
+        for (int b = 0; b < c; b += 32) {
+          bool f = false;
+          if (b + lane < c) {
+            const unsigned long long k = xa[pa[s + b + lane]];
+            f = md == 0 ? k < km : k - km <= wide;
+          }
+          const unsigned fm = __ballot_sync(0xffffffffu, f);
+          if (md == 0) {
+            nl += __popc(fm);
+          } else if (fm) {
+            ext = b + __ffs(fm) - 1;
+            break;
+          }
+        }
+        if (md != 0) nl = md == 1 ? 1 : c - 1;
+        int lp = 0;  // left points before this chunk
+        for (int b = 0; b < c; b += 32) {
+          const int i = b + lane;
+          const uint16_t ix = i < c ? pa[s + i] : (uint16_t)0;
+          bool f = false;
+          int r = 0;
+          if (md == 0) {
+            f = i < c && xa[ix] < km;
+            const unsigned fm = __ballot_sync(0xffffffffu, f);
+            r = f ? lp + __popc(fm & lt) : i - lp - __popc(fm & lt);
+            lp += __popc(fm);
+          } else {
+            f = (i == ext) == (md == 1);
+            r = i == ext ? 0 : i - (i > ext ? 1 : 0);
+          }
+          if (i < c) place(ix, s + (f ? r : nl + r), f ? nl : c - nl);
+        }
+        children(e, a, s, c, nl, axis, mid, lo, hi, lane);
+      }
+      ++depth;
+      __syncthreads();
+      m = s_next;
+      cur ^= 1;
+      __syncthreads();  // s_next is read before the next level clears it
+    }
+    if (ok) deepest = max(deepest, depth);
+    __syncthreads();  // s_job and the shared arrays serve the next subtree
+  }
+  if (tid == 0) atomicMax(&ctr[1], deepest);
+}
+
 // bounding boxes of the leaves from the final leaf-ordered points
 template <int D>
 __global__ void k_leaf_box(const NodeMeta* __restrict__ meta, int32_t n_nodes, int leaf,
@@ -896,13 +1233,22 @@ cudaError_t grow(T** p, int64_t old_n, int64_t new_n, cudaStream_t s) {
   return cudaSuccess;
 }
 
+ckd_status ensure_tree_cap(BuildBufs& B, int64_t need, cudaStream_t s) {
+  if (need <= B.tcap) return CKD_OK;
+  int64_t nc = std::max<int64_t>(need, B.tcap * 2);
+  int d2 = 2 * B.d;
+  CKD_CUDA(grow(&B.meta, B.tcap, nc, s));
+  CKD_CUDA(grow(&B.cell, B.tcap * d2, nc * d2, s));
+  CKD_CUDA(grow(&B.box, B.tcap * d2, nc * d2, s));
+  B.tcap = nc;
+  return CKD_OK;
+}
+
 ckd_status ensure_node_cap(BuildBufs& B, int64_t need, cudaStream_t s) {
+  CKD_TRY(ensure_tree_cap(B, need, s));
   if (need <= B.cap) return CKD_OK;
   int64_t nc = std::max<int64_t>(need, B.cap * 2);
   int d2 = 2 * B.d;
-  CKD_CUDA(grow(&B.meta, B.cap, nc, s));
-  CKD_CUDA(grow(&B.cell, B.cap * d2, nc * d2, s));
-  CKD_CUDA(grow(&B.box, B.cap * d2, nc * d2, s));
   CKD_CUDA(grow(&B.keys, B.cap * d2, nc * d2, s));
   CKD_CUDA(grow(&B.ext, B.cap, nc, s));
   CKD_CUDA(grow(&B.mode, B.cap, nc, s));
@@ -927,10 +1273,17 @@ void free_bufs(BuildBufs& B, cudaStream_t s) {
   B = BuildBufs();
 }
 
+// node_cap: capacity of the node arrays for the subtrees finished in shared memory;
+// 0 takes four nodes per full leaf.  When the tree needs more, *again is set and the
+// caller builds once more with the largest count a tree can have.
 template <int D>
-ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t s) {
+ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t s,
+                      int64_t node_cap, bool* again) {
   const int64_t n = t->n;
-  const int leaf = t->leaf;
+  // the level passes end at nodes that a block finishes in shared memory
+  const int tree_leaf = t->leaf;
+  const bool finish = tree_leaf < finish_max(D);
+  const int leaf = finish ? finish_max(D) : tree_leaf;
   BuildBufs B;
   B.d = D;
   B.n = n;
@@ -982,7 +1335,11 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   double* Ldev = nullptr;
   CKD_CUDA(sc.alloc(&Ldev, sizeof(double) * CKD_MAX_D));
   CKD_CUDA(cudaMemcpyAsync(Ldev, t->L, sizeof(double) * CKD_MAX_D, cudaMemcpyHostToDevice, s));
-  CKD_TRY(ensure_node_cap(B, (int64_t)T + std::max<int64_t>(64, 4 * (n / std::max(1, leaf)) + 64), s));
+  CKD_TRY(ensure_tree_cap(
+      B, node_cap > 0 ? node_cap
+                      : (int64_t)T + std::min<int64_t>(2 * n, 4 * (n / tree_leaf) + 64),
+      s));
+  CKD_TRY(ensure_node_cap(B, (int64_t)T + 4 * (n / leaf) + 64, s));
   k_root_init<D><<<(unsigned)cdiv(T, 128), 128, 0, s>>>(B.meta, B.cell, B.keys, off_dev, T, Ldev,
                                                         t->periodic);
   CKD_LAUNCH_CHECK();
@@ -1138,7 +1495,39 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   int32_t err = 0;
   CKD_CUDA(cudaMemcpyAsync(&err, B.scal + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
 
-  k_leaf_box<D><<<(unsigned)cdiv(n_nodes, 128), 128, 0, s>>>(B.meta, n_nodes, leaf, t->pts, n,
+  if (finish) {
+    int32_t *list = nullptr, *ctr = nullptr;  // ctr[4]: entries of the list
+    CKD_CUDA(sc.alloc(&list, sizeof(int32_t) * n_nodes));
+    CKD_CUDA(sc.alloc(&ctr, sizeof(int32_t) * 5));
+    int32_t h[5] = {n_nodes, depth_levels, 0, 0, 0};
+    CKD_CUDA(cudaMemcpyAsync(ctr, h, sizeof(h), cudaMemcpyHostToDevice, s));
+    k_finish_list<<<(unsigned)cdiv(n_nodes, 256), 256, 0, s>>>(B.meta, n_nodes, tree_leaf, list,
+                                                               ctr + 4);
+    CKD_LAUNCH_CHECK();
+    int dev = 0, sms = 148, per_sm = 1;
+    CKD_CUDA(cudaGetDevice(&dev));
+    CKD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const size_t sm = finish_smem(D, tree_leaf);
+    CKD_CUDA(cudaFuncSetAttribute(k_finish<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sm));
+    CKD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_finish<D>, kFinT, sm));
+    const int64_t g = std::min<int64_t>(n_nodes, (int64_t)sms * std::max(1, per_sm));
+    k_finish<D><<<(unsigned)g, kFinT, sm, s>>>(
+        list, ctr + 4, B.meta, B.cell, B.box, t->pts, t->ids, n, tree_leaf,
+        (int32_t)std::min<int64_t>(B.tcap, INT32_MAX), kMaxLevels, ctr);
+    CKD_LAUNCH_CHECK();
+    CKD_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
+    CKD_CUDA(cudaStreamSynchronize(s));
+    if (h[2] == 2)
+      return fail(CKD_ERR_DEPTH, "tree depth exceeds the build's level cap (8192 levels)");
+    if (h[2] == 1) {
+      *again = true;
+      return CKD_OK;
+    }
+    n_nodes = h[0];
+    depth_levels = std::max(depth_levels, (int)h[1]);
+  }
+  k_leaf_box<D><<<(unsigned)cdiv(n_nodes, 128), 128, 0, s>>>(B.meta, n_nodes, tree_leaf, t->pts, n,
                                                              B.box);
   CKD_LAUNCH_CHECK();
   t->n_nodes = n_nodes;
@@ -1185,16 +1574,25 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
 }  // namespace
 
 ckd_status build_dispatch(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t s) {
-  switch (t->d) {
-    case 1: return build_impl<1>(t, pts_dev, dtype, s);
-    case 2: return build_impl<2>(t, pts_dev, dtype, s);
-    case 3: return build_impl<3>(t, pts_dev, dtype, s);
-    case 4: return build_impl<4>(t, pts_dev, dtype, s);
-    case 5: return build_impl<5>(t, pts_dev, dtype, s);
-    case 6: return build_impl<6>(t, pts_dev, dtype, s);
-    case 7: return build_impl<7>(t, pts_dev, dtype, s);
-    case 8: return build_impl<8>(t, pts_dev, dtype, s);
-    default: return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
+  bool again = false;
+  int64_t cap = 0;
+  for (;;) {
+    ckd_status st = CKD_OK;
+    switch (t->d) {
+#define CKD_BD(DD) \
+  case DD: st = build_impl<DD>(t, pts_dev, dtype, s, cap, &again); break;
+      CKD_BD(1) CKD_BD(2) CKD_BD(3) CKD_BD(4) CKD_BD(5) CKD_BD(6) CKD_BD(7) CKD_BD(8)
+#undef CKD_BD
+      default: return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
+    }
+    if (st != CKD_OK || !again) return st;
+    // more nodes than planned: once more with room for every tree of these points
+    again = false;
+    cap = t->n_trees + 2 * t->n;
+    dev_free(t->pts, s);
+    dev_free(t->ids, s);
+    t->pts = nullptr;
+    t->ids = nullptr;
   }
 }
 
