@@ -16,7 +16,6 @@
 // union of the lanes' paths with a per-entry lane mask, left first, so every
 // row comes out in the reference's order.
 #include <algorithm>
-#include <cmath>
 
 #include "ckd_common.cuh"
 #include "ckd_knn.cuh"
@@ -1121,10 +1120,6 @@ constexpr int64_t kBallWarpMax = 200000;
 constexpr int kPacketBudget = 512;
 constexpr int64_t kPacketRow = 64;
 bool ball_warp_ok(const ckd_tree* t) { return t->screen_ok && t->depth < kBallReserve - 3; }
-// uneven density: a tree much deeper than its leaf count needs
-bool uneven(const ckd_tree* t) {
-  return t->depth > 1.5 * std::log2((double)t->n / t->leaf + 2.0);
-}
 
 template <int D, bool PER>
 ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
@@ -1160,7 +1155,7 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
           offsets, order, nq, warp ? kPacketRow : kHeavyRow, heavy, cnt, light, cnt + 1);
       CKD_LAUNCH_CHECK();
     }
-    int32_t* bail = warp && uneven(t) && nq * 2 <= t->n ? heavy : nullptr;
+    int32_t* bail = warp && tree_uneven(t) && nq * 2 <= t->n ? heavy : nullptr;
     const int w2 = sorted ? 1 : 0;
     if (fill && qroot)
       k_ball<D, PER, true, true><<<blocks, threads, 0, s>>>(
@@ -1318,7 +1313,7 @@ ckd_status query_order_roots(const ckd_tree* t, const double* q, int64_t nq, int
 // points 611 against 533, the ordering included).
 bool want_ball_order(const ckd_tree* t, int64_t nq) {
   if (query_order_mode() != 0 || nq > kBallWarpMax || !ball_warp_ok(t)) return want_order(t, nq);
-  return nq >= 50000 && uneven(t) && want_order(t, nq);
+  return nq >= 50000 && tree_uneven(t) && want_order(t, nq);
 }
 
 ckd_status ball_run(const ckd_tree* t, const double* q, int64_t nq, double r, bool fill, int sorted,

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <cfloat>
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -275,3 +276,11 @@ struct ckd_tree {
     return v;
   }
 };
+
+namespace ckd {
+// uneven density: a tree much deeper than its leaf count needs (2^22 points, leaf 16:
+// depth 20 uniform, 52 clustered)
+inline bool tree_uneven(const ckd_tree* t) {
+  return t->depth > 1.5 * std::log2((double)t->n / t->leaf + 2.0);
+}
+}  // namespace ckd

@@ -20,9 +20,12 @@
 
 namespace ckd {
 
-// a warp per query (knn_warp.cu): sorted rows, k <= 128
-ckd_status knn_warp(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq, int k,
-                    double* dist, int64_t* idx, const int32_t* qroot, cudaStream_t s);
+// a group of lanes per query (ckd_knn_group.cuh): sorted rows, k <= 128
+#define CKD_KG(DD)                                                                            \
+  ckd_status knn_group_d##DD(const ckd_tree*, const double*, const int32_t*, int64_t, int,    \
+                             double*, int64_t*, const int32_t*, cudaStream_t);
+CKD_KG(1) CKD_KG(2) CKD_KG(3) CKD_KG(4) CKD_KG(5) CKD_KG(6) CKD_KG(7) CKD_KG(8)
+#undef CKD_KG
 
 namespace {
 
@@ -311,30 +314,44 @@ __global__ void k_bucket_scatter(const int32_t* __restrict__ key, int64_t nq,
   order[pos] = (int32_t)i;
 }
 
-// Whether the automatic choice takes a warp per query (knn_warp.cu) instead of the
-// per-lane kernel.  Sorted rows only: an unsorted row is in the order of its
-// kernel's heap.  The lines are where the two cross, measured on 2^20 uniform,
-// 2^22 clustered and 2^22 6-D points (us a call, per-lane / warp):
-//   k = 16: 50k queries 323 / 266, 100k 359 / 515 (uniform 3-D)
-//   k = 32: 100k 1207 / 1113, 200k 1733 / 1925 (clustered 3-D)
-//   k = 48: 400k 3146 / 2947, 1M 6594 / 7224 (uniform 3-D)
-//   k = 64: 100k 2723 / 1272, 1M 14376 / 10003 (clustered 3-D): always the warp
-//   k = 16, 6-D: 200k 4542 / 3819, 400k 7089 / 7344;  k >= 48, 6-D: always the warp
+ckd_status knn_group(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq, int k,
+                     double* dist, int64_t* idx, const int32_t* qroot, cudaStream_t s) {
+  switch (t->d) {
+#define CKD_KG(DD) \
+  case DD: return knn_group_d##DD(t, q, order, nq, k, dist, idx, qroot, s);
+    CKD_KG(1) CKD_KG(2) CKD_KG(3) CKD_KG(4) CKD_KG(5) CKD_KG(6) CKD_KG(7) CKD_KG(8)
+#undef CKD_KG
+  }
+  return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
+}
+
+// Whether the automatic choice takes a group of lanes per query
+// (ckd_knn_group.cuh) instead of the per-lane kernel.  Sorted rows only: an unsorted
+// row is in the order of its kernel's heap.  The lines are where the two cross,
+// measured on 2^20 uniform, 2^22 clustered and 2^22 6-D points (us a call, per-lane /
+// groups):
+//   k = 8: 150k queries 406 / 375, 200k 427 / 471 (uniform), 857 / 831 (clustered)
+//   k = 16: 50k 316 / 206, 100k 359 / 376 (uniform), 300k 1389 / 1375 (clustered)
+//   k = 32: 300k 1287 / 1319 (uniform), 2148 / 1935, 500k 2915 / 2992 (clustered)
+//   k = 48: 400k 3146 / 2947, 1M 6594 / 7224 (uniform)
+//   k = 64: 100k 2723 / 1232, 1M 14376 / 9726 (clustered): always groups
+//   k = 16, 6-D: 200k 4505 / 3687, 400k 7089 / 7344;  k >= 48, 6-D: always groups
 //   k = 100: 30k 16414 / 810 (against the packet kernel in the output rows)
-bool use_knn_warp(const ckd_tree* t, int64_t nq, int k, int sorted) {
+bool use_knn_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
   if (!sorted || k > 128 || !t->screen_ok || t->depth >= kLaneStack - 1 || knn_variant() != 0 ||
       g_stats_on)
     return false;
   if (t->d <= 4) {
-    if (k <= 32) return nq <= 32768 + 2200 * (int64_t)k;
-    return k >= 64 || nq <= 500000;
+    if (k <= 8) return nq <= 180000;
+    if (k <= 16) return nq <= (tree_uneven(t) ? 180000 : 90000);
+    return k >= 64 || nq <= (k <= 32 ? 300000 : 500000);
   }
   return k >= 48 || nq <= 32768 + 20000 * (int64_t)k;
 }
 
 // Kernel choice (ckd_set_knn_variant): 0 automatic, 1 FP64 packet traversal,
 // 7 per-lane compact heap, 8 the same expanding nodes from child-pair records.
-// Automatic takes a warp per query where use_knn_warp says so, else 8; trees too
+// Automatic takes a group of lanes per query where use_knn_group says so, else 8; trees too
 // deep for their stacks, coordinates beyond the FP32 screen's range, unsorted
 // rows of k > 64 and k > 128 take the packet kernel.
 template <int D, bool PER>
@@ -351,7 +368,7 @@ ckd_status knn_launch(const ckd_tree* t, const double* q, const int32_t* order, 
       if (on) timing_end(s);
     }
   } timing_guard{s, force_variant < 0};
-  if (use_knn_warp(t, nq, k, sorted)) return knn_warp(t, q, order, nq, k, dist, idx, nullptr, s);
+  if (use_knn_group(t, nq, k, sorted)) return knn_group(t, q, order, nq, k, dist, idx, nullptr, s);
   if (k <= kSmemK && t->screen_ok && var != 1 && t->depth < kLaneStack - 1) {
     const int nw7 = std::min(4, knn_warps_per_block());
     const unsigned blocks7 = (unsigned)cdiv(cdiv(nq, 32), nw7);
@@ -473,15 +490,17 @@ ckd_status query_order_roots(const ckd_tree* t, const double* q, int64_t nq, int
   return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
 }
 
-// Queries of the warp-per-query kernel gain from leaf order through L1 and L2
-// alone, so it pays later than for the per-lane kernel: at 100k queries in 3-D
-// (k = 16: 988 ordered, 1001 us in the caller's order; 50k: 619 / 566), at 25k in
-// 6-D, where a query reads many leaves (k = 8: 587 / 615 us; k = 1: 197 / 117).
-bool want_order_warp(const ckd_tree* t, int64_t nq, int k) {
+// Queries of the group kernel gain from leaf order through L1 and L2 alone, so it
+// pays later than for the per-lane kernel (us, caller's order / ordered): 3-D, k = 16:
+// 50k 416 / 466, 100k 701 / 663 (2^22 clustered points), k = 8: 150k 471 / 481, 200k
+// 618 / 612 (2^20 uniform); 6-D, where a query reads many leaves: 25k, k = 8: 615 / 587,
+// k = 1: 117 / 197.
+bool want_order_group(const ckd_tree* t, int64_t nq, int k) {
   const int mode = query_order_mode();
   if (mode != 0) return mode == 1 && nq > 1;
   if (nq * 8 < t->n / 64) return false;
-  return t->d <= 4 ? nq >= 100000 : nq * std::min(k, 4) >= 100000;
+  return t->d <= 4 ? nq >= 100000 && nq * std::min(k, 16) >= 1600000
+                   : nq * std::min(k, 4) >= 100000;
 }
 
 // Queries are ordered by leaf when there are enough of them to fill many warps.
@@ -512,7 +531,7 @@ ckd_status knn_run(const ckd_tree* t, const double* q, int64_t nq, int k, int so
                    int64_t* idx, cudaStream_t s) {
   Scratch sc(s);
   int32_t* order = nullptr;
-  if (use_knn_warp(t, nq, k, sorted) ? want_order_warp(t, nq, k) : want_order(t, nq)) {
+  if (use_knn_group(t, nq, k, sorted) ? want_order_group(t, nq, k) : want_order(t, nq)) {
     CKD_CUDA(sc.alloc(&order, sizeof(int32_t) * nq));
     CKD_TRY(query_order(t, q, nq, order, s));
   }
@@ -530,14 +549,14 @@ ckd_status forest_knn_impl(const ckd_tree* t, const double* q, const int32_t* qr
                            int k, int sorted, double* dist, int64_t* idx, cudaStream_t s) {
   Scratch sc(s);
   int32_t* order = nullptr;
-  const bool warp = use_knn_warp(t, nq, k, sorted);
-  if (!warp || want_order_warp(t, nq, k)) {
+  const bool warp = use_knn_group(t, nq, k, sorted);
+  if (!warp || want_order_group(t, nq, k)) {
     CKD_CUDA(sc.alloc(&order, sizeof(int32_t) * nq));
     CKD_TRY(order_impl<D>(t, q, nq, order, nullptr, s, nullptr, qroot));
   }
   timing_begin(s);
   if (warp) {
-    CKD_TRY(knn_warp(t, q, order, nq, k, dist, idx, qroot, s));
+    CKD_TRY(knn_group(t, q, order, nq, k, dist, idx, qroot, s));
     timing_end(s);
     return CKD_OK;
   }

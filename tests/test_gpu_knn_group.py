@@ -1,5 +1,6 @@
-"""The warp-per-query kNN kernel (sorted rows, k <= 128) against the oracle, at the edges of
-its register lists (k around 32, 64 and 128), its scan units and its dispatch.  Ids and FP64
+"""The kNN kernel with a group of lanes per query (sorted rows, k <= 128) against the oracle,
+at the edges of its register lists (k around 8, 16, 32, 64 and 128), its scan units and its
+dispatch.  Ids and FP64
 distances are compared for equality: both sides round every product and sum separately."""
 import numpy as np
 import pytest
@@ -33,7 +34,7 @@ CASES = [
 
 @pytest.mark.parametrize("order", [1, 2], ids=["leaf_order", "caller_order"])
 @pytest.mark.parametrize("name,n,d,periodic,leaf,nq,k", CASES)
-def test_gpu_knn_warp_matches_oracle(gpu, oracle, name, n, d, periodic, leaf, nq, k, order):
+def test_gpu_knn_group_matches_oracle(gpu, oracle, name, n, d, periodic, leaf, nq, k, order):
     from cosmokdtree_b200 import _lib
     L = _lib.load()
     P = make_points(name, n, d, periodic)
@@ -55,7 +56,7 @@ def test_gpu_knn_warp_matches_oracle(gpu, oracle, name, n, d, periodic, leaf, nq
 
 
 @pytest.mark.parametrize("k", [1, 33, 64])
-def test_gpu_knn_warp_forest(gpu, oracle, k):
+def test_gpu_knn_group_forest(gpu, oracle, k):
     rng = np.random.default_rng(23)
     parts = [rng.random((n, 3)) - 0.5 for n in (1, 16, 17, 700, 4000)]
     qs = [rng.random((m, 3)) - 0.5 for m in (2, 1, 3, 40, 1)]
@@ -68,19 +69,42 @@ def test_gpu_knn_warp_forest(gpu, oracle, k):
         np.testing.assert_array_equal(d[qoff[t]:qoff[t + 1]].cpu().numpy(), od)
 
 
-@pytest.mark.parametrize("nq", [32768 + 2200 * 16, 32768 + 2200 * 16 + 1])
-def test_gpu_knn_warp_at_its_dispatch_line(gpu, nq):
-    """Both sides of the rule that chooses the kernel give the rows of the per-lane kernel."""
+@pytest.mark.parametrize("nq,k", [
+    (4000, 8), (4001, 8), (9000, 8), (9001, 8), (9001, 7), (4001, 9), (9001, 16), (75000, 16),
+    (75001, 16), (75001, 8), (4001, 17), (4001, 32), (75001, 32), (9001, 33), (180000, 1),
+    (180001, 1), (90000, 16), (90001, 16), (300000, 17), (300001, 32), (100000, 100),
+])
+@pytest.mark.parametrize("name,d,periodic", [("uniform3d", 3, False), ("lattice_periodic", 3, True)])
+def test_gpu_knn_group_at_its_dispatch_lines(gpu, nq, k, name, d, periodic):
+    """Both sides of the rules that choose the kernel and its lanes per query give the rows of
+    the per-lane (k <= 64) or packet kernel."""
     from cosmokdtree_b200 import _lib
     L = _lib.load()
+    P = make_points(name, 30011, d, periodic)
     rng = np.random.default_rng(29)
-    t = gpu.kdtree.build_kdtree(rng.random((30011, 3)))
-    q = rng.random((nq, 3))
-    d, i = gpu.kdtree.knn_search(t, q, 16)
-    _lib.check(L.ckd_set_knn_variant(8))
+    t = gpu.kdtree.build_kdtree(P, boxsize=1.0 if periodic else None)
+    q = np.concatenate([P[rng.integers(0, len(P), nq // 2)],
+                        rng.random((nq - nq // 2, d)) - (0.5 if periodic else 0.0)])
+    gd, gi = gpu.kdtree.knn_search(t, q, k)
+    _lib.check(L.ckd_set_knn_variant(8 if k <= 64 else 1))
     try:
-        ld, li = gpu.kdtree.knn_search(t, q, 16)
+        ld, li = gpu.kdtree.knn_search(t, q, k)
     finally:
         _lib.check(L.ckd_set_knn_variant(0))
-    np.testing.assert_array_equal(i, li)
-    np.testing.assert_array_equal(d, ld)
+    np.testing.assert_array_equal(gi, li)
+    np.testing.assert_array_equal(gd, ld)
+
+
+@pytest.mark.parametrize("d,leaf", [(1, 16), (2, 1), (3, 50), (4, 16)])
+@pytest.mark.parametrize("k", [3, 8, 13, 30])
+def test_gpu_knn_group_narrow_groups(gpu, oracle, d, leaf, k):
+    """8 and 16 lanes per query in every dimension that uses them."""
+    P = make_points("periodic_clustered", 9000, d, True)
+    rng = np.random.default_rng(31)
+    q = np.concatenate([P[rng.integers(0, 9000, 5000)], rng.random((5003, d)) - 0.5])
+    t = gpu.kdtree.build_kdtree(P, leaf=leaf, boxsize=1.0)
+    od, oi = oracle.OracleTree(P, leaf, 1.0).knn(q, k)
+    for part in (slice(0, None), slice(0, 4501)):
+        gd, gi = gpu.kdtree.knn_search(t, q[part], k)
+        np.testing.assert_array_equal(gi, oi[part])
+        np.testing.assert_array_equal(gd, od[part])
