@@ -175,8 +175,13 @@ static void release_tree(ckd_tree* t) {
   cudaDeviceSynchronize();
   void* ps[] = {t->meta, t->box,   t->cell, t->pts,    t->ids,   t->box32,
                 t->pts32, t->pts64, t->pair, t->cell32, t->centre};
-  for (void* p : ps)
-    if (p) cudaFreeAsync(p, 0);
+  if (t->block[0] || t->block[1]) {
+    for (void* p : t->block)
+      if (p) cudaFreeAsync(p, 0);
+  } else {
+    for (void* p : ps)
+      if (p) cudaFreeAsync(p, 0);
+  }
   delete t;
 }
 

@@ -58,6 +58,12 @@ struct __align__(16) FlagRec {
 struct BuildBufs {
   int d = 0;
   int64_t n = 0;
+  // one block holds every buffer below; only arrays that had to grow leave it
+  char* arena = nullptr;
+  size_t arena_bytes = 0;
+  bool owns(const void* p) const {
+    return p && !(static_cast<const char*>(p) >= arena && static_cast<const char*>(p) < arena + arena_bytes);
+  }
   double* X[2] = {nullptr, nullptr};
   int32_t* I[2] = {nullptr, nullptr};
   int32_t* NID[2] = {nullptr, nullptr};
@@ -510,46 +516,29 @@ __global__ void __launch_bounds__(kBT) k_flags(const double* __restrict__ X,
   if (threadIdx.x == 0) tile_sum[blockIdx.x] = tot;
 }
 
-// n_left, child pairs and cells; counts the next open list and its working
-// points (cosmokdtree.f90:412-448)
+// One open node's left count and its children's records (cosmokdtree.f90:412-448);
+// returns the left count and leaves the node's prefix base in P0.
 template <int D>
-__global__ void k_children(const int32_t* __restrict__ act, const int4* __restrict__ st, int mb,
-                           NodeMeta* __restrict__ meta,
-                           double* __restrict__ cell, const int32_t* __restrict__ pstart,
-                           const int32_t* __restrict__ pend, const int32_t* __restrict__ tile_off,
-                           const int32_t* __restrict__ wst, const int32_t* __restrict__ mode,
-                           const int32_t* __restrict__ ext, int32_t* __restrict__ nleft,
-                           int32_t* __restrict__ pbase, unsigned long long* __restrict__ keys,
-                           int leaf, int64_t* __restrict__ nxt_cnt, int32_t* __restrict__ err) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int m = st->x;
-  const int32_t first_child = st->z;
-  if (i >= m) {  // zeros up to the launch bound, so the scan over mb entries is exact
-    if (i < mb) nxt_cnt[i] = 0;
-    return;
-  }
-  int32_t a = act[i];
-  NodeMeta pm = meta[a];
-  const int md = mode[a];
-  int32_t nl, P0 = 0;
+__device__ __forceinline__ int32_t make_children(
+    int32_t a, int32_t c0, const NodeMeta& pm, NodeMeta* meta, double* cell,
+    const int32_t* __restrict__ pstart, const int32_t* __restrict__ pend, const int32_t* tile_off,
+    int32_t w0, int md, int32_t ext, unsigned long long* __restrict__ keys, int32_t* err,
+    int32_t& P0) {
+  int32_t nl;
+  P0 = 0;
   if (md == 0) {
-    int64_t s = wst[a], e = (int64_t)wst[a] + pm.count - 1;
+    int64_t s = w0, e = (int64_t)w0 + pm.count - 1;
     P0 = tile_off[s / kTile] + pstart[a];
-    int32_t P1 = tile_off[e / kTile] + pend[a];
-    nl = P1 - P0;
+    nl = tile_off[e / kTile] + pend[a] - P0;
   } else {
     nl = md == 1 ? 1 : pm.count - 1;
-    if (ext[a] == 0x7fffffff) nl = 0;  // no slide point found: flagged below
+    if (ext == 0x7fffffff) nl = 0;  // no slide point found: flagged below
   }
   if (nl <= 0 || nl >= pm.count) {  // cannot happen for a valid sliding-midpoint split
     atomicExch(err, 1);
     nl = nl <= 0 ? 1 : pm.count - 1;
   }
-  nleft[a] = nl;
-  pbase[a] = P0;
-  int32_t c0 = first_child + 2 * i;
   meta[a].left = c0;
-  int cnt = 0, pts = 0;
   for (int side = 0; side < 2; ++side) {
     int32_t c = c0 + side;
     NodeMeta cm;
@@ -573,12 +562,121 @@ __global__ void k_children(const int32_t* __restrict__ act, const int4* __restri
       keys[(int64_t)c * 2 * D + 2 * j] = ~0ull;
       keys[(int64_t)c * 2 * D + 2 * j + 1] = 0ull;
     }
-    if (cm.count > leaf) {
-      ++cnt;
-      pts += cm.count;
+  }
+  return nl;
+}
+
+// n_left, child pairs and cells; counts the next open list and its working points
+template <int D>
+__global__ void k_children(const int32_t* __restrict__ act, const int4* __restrict__ st, int mb,
+                           NodeMeta* __restrict__ meta,
+                           double* __restrict__ cell, const int32_t* __restrict__ pstart,
+                           const int32_t* __restrict__ pend, const int32_t* __restrict__ tile_off,
+                           const int32_t* __restrict__ wst, const int32_t* __restrict__ mode,
+                           const int32_t* __restrict__ ext, int32_t* __restrict__ nleft,
+                           int32_t* __restrict__ pbase, unsigned long long* __restrict__ keys,
+                           int leaf, int64_t* __restrict__ nxt_cnt, int32_t* __restrict__ err) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int m = st->x;
+  if (i >= m) {  // zeros up to the launch bound, so the scan over mb entries is exact
+    if (i < mb) nxt_cnt[i] = 0;
+    return;
+  }
+  const int32_t a = act[i];
+  const NodeMeta pm = meta[a];
+  int32_t P0;
+  const int32_t nl = make_children<D>(a, st->z + 2 * i, pm, meta, cell, pstart, pend, tile_off,
+                                      wst[a], mode[a], ext[a], keys, err, P0);
+  nleft[a] = nl;
+  pbase[a] = P0;
+  const int nr = pm.count - nl;
+  const int cnt = (nl > leaf ? 1 : 0) + (nr > leaf ? 1 : 0);
+  const int pts = (nl > leaf ? nl : 0) + (nr > leaf ? nr : 0);
+  nxt_cnt[i] = ((int64_t)cnt << 32) | (int64_t)pts;
+}
+
+// The node work of a level between the flags and the scatter, by one block: the scan
+// of the tiles' left counts, the children, the next open list, its working starts
+// and the scatter records.  With at most a few thousand open nodes five launches of
+// almost idle kernels (24 us and their gaps) cost more than one busy block (with the
+// records of the tree written by two kernels and one block of memory for all of the
+// build: 20011 clustered points 658 -> 573 us, 2^24 12.66 -> 12.24 ms); past kNodesMax
+// nodes the parallel kernels are taken.
+constexpr int kNodesT = 1024;
+constexpr int kNodesMax = 4096;      // open nodes of a level (its launch bound)
+constexpr unsigned kNodesTiles = 32768;
+template <int D>
+__global__ void __launch_bounds__(kNodesT) k_level_nodes(
+    const int32_t* __restrict__ act, const int4* __restrict__ st, int4* __restrict__ st_next,
+    int ntw, NodeMeta* meta, double* cell, const int32_t* __restrict__ pstart,
+    const int32_t* __restrict__ pend, const int32_t* __restrict__ tile_sum, int32_t* tile_off,
+    int32_t* wst, const int32_t* __restrict__ mode, const int32_t* __restrict__ ext,
+    unsigned long long* __restrict__ keys, int leaf, int32_t* __restrict__ nxt,
+    int4* __restrict__ srec, int32_t* err) {
+  __shared__ int32_t tmp[kNodesT / 32];
+  __shared__ int64_t tmp2[kNodesT / 32];
+  const int tid = threadIdx.x;
+  const int4 cs = *st;
+  const int m = cs.x;
+  {  // tile offsets
+    const int used = (int)min((int64_t)ntw, ((int64_t)cs.y + kTile - 1) / kTile);
+    const int per = (used + kNodesT - 1) / kNodesT;
+    const int b0 = min(used, tid * per), b1 = min(used, b0 + per);
+    int32_t s = 0;
+    for (int i = b0; i < b1; ++i) s += tile_sum[i];
+    int32_t tot;
+    int32_t pre = block_exclusive_scan<int32_t, kNodesT>(s, tmp, tot);
+    for (int i = b0; i < b1; ++i) {
+      const int32_t v = tile_sum[i];
+      tile_off[i] = pre;
+      pre += v;
     }
   }
-  nxt_cnt[i] = ((int64_t)cnt << 32) | (int64_t)pts;
+  __syncthreads();
+  int64_t done = 0;  // (open children << 32) | their points, of the nodes before this pass
+  for (int i0 = 0; i0 < m; i0 += kNodesT) {
+    const int i = i0 + tid;
+    int32_t a = 0, nl = 0, nr = 0, P0 = 0, w0 = 0, e = 0, c0 = 0;
+    int md = 0;
+    int4 r0 = make_int4(0, 0, 0, 0);
+    if (i < m) {
+      a = act[i];
+      c0 = cs.z + 2 * i;
+      const NodeMeta pm = meta[a];
+      md = mode[a];
+      e = ext[a];
+      w0 = wst[a];
+      nl = make_children<D>(a, c0, pm, meta, cell, pstart, pend, tile_off, w0, md, e, keys, err, P0);
+      nr = pm.count - nl;
+      r0 = make_int4(pm.start, w0, nl, pm.count);
+    }
+    const bool ol = nl > leaf, orr = nr > leaf;
+    const int64_t v = ((int64_t)((ol ? 1 : 0) + (orr ? 1 : 0)) << 32) |
+                      (int64_t)((ol ? nl : 0) + (orr ? nr : 0));
+    int64_t tot;
+    const int64_t at = done + block_exclusive_scan<int64_t, kNodesT>(v, tmp2, tot);
+    done += tot;
+    if (i < m) {
+      int32_t o = (int32_t)(at >> 32), w = (int32_t)(at & 0xffffffffll);
+      int32_t wl = md == 1 ? -2 : -1, wr = md == 2 ? -2 : -1;
+      if (ol) {
+        nxt[o++] = c0;
+        wst[c0] = w;
+        wl = w;
+        w += nl;
+      }
+      if (orr) {
+        nxt[o] = c0 + 1;
+        wst[c0 + 1] = w;
+        wr = w;
+      }
+      srec[2 * (int64_t)a] = r0;
+      srec[2 * (int64_t)a + 1] = make_int4(md == 0 ? P0 : e, c0, wl, wr);
+    }
+  }
+  if (tid == 0)
+    *st_next = make_int4((int32_t)(done >> 32), (int32_t)(done & 0xffffffffll), cs.z + 2 * m,
+                         cs.w + (m > 0 ? 1 : 0));
 }
 
 // next open list (children in list order, so in leaf order) and their working starts
@@ -1098,77 +1196,70 @@ __global__ void k_leaf_box(const NodeMeta* __restrict__ meta, int32_t n_nodes, i
   }
 }
 
-// FP32 node boxes rounded outwards (lo down, hi up): every FP32 gap computed from
-// them is a lower bound of the FP64 gap up to the screen's rounding slack.
+// Per point: the FP64 coordinates as a packed record of (d + 3) / 4 double4s and the
+// absolute coordinates rounded to FP32 in float4s (both zero padded).
 template <int D>
-__global__ void k_box32(const double* __restrict__ box, int32_t n_nodes, float* __restrict__ box32) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)n_nodes * 2 * D) return;
-  double v = box[i];
-  box32[i] = (i & 1) ? __double2float_ru(v) : __double2float_rd(v);
-}
-
-// FP64 points as packed records of (d + 3) / 4 double4s (zero padded)
-template <int D>
-__global__ void k_pts64(const double* __restrict__ Pf, int64_t n, double4* __restrict__ P64) {
+__global__ void k_point_records(const double* __restrict__ Pf, int64_t n, double4* __restrict__ P64,
+                                float4* __restrict__ P32) {
   constexpr int NV = (D + 3) / 4;
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   double v[4 * NV];
+  float f[4 * NV];
 #pragma unroll
-  for (int j = 0; j < 4 * NV; ++j) v[j] = j < D ? Pf[(int64_t)(j < D ? j : 0) * n + p] : 0.0;
+  for (int j = 0; j < 4 * NV; ++j) {
+    v[j] = j < D ? Pf[(int64_t)(j < D ? j : 0) * n + p] : 0.0;
+    f[j] = j < D ? __double2float_rn(v[j]) : 0.0f;
+  }
 #pragma unroll
-  for (int h = 0; h < NV; ++h)
+  for (int h = 0; h < NV; ++h) {
     P64[p * NV + h] = make_double4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+    P32[p * NV + h] = make_float4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
+  }
 }
 
-// Absolute coordinates rounded to FP32, packed in float4s (zero padded).
+// Per node: the record, box and cell at their final place, the box rounded outwards
+// (lo down, hi up: every FP32 gap computed from it is a lower bound of the FP64 gap up
+// to the screen's rounding slack), the cell rounded inwards, a leaf's FP64 centre, and
+// an internal node's child-pair record (both children's outward FP32 boxes, ids,
+// leaf flags and position ranges), so one load serves a whole expansion.
 template <int D>
-__global__ void k_pts32(const double* __restrict__ Pf, int64_t n, float4* __restrict__ P32) {
-  constexpr int NV = (D + 3) / 4;
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  float v[4 * NV];
-#pragma unroll
-  for (int j = 0; j < 4 * NV; ++j) v[j] = j < D ? __double2float_rn(Pf[(int64_t)(j < D ? j : 0) * n + p]) : 0.0f;
-#pragma unroll
-  for (int h = 0; h < NV; ++h)
-    P32[p * NV + h] = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
-}
-
-// Search records: inward-rounded FP32 cells, FP64 leaf centres, and for each
-// internal node the child-pair record (both children's outward FP32 boxes, ids,
-// leaf flags and position ranges) so one load serves a whole expansion.
-template <int D>
-__global__ void k_search_records(const NodeMeta* __restrict__ meta, int32_t n_nodes,
-                                 const double* __restrict__ box, const double* __restrict__ cell,
-                                 float4* __restrict__ pair, float* __restrict__ cell32,
-                                 double* __restrict__ centre) {
+__global__ void k_node_records(const NodeMeta* __restrict__ bmeta, int32_t n_nodes,
+                               const double* __restrict__ bbox, const double* __restrict__ bcell,
+                               NodeMeta* __restrict__ meta, double* __restrict__ box,
+                               double* __restrict__ cell, float* __restrict__ box32,
+                               float4* __restrict__ pair, float* __restrict__ cell32,
+                               double* __restrict__ centre) {
   constexpr int NV = (D + 3) / 4;
   constexpr int PF = pair_f4(D);
   int32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n_nodes) return;
-  NodeMeta m = meta[a];
+  const NodeMeta m = bmeta[a];
+  meta[a] = m;
+  const int64_t b0 = (int64_t)a * 2 * D;
+  const double2* bx = reinterpret_cast<const double2*>(bbox + b0);
+  const double2* bc = reinterpret_cast<const double2*>(bcell + b0);
 #pragma unroll
   for (int j = 0; j < D; ++j) {
-    cell32[(int64_t)a * 2 * D + 2 * j] = __double2float_ru(cell[(int64_t)a * 2 * D + 2 * j]);
-    cell32[(int64_t)a * 2 * D + 2 * j + 1] = __double2float_rd(cell[(int64_t)a * 2 * D + 2 * j + 1]);
+    const double2 x = bx[j], c = bc[j];
+    reinterpret_cast<double2*>(box + b0)[j] = x;
+    reinterpret_cast<double2*>(cell + b0)[j] = c;
+    reinterpret_cast<float2*>(box32 + b0)[j] =
+        make_float2(__double2float_rd(x.x), __double2float_ru(x.y));
+    reinterpret_cast<float2*>(cell32 + b0)[j] =
+        make_float2(__double2float_ru(c.x), __double2float_rd(c.y));
+    if (m.left < 0) centre[(int64_t)a * D + j] = leaf_centre(x.x, x.y);
   }
-  if (m.left < 0) {
-#pragma unroll
-    for (int j = 0; j < D; ++j)
-      centre[(int64_t)a * D + j] =
-          leaf_centre(box[(int64_t)a * 2 * D + 2 * j], box[(int64_t)a * 2 * D + 2 * j + 1]);
-    return;
-  }
+  if (m.left < 0) return;
   float4* rec = pair + (int64_t)a * PF;
   for (int side = 0; side < 2; ++side) {
-    int32_t c = m.left + side;
+    const double2* cx = reinterpret_cast<const double2*>(bbox + (int64_t)(m.left + side) * 2 * D);
     float lo[4 * NV], hi[4 * NV];
 #pragma unroll
     for (int j = 0; j < 4 * NV; ++j) {
-      lo[j] = j < D ? __double2float_rd(box[(int64_t)c * 2 * D + 2 * (j < D ? j : 0)]) : 0.0f;
-      hi[j] = j < D ? __double2float_ru(box[(int64_t)c * 2 * D + 2 * (j < D ? j : 0) + 1]) : 0.0f;
+      const double2 x = j < D ? cx[j < D ? j : 0] : make_double2(0.0, 0.0);
+      lo[j] = j < D ? __double2float_rd(x.x) : 0.0f;
+      hi[j] = j < D ? __double2float_ru(x.y) : 0.0f;
     }
 #pragma unroll
     for (int h = 0; h < NV; ++h) {
@@ -1177,7 +1268,7 @@ __global__ void k_search_records(const NodeMeta* __restrict__ meta, int32_t n_no
           make_float4(hi[4 * h], hi[4 * h + 1], hi[4 * h + 2], hi[4 * h + 3]);
     }
   }
-  const NodeMeta ml = meta[m.left], mr = meta[m.left + 1];
+  const NodeMeta ml = bmeta[m.left], mr = bmeta[m.left + 1];
   int4 info = make_int4(m.left, m.left + 1, ml.left < 0 ? 1 : 0, mr.left < 0 ? 1 : 0);
   rec[4 * NV] = *reinterpret_cast<float4*>(&info);
   int4 range = make_int4(ml.start, ml.count, mr.start, mr.count);
@@ -1220,14 +1311,17 @@ __global__ void k_root_cells(double* cell, const unsigned long long* __restrict_
 // ------------------------------------------------------------------ host side
 
 template <typename T>
-cudaError_t grow(T** p, int64_t old_n, int64_t new_n, cudaStream_t s) {
+cudaError_t grow(const BuildBufs& B, T** p, int64_t old_n, int64_t new_n, cudaStream_t s) {
   T* q = nullptr;
   cudaError_t e = dev_alloc((void**)&q, sizeof(T) * new_n, s);
   if (e != cudaSuccess) return e;
   if (*p && old_n > 0) {
     e = cudaMemcpyAsync(q, *p, sizeof(T) * old_n, cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return e;
-    dev_free(*p, s);
+    if (e != cudaSuccess) {
+      dev_free(q, s);
+      return e;
+    }
+    if (B.owns(*p)) dev_free(*p, s);
   }
   *p = q;
   return cudaSuccess;
@@ -1237,9 +1331,9 @@ ckd_status ensure_tree_cap(BuildBufs& B, int64_t need, cudaStream_t s) {
   if (need <= B.tcap) return CKD_OK;
   int64_t nc = std::max<int64_t>(need, B.tcap * 2);
   int d2 = 2 * B.d;
-  CKD_CUDA(grow(&B.meta, B.tcap, nc, s));
-  CKD_CUDA(grow(&B.cell, B.tcap * d2, nc * d2, s));
-  CKD_CUDA(grow(&B.box, B.tcap * d2, nc * d2, s));
+  CKD_CUDA(grow(B, &B.meta, B.tcap, nc, s));
+  CKD_CUDA(grow(B, &B.cell, B.tcap * d2, nc * d2, s));
+  CKD_CUDA(grow(B, &B.box, B.tcap * d2, nc * d2, s));
   B.tcap = nc;
   return CKD_OK;
 }
@@ -1249,27 +1343,26 @@ ckd_status ensure_node_cap(BuildBufs& B, int64_t need, cudaStream_t s) {
   if (need <= B.cap) return CKD_OK;
   int64_t nc = std::max<int64_t>(need, B.cap * 2);
   int d2 = 2 * B.d;
-  CKD_CUDA(grow(&B.keys, B.cap * d2, nc * d2, s));
-  CKD_CUDA(grow(&B.ext, B.cap, nc, s));
-  CKD_CUDA(grow(&B.mode, B.cap, nc, s));
-  CKD_CUDA(grow(&B.pstart, B.cap, nc, s));
-  CKD_CUDA(grow(&B.pend, B.cap, nc, s));
-  CKD_CUDA(grow(&B.nleft, B.cap, nc, s));
-  CKD_CUDA(grow(&B.pbase, B.cap, nc, s));
-  CKD_CUDA(grow(&B.wst, B.cap, nc, s));
-  CKD_CUDA(grow(&B.frec, B.cap, nc, s));
-  CKD_CUDA(grow(&B.srec, B.cap * 2, nc * 2, s));
+  CKD_CUDA(grow(B, &B.keys, B.cap * d2, nc * d2, s));
+  CKD_CUDA(grow(B, &B.ext, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.mode, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.pstart, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.pend, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.nleft, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.pbase, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.wst, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.frec, B.cap, nc, s));
+  CKD_CUDA(grow(B, &B.srec, B.cap * 2, nc * 2, s));
   B.cap = nc;
   return CKD_OK;
 }
 
 void free_bufs(BuildBufs& B, cudaStream_t s) {
-  void* ps[] = {B.X[0],   B.X[1],    B.I[0],      B.I[1],     B.NID[0],  B.NID[1], B.meta,
-                B.cell,   B.box,     B.keys,      B.ext,      B.mode,    B.pstart, B.pend,
-                B.nleft,  B.pbase,   B.wst,       B.act[0],   B.act[1],  B.nxt_cnt, B.nxt_off,
-                B.tile_sum, B.tile_off, B.scal, B.flags, B.frec, B.srec, B.lst};
+  void* ps[] = {B.meta, B.cell,  B.box, B.keys,  B.ext,  B.mode, B.pstart,
+                B.pend, B.nleft, B.pbase, B.wst, B.frec, B.srec};
   for (void* p : ps)
-    if (p) dev_free(p, s);
+    if (B.owns(p)) dev_free(p, s);
+  if (B.arena) dev_free(B.arena, s);
   B = BuildBufs();
 }
 
@@ -1294,32 +1387,67 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   } guard{&B, s};
 
   const int64_t ntiles = cdiv(n, kTile);
-  for (int b = 0; b < 2; ++b) {
-    CKD_CUDA(dev_alloc((void**)&B.X[b], sizeof(double) * D * n, s));
-    CKD_CUDA(dev_alloc((void**)&B.I[b], sizeof(int32_t) * (n + 4), s));  // + the copy's rounding
-    CKD_CUDA(dev_alloc((void**)&B.NID[b], sizeof(int32_t) * n, s));
+  const int32_t T = (int32_t)t->n_trees;
+  const int64_t max_open = n / (leaf + 1) + 2 + T;
+  B.tcap = node_cap > 0 ? node_cap
+                        : (int64_t)T + std::min<int64_t>(2 * n, 4 * (n / tree_leaf) + 64);
+  B.cap = (int64_t)T + 4 * (n / leaf) + 64;
+  B.tcap = std::max(B.tcap, B.cap);
+  int64_t* off_dev = nullptr;
+  double* Ldev = nullptr;
+  int32_t *flist = nullptr, *fctr = nullptr;  // nodes to finish; k_finish's counters, list length
+  for (int pass = 0; pass < 2; ++pass) {
+    Carve c(B.arena);
+    for (int b = 0; b < 2; ++b) {
+      c.take(&B.X[b], (size_t)D * n);
+      c.take(&B.I[b], n + 4);  // + the bulk copy's rounding
+      c.take(&B.NID[b], n);
+      c.take(&B.act[b], max_open);
+    }
+    c.take(&B.nxt_cnt, max_open);
+    c.take(&B.nxt_off, max_open + 1);
+    c.take(&B.tile_sum, ntiles);
+    c.take(&B.tile_off, ntiles + 1);
+    c.take(&B.flags, ntiles * (kTile / 32));
+    c.take(&B.scal, 4);
+    c.take(&B.lst, 2);
+    c.take(&B.meta, B.tcap);
+    c.take(&B.cell, B.tcap * 2 * D);
+    c.take(&B.box, B.tcap * 2 * D);
+    c.take(&B.keys, B.cap * 2 * D);
+    c.take(&B.ext, B.cap);
+    c.take(&B.mode, B.cap);
+    c.take(&B.pstart, B.cap);
+    c.take(&B.pend, B.cap);
+    c.take(&B.nleft, B.cap);
+    c.take(&B.pbase, B.cap);
+    c.take(&B.wst, B.cap);
+    c.take(&B.frec, B.cap);
+    c.take(&B.srec, B.cap * 2);
+    c.take(&off_dev, T + 1);
+    c.take(&Ldev, CKD_MAX_D);
+    c.take(&fctr, 8);
+    if (pass == 0) {
+      B.arena_bytes = c.off;
+      CKD_CUDA(dev_alloc((void**)&B.arena, c.off, s));
+    }
   }
-  int64_t max_open = n / (leaf + 1) + 2 + t->n_trees;
-  for (int b = 0; b < 2; ++b) CKD_CUDA(dev_alloc((void**)&B.act[b], sizeof(int32_t) * max_open, s));
-  CKD_CUDA(dev_alloc((void**)&B.nxt_cnt, sizeof(int64_t) * max_open, s));
-  CKD_CUDA(dev_alloc((void**)&B.nxt_off, sizeof(int64_t) * (max_open + 1), s));
-  CKD_CUDA(dev_alloc((void**)&B.tile_sum, sizeof(int32_t) * ntiles, s));
-  CKD_CUDA(dev_alloc((void**)&B.tile_off, sizeof(int32_t) * (ntiles + 1), s));
-  CKD_CUDA(dev_alloc((void**)&B.flags, sizeof(unsigned) * ntiles * (kTile / 32), s));
-  CKD_CUDA(dev_alloc((void**)&B.scal, sizeof(int32_t) * 4, s));
-  CKD_CUDA(dev_alloc((void**)&B.lst, sizeof(int4) * 2, s));
   CKD_CUDA(cudaMemsetAsync(B.scal, 0, sizeof(int32_t) * 4, s));
 
-  // final outputs
-  CKD_CUDA(dev_alloc((void**)&t->pts, sizeof(double) * D * n, s));
-  CKD_CUDA(dev_alloc((void**)&t->ids, sizeof(int32_t) * n, s));
+  // the tree's arrays per point
+  constexpr int NV = (D + 3) / 4;
+  for (int pass = 0; pass < 2; ++pass) {
+    Carve c(t->block[0]);
+    c.take(&t->pts, (size_t)D * n);
+    c.take(&t->ids, n);
+    c.take(&t->pts32, (size_t)NV * n);
+    c.take(&t->pts64, (size_t)NV * n);
+    if (pass == 0) CKD_CUDA(dev_alloc(&t->block[0], c.off, s));
+  }
 
   // trees of a forest: positions off[t] .. off[t+1]-1, root node t
-  const int32_t T = (int32_t)t->n_trees;
   const std::vector<int64_t>& off = t->tree_off;
-  Scratch sc(s);  // small per-build buffers (tree offsets, box sides)
-  int64_t* off_dev = nullptr;
-  CKD_CUDA(sc.alloc(&off_dev, sizeof(int64_t) * (T + 1)));
+  Scratch sc(s);
   CKD_CUDA(cudaMemcpyAsync(off_dev, off.data(), sizeof(int64_t) * (T + 1), cudaMemcpyHostToDevice, s));
   {
     unsigned g = (unsigned)cdiv(n, 256);
@@ -1332,14 +1460,7 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
                                               B.NID[0], B.NID[1], offp, T);
     CKD_LAUNCH_CHECK();
   }
-  double* Ldev = nullptr;
-  CKD_CUDA(sc.alloc(&Ldev, sizeof(double) * CKD_MAX_D));
   CKD_CUDA(cudaMemcpyAsync(Ldev, t->L, sizeof(double) * CKD_MAX_D, cudaMemcpyHostToDevice, s));
-  CKD_TRY(ensure_tree_cap(
-      B, node_cap > 0 ? node_cap
-                      : (int64_t)T + std::min<int64_t>(2 * n, 4 * (n / tree_leaf) + 64),
-      s));
-  CKD_TRY(ensure_node_cap(B, (int64_t)T + 4 * (n / leaf) + 64, s));
   k_root_init<D><<<(unsigned)cdiv(T, 128), 128, 0, s>>>(B.meta, B.cell, B.keys, off_dev, T, Ldev,
                                                         t->periodic);
   CKD_LAUNCH_CHECK();
@@ -1405,7 +1526,6 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   if (!roots.empty())
     CKD_CUDA(cudaMemcpyAsync(B.act[0], roots.data(), sizeof(int32_t) * roots.size(),
                              cudaMemcpyHostToDevice, s));
-  CKD_CUDA(cudaStreamSynchronize(s));  // `roots`, `wst0` and `rk` are host buffers of the copies
 
   // the staged scatter needs 16-byte aligned rows (even stride) and fits D <= 4
   // (<= 72 KB of shared memory per block)
@@ -1462,15 +1582,23 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
       k_flags<<<ntw, kBT, 0, s>>>(B.X[cur], B.NID[cur], B.frec, B.ext, n, st, B.tile_sum,
                                   B.pstart, B.pend, B.flags);
       CKD_LAUNCH_CHECK();
-      CKD_TRY(scan_i32(B.tile_sum, B.tile_off, ntw, s));
-      k_children<D><<<gm, 128, 0, s>>>(act, st, mbi, B.meta, B.cell, B.pstart, B.pend, B.tile_off,
-                                       B.wst, B.mode, B.ext, B.nleft, B.pbase, B.keys, leaf,
-                                       B.nxt_cnt, B.scal + 1);
-      CKD_LAUNCH_CHECK();
-      CKD_TRY(scan_i64(B.nxt_cnt, B.nxt_off, mbi, s));
-      k_next_list<<<gm, 128, 0, s>>>(act, st, st_next, mbi, B.meta, B.nxt_off, leaf, B.mode, B.ext,
-                                     B.nleft, B.pbase, B.act[1 - alist], B.wst, B.srec);
-      CKD_LAUNCH_CHECK();
+      if (mbi <= kNodesMax && ntw <= kNodesTiles) {
+        k_level_nodes<D><<<1, kNodesT, 0, s>>>(act, st, st_next, (int)ntw, B.meta, B.cell,
+                                               B.pstart, B.pend, B.tile_sum, B.tile_off, B.wst,
+                                               B.mode, B.ext, B.keys, leaf, B.act[1 - alist],
+                                               B.srec, B.scal + 1);
+        CKD_LAUNCH_CHECK();
+      } else {
+        CKD_TRY(scan_i32(B.tile_sum, B.tile_off, ntw, s));
+        k_children<D><<<gm, 128, 0, s>>>(act, st, mbi, B.meta, B.cell, B.pstart, B.pend,
+                                         B.tile_off, B.wst, B.mode, B.ext, B.nleft, B.pbase,
+                                         B.keys, leaf, B.nxt_cnt, B.scal + 1);
+        CKD_LAUNCH_CHECK();
+        CKD_TRY(scan_i64(B.nxt_cnt, B.nxt_off, mbi, s));
+        k_next_list<<<gm, 128, 0, s>>>(act, st, st_next, mbi, B.meta, B.nxt_off, leaf, B.mode,
+                                       B.ext, B.nleft, B.pbase, B.act[1 - alist], B.wst, B.srec);
+        CKD_LAUNCH_CHECK();
+      }
       if (staged)
         k_scatter<D, true><<<ntw, kBT, scatter_smem(D), s>>>(
             B.X[cur], B.I[cur], B.NID[cur], B.srec, B.tile_off, B.flags, n, st, B.X[1 - cur],
@@ -1496,12 +1624,11 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   CKD_CUDA(cudaMemcpyAsync(&err, B.scal + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
 
   if (finish) {
-    int32_t *list = nullptr, *ctr = nullptr;  // ctr[4]: entries of the list
-    CKD_CUDA(sc.alloc(&list, sizeof(int32_t) * n_nodes));
-    CKD_CUDA(sc.alloc(&ctr, sizeof(int32_t) * 5));
+    int32_t* const ctr = fctr;
+    CKD_CUDA(sc.alloc(&flist, sizeof(int32_t) * n_nodes));
     int32_t h[5] = {n_nodes, depth_levels, 0, 0, 0};
     CKD_CUDA(cudaMemcpyAsync(ctr, h, sizeof(h), cudaMemcpyHostToDevice, s));
-    k_finish_list<<<(unsigned)cdiv(n_nodes, 256), 256, 0, s>>>(B.meta, n_nodes, tree_leaf, list,
+    k_finish_list<<<(unsigned)cdiv(n_nodes, 256), 256, 0, s>>>(B.meta, n_nodes, tree_leaf, flist,
                                                                ctr + 4);
     CKD_LAUNCH_CHECK();
     int dev = 0, sms = 148, per_sm = 1;
@@ -1513,7 +1640,7 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
     CKD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_finish<D>, kFinT, sm));
     const int64_t g = std::min<int64_t>(n_nodes, (int64_t)sms * std::max(1, per_sm));
     k_finish<D><<<(unsigned)g, kFinT, sm, s>>>(
-        list, ctr + 4, B.meta, B.cell, B.box, t->pts, t->ids, n, tree_leaf,
+        flist, ctr + 4, B.meta, B.cell, B.box, t->pts, t->ids, n, tree_leaf,
         (int32_t)std::min<int64_t>(B.tcap, INT32_MAX), kMaxLevels, ctr);
     CKD_LAUNCH_CHECK();
     CKD_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -1532,12 +1659,17 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   CKD_LAUNCH_CHECK();
   t->n_nodes = n_nodes;
   t->depth = depth_levels;
-  CKD_CUDA(dev_alloc((void**)&t->meta, sizeof(NodeMeta) * n_nodes, s));
-  CKD_CUDA(dev_alloc((void**)&t->box, sizeof(double) * 2 * D * n_nodes, s));
-  CKD_CUDA(dev_alloc((void**)&t->cell, sizeof(double) * 2 * D * n_nodes, s));
-  CKD_CUDA(cudaMemcpyAsync(t->meta, B.meta, sizeof(NodeMeta) * n_nodes, cudaMemcpyDeviceToDevice, s));
-  CKD_CUDA(cudaMemcpyAsync(t->box, B.box, sizeof(double) * 2 * D * n_nodes, cudaMemcpyDeviceToDevice, s));
-  CKD_CUDA(cudaMemcpyAsync(t->cell, B.cell, sizeof(double) * 2 * D * n_nodes, cudaMemcpyDeviceToDevice, s));
+  for (int pass = 0; pass < 2; ++pass) {  // the tree's arrays per node
+    Carve c(t->block[1]);
+    c.take(&t->meta, n_nodes);
+    c.take(&t->box, (size_t)2 * D * n_nodes);
+    c.take(&t->cell, (size_t)2 * D * n_nodes);
+    c.take(&t->box32, (size_t)2 * D * n_nodes);
+    c.take(&t->pair, (size_t)pair_f4(D) * n_nodes);
+    c.take(&t->cell32, (size_t)2 * D * n_nodes);
+    c.take(&t->centre, (size_t)D * n_nodes);
+    if (pass == 0) CKD_CUDA(dev_alloc(&t->block[1], c.off, s));
+  }
   // FP32 screening copies.  The node-gap slack per axis is 2^-21 * (|q| + B) with
   // B bounding every stored coordinate (and the box side when periodic); the
   // screen is disabled for coordinates near the FP32 range.
@@ -1547,21 +1679,11 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
     if (!(b < 1e18)) t->screen_ok = false;
     t->slack[j] = (float)(b * (1.0 + 1e-6));
   }
-  constexpr int NV = (D + 3) / 4;
-  CKD_CUDA(dev_alloc((void**)&t->box32, sizeof(float) * 2 * D * n_nodes, s));
-  CKD_CUDA(dev_alloc((void**)&t->pts32, sizeof(float4) * NV * n, s));
-  CKD_CUDA(dev_alloc((void**)&t->pts64, sizeof(double4) * NV * n, s));
-  k_pts64<D><<<(unsigned)cdiv(n, 256), 256, 0, s>>>(t->pts, n, t->pts64);
+  k_point_records<D><<<(unsigned)cdiv(n, 256), 256, 0, s>>>(t->pts, n, t->pts64, t->pts32);
   CKD_LAUNCH_CHECK();
-  k_pts32<D><<<(unsigned)cdiv(n, 256), 256, 0, s>>>(t->pts, n, t->pts32);
-  CKD_LAUNCH_CHECK();
-  k_box32<D><<<(unsigned)cdiv((int64_t)n_nodes * 2 * D, 256), 256, 0, s>>>(t->box, n_nodes, t->box32);
-  CKD_LAUNCH_CHECK();
-  CKD_CUDA(dev_alloc((void**)&t->pair, sizeof(float4) * pair_f4(D) * n_nodes, s));
-  CKD_CUDA(dev_alloc((void**)&t->cell32, sizeof(float) * 2 * D * n_nodes, s));
-  CKD_CUDA(dev_alloc((void**)&t->centre, sizeof(double) * D * n_nodes, s));
-  k_search_records<D><<<(unsigned)cdiv(n_nodes, 128), 128, 0, s>>>(
-      t->meta, n_nodes, t->box, t->cell, t->pair, t->cell32, t->centre);
+  k_node_records<D><<<(unsigned)cdiv(n_nodes, 128), 128, 0, s>>>(
+      B.meta, n_nodes, B.box, B.cell, t->meta, t->box, t->cell, t->box32, t->pair, t->cell32,
+      t->centre);
   CKD_LAUNCH_CHECK();
   CKD_CUDA(cudaStreamSynchronize(s));
   if (err == 3) return fail(CKD_ERR_TIMEOUT, "build: a tile copy into shared memory timed out");
@@ -1589,10 +1711,12 @@ ckd_status build_dispatch(ckd_tree* t, const void* pts_dev, int dtype, cudaStrea
     // more nodes than planned: once more with room for every tree of these points
     again = false;
     cap = t->n_trees + 2 * t->n;
-    dev_free(t->pts, s);
-    dev_free(t->ids, s);
+    dev_free(t->block[0], s);
+    t->block[0] = nullptr;
     t->pts = nullptr;
     t->ids = nullptr;
+    t->pts32 = nullptr;
+    t->pts64 = nullptr;
   }
 }
 

@@ -106,6 +106,19 @@ struct Scratch {
   }
 };
 
+// Parts of one block: laid out once to find its size (base null), once more to
+// place the pointers.
+struct Carve {
+  char* base;
+  size_t off = 0;
+  explicit Carve(void* b) : base(static_cast<char*>(b)) {}
+  template <typename T>
+  void take(T** p, size_t count) {
+    *p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+    off += (count * sizeof(T) + 255) & ~size_t(255);
+  }
+};
+
 // ------------------------------------------------------------- node layout
 // One 32-byte record per node.  Children of an internal node are allocated as a
 // pair: right = left + 1.  start/count give the node's range in the leaf-ordered
@@ -254,6 +267,9 @@ struct ckd_tree {
   float4* pair = nullptr;
   float* cell32 = nullptr;
   double* centre = nullptr;
+  // a built tree's arrays are parts of two pool blocks: per point and per node
+  // (null: every array is a block of its own)
+  void* block[2] = {nullptr, nullptr};
   ckd::TreeView view() const {
     ckd::TreeView v;
     v.n = (int32_t)n;
