@@ -105,6 +105,8 @@ SIGNATURES = {
     "ckd_box_count_host": [_vp, _vp, _i64, _vp, _vp],
     "ckd_box_fill_host": [_vp, _vp, _i64, _vp, _vp, _vp],
     "ckd_exclusive_scan": [_vp, _vp, _i64, _vp],
+    "ckd_csr_offsets": [_vp, _vp, _i64, _pi64, _vp],
+    "ckd_queries_inside": [_vp, _vp, _i64, _pint, _vp],
     "ckd_tree_save": [_vp, ctypes.c_char_p],
     "ckd_tree_load": [ctypes.c_char_p, ctypes.POINTER(_vp)],
     "ckd_forest_build": [_vp, _pi64, _i64, _int, _int, _int, _pdbl, _int, _vp,

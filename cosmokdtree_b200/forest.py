@@ -32,7 +32,7 @@ import torch
 
 from . import _lib
 from ._lib import CKDArgumentError, check
-from .kdtree import _check_k, _on_device, _ptr, _stream
+from .kdtree import _check_inside, _check_k, _csr_offsets, _on_device, _ptr, _stream
 
 __all__ = ["Forest", "ForestPlan", "build_forest"]
 
@@ -99,11 +99,8 @@ class Forest:
     def _grouped(self, x, off, name, width):
         x = _rows(x, width, self.device, name)
         o = _offsets(off, self.n_trees, x.shape[0], f"{name} offsets")
-        if name == "queries" and self.periodic and x.shape[0] > 0:
-            half = torch.as_tensor(self.boxsize / 2.0, dtype=torch.float64, device=x.device)
-            if bool(((x < -half) | (x > half) | torch.isnan(x)).any()):
-                raise CKDArgumentError(_lib.CKD_ERR_OUT_OF_BOX,
-                                       "periodic forest: query points must lie in [-L/2, L/2]")
+        if name == "queries":
+            _check_inside(self, x, "forest")
         return x, torch.from_numpy(o).to(f"cuda:{self.device}")
 
     def knn(self, queries, query_offsets, k, sorted=True):
@@ -138,14 +135,10 @@ class Forest:
             b, bo = self._grouped(boxes, box_offsets, "boxes", 2 * self.d)
             nb = b.shape[0]
             counts = torch.empty(nb, dtype=torch.int64, device=b.device)
-            # the scan writes every entry
-            offsets = (torch.empty if nb > 0 else torch.zeros)(nb + 1, dtype=torch.int64,
-                                                                device=b.device)
             if nb > 0:
                 check(L.ckd_forest_box_count(self.handle, _ptr(b), _ptr(bo), nb, _ptr(counts),
                                              _stream()))
-                check(L.ckd_exclusive_scan(_ptr(counts), _ptr(offsets), nb, _stream()))
-            total = int(offsets[-1].item())
+            offsets, total = _csr_offsets(counts, nb)
             idx = torch.empty(total, dtype=torch.int64, device=b.device)
             if nb > 0 and total > 0:
                 check(L.ckd_forest_box_fill(self.handle, _ptr(b), _ptr(bo), nb, _ptr(offsets),
@@ -164,14 +157,10 @@ class Forest:
             q, qo = self._grouped(queries, query_offsets, "queries", self.d)
             nq = q.shape[0]
             counts = torch.empty(nq, dtype=torch.int64, device=q.device)
-            # the scan writes every entry
-            offsets = (torch.empty if nq > 0 else torch.zeros)(nq + 1, dtype=torch.int64,
-                                                                device=q.device)
             if nq > 0:
                 check(L.ckd_forest_ball_count(self.handle, _ptr(q), _ptr(qo), nq, radius,
                                               _ptr(counts), _stream()))
-                check(L.ckd_exclusive_scan(_ptr(counts), _ptr(offsets), nq, _stream()))
-            total = int(offsets[-1].item())
+            offsets, total = _csr_offsets(counts, nq)
             idx = torch.empty(total, dtype=torch.int64, device=q.device)
             dist = torch.empty(total, dtype=torch.float64, device=q.device)
             if nq > 0 and total > 0:

@@ -22,6 +22,7 @@ reference returns them.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 
@@ -44,6 +45,14 @@ def _stream():
 
 def _ptr(t: torch.Tensor):
     return ctypes.c_void_p(t.data_ptr())
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(device: int):
+    """``torch.cuda.device(device)``, or nothing to enter when it is current."""
+    return _HERE if torch.cuda.current_device() == device else torch.cuda.device(device)
 
 
 class KDTree:
@@ -110,7 +119,9 @@ def _queries(tree: KDTree, target) -> tuple[torch.Tensor, bool]:
     caller passed device data.  A 1-D target is one point (kdtree.py:45-46)."""
     dev = _on_device(target)
     if dev:
-        q = target.to(device=f"cuda:{tree.device}", dtype=torch.float64)
+        q = target
+        if q.dtype is not torch.float64 or q.device.index != tree.device:
+            q = q.to(device=f"cuda:{tree.device}", dtype=torch.float64)
     else:
         q = torch.from_numpy(np.ascontiguousarray(np.atleast_1d(np.asarray(target,
                                                                            dtype=np.float64))))
@@ -121,20 +132,46 @@ def _queries(tree: KDTree, target) -> tuple[torch.Tensor, bool]:
                                "target dimensionality does not match the tree")
     if not dev:
         q = q.pin_memory().to(f"cuda:{tree.device}", non_blocking=True)
-    if tree.periodic and q.shape[0] > 0:  # checked on the device
-        half = torch.as_tensor(tree.boxsize / 2.0, dtype=torch.float64, device=q.device)
-        bad = (q < -half) | (q > half) | torch.isnan(q)
-        if bool(bad.any()):
+    q = q.contiguous()
+    _check_inside(tree, q, "tree")
+    return q, dev
+
+
+def _check_inside(tree, q: torch.Tensor, what: str) -> None:
+    """Raise unless the device queries of a periodic tree or forest lie in its box."""
+    if tree.periodic and q.shape[0] > 0:
+        inside = ctypes.c_int(1)
+        check(_lib.load().ckd_queries_inside(tree.handle, _ptr(q), q.shape[0],
+                                             ctypes.byref(inside), _stream()))
+        if not inside.value:
             raise CKDArgumentError(_lib.CKD_ERR_OUT_OF_BOX,
-                                   "periodic tree: query points must lie in [-L/2, L/2]")
-    return q.contiguous(), dev
+                                   f"periodic {what}: query points must lie in [-L/2, L/2]")
+
+
+def _csr_offsets(counts: torch.Tensor, n: int) -> tuple[torch.Tensor, int]:
+    """Row offsets (n + 1,) of the counts, and their total."""
+    if n == 0:
+        return torch.zeros(1, dtype=torch.int64, device=counts.device), 0
+    offsets = torch.empty(n + 1, dtype=torch.int64, device=counts.device)
+    total = ctypes.c_int64()
+    check(_lib.load().ckd_csr_offsets(_ptr(counts), _ptr(offsets), n, ctypes.byref(total),
+                                      _stream()))
+    return offsets, int(total.value)
 
 
 def _to_host(t: torch.Tensor) -> np.ndarray:
-    h = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
-    h.copy_(t, non_blocking=True)
+    return _all_to_host(t)[0]
+
+
+def _all_to_host(*ts: torch.Tensor) -> tuple[np.ndarray, ...]:
+    """Pinned host copies of device tensors, waited for once."""
+    hs = []
+    for t in ts:
+        h = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
+        h.copy_(t, non_blocking=True)
+        hs.append(h)
     torch.cuda.current_stream().synchronize()
-    return h.numpy()
+    return tuple(h.numpy() for h in hs)
 
 
 # ---------------------------------------------------------------- build
@@ -177,7 +214,7 @@ def build_kdtree(points, leaf=None, boxsize=None) -> KDTree:
         device = pts.device.index if pts.device.index is not None else torch.cuda.current_device()
     else:
         device = torch.cuda.current_device()
-    with torch.cuda.device(device):
+    with _on(device):
         if not dev_in:
             pts = pts.pin_memory().to(f"cuda:{device}", non_blocking=True)
         pts = pts.contiguous()
@@ -215,7 +252,7 @@ def _check_k(k):
 def knn_search_batch(tree: KDTree, target, k, sorted=True):
     """k nearest neighbours of every target point; (dist, idx) CUDA tensors (nq, k)."""
     k = _check_k(k)
-    with torch.cuda.device(tree.device):
+    with _on(tree.device):
         q, _ = _queries(tree, target)
         nq = q.shape[0]
         dist = torch.empty((nq, k), dtype=torch.float64, device=q.device)
@@ -314,13 +351,13 @@ def knn_search(tree: KDTree, target, k, sorted=True):
         k = _check_k(k)
         nq = np.shape(target)[0] if np.ndim(target) == 2 else 1
         if nq >= _PIPE_MIN_ROWS:
-            with torch.cuda.device(tree.device):
+            with _on(tree.device):
                 return _knn_host_pipelined(tree, target, k, sorted)
     dist, idx = knn_search_batch(tree, target, k, sorted)
     if _on_device(target):
         return dist, idx
-    with torch.cuda.device(tree.device):
-        return _to_host(dist), _to_host(idx)
+    with _on(tree.device):
+        return _all_to_host(dist, idx)
 
 
 def knn_search_multi_k(tree: KDTree, target, ks, sorted=True):
@@ -329,7 +366,7 @@ def knn_search_multi_k(tree: KDTree, target, ks, sorted=True):
     (ntar, max(ks)); a row's slots past its own k hold id -2 and distance
     1.8446743523953730e19 (the k > n marker).  numpy for host input, CUDA tensors
     for CUDA-tensor input."""
-    with torch.cuda.device(tree.device):
+    with _on(tree.device):
         q, _ = _queries(tree, target)
         nq = q.shape[0]
         kt = torch.as_tensor(np.asarray(ks) if not isinstance(ks, torch.Tensor) else ks)
@@ -348,7 +385,7 @@ def knn_search_multi_k(tree: KDTree, target, ks, sorted=True):
                                               int(bool(sorted)), _ptr(dist), _ptr(idx), _stream()))
         if _on_device(target):
             return dist, idx
-        return _to_host(dist), _to_host(idx)
+        return _all_to_host(dist, idx)
 
 
 # ---------------------------------------------------------------- ball
@@ -364,17 +401,13 @@ def ball_search_csr(tree: KDTree, target, radius, sorted=False):
     (offsets (nq+1,), idx, dist)."""
     radius = _check_radius(radius)
     L = _lib.load()
-    with torch.cuda.device(tree.device):
+    with _on(tree.device):
         q, _ = _queries(tree, target)
         nq = q.shape[0]
         counts = torch.empty(nq, dtype=torch.int64, device=q.device)
-        # the scan writes every entry
-        offsets = (torch.empty if nq > 0 else torch.zeros)(nq + 1, dtype=torch.int64,
-                                                            device=q.device)
         if nq > 0:
             check(L.ckd_ball_count(tree.handle, _ptr(q), nq, radius, _ptr(counts), _stream()))
-            check(L.ckd_exclusive_scan(_ptr(counts), _ptr(offsets), nq, _stream()))
-        total = int(offsets[-1].item())
+        offsets, total = _csr_offsets(counts, nq)
         idx = torch.empty(total, dtype=torch.int64, device=q.device)
         dist = torch.empty(total, dtype=torch.float64, device=q.device)
         if nq > 0 and total > 0:
@@ -386,8 +419,8 @@ def ball_search_csr(tree: KDTree, target, radius, sorted=False):
 def ball_search(tree: KDTree, target, radius, sorted=False):
     """Ball search (kdtree.py:56-79): per target lists of distances and 0-based ids."""
     offsets, idx, dist = ball_search_csr(tree, target, radius, sorted)
-    with torch.cuda.device(tree.device):
-        off, i, d = _to_host(offsets), _to_host(idx), _to_host(dist)
+    with _on(tree.device):
+        off, i, d = _all_to_host(offsets, idx, dist)
     n = len(off) - 1
     return ([d[off[j]:off[j + 1]] for j in range(n)], [i[off[j]:off[j + 1]] for j in range(n)])
 
@@ -398,9 +431,11 @@ def box_search_csr(tree: KDTree, boxes):
     """Points inside each of many axis-aligned boxes ([lo0, hi0, lo1, hi1, ...] rows),
     CSR CUDA tensors (offsets (nb+1,), idx)."""
     L = _lib.load()
-    with torch.cuda.device(tree.device):
+    with _on(tree.device):
         if _on_device(boxes):
-            b = boxes.to(device=f"cuda:{tree.device}", dtype=torch.float64)
+            b = boxes
+            if b.dtype is not torch.float64 or b.device.index != tree.device:
+                b = b.to(device=f"cuda:{tree.device}", dtype=torch.float64)
         else:
             b = torch.from_numpy(np.array(boxes, dtype=np.float64, copy=True, ndmin=1))
         if b.dim() == 1:
@@ -408,16 +443,14 @@ def box_search_csr(tree: KDTree, boxes):
         if b.shape[-1] != 2 * tree.d:  # cosmokdtree2py.f90:275-277
             raise CKDArgumentError(_lib.CKD_ERR_BAD_DIM,
                                    "Error: box size does not match tree dimensionality.")
-        b = b.to(f"cuda:{tree.device}").contiguous()
+        if not b.is_cuda:
+            b = b.to(f"cuda:{tree.device}")
+        b = b.contiguous()
         nb = b.shape[0]
         counts = torch.empty(nb, dtype=torch.int64, device=b.device)
-        # the scan writes every entry
-        offsets = (torch.empty if nb > 0 else torch.zeros)(nb + 1, dtype=torch.int64,
-                                                            device=b.device)
         if nb > 0:
             check(L.ckd_box_count(tree.handle, _ptr(b), nb, _ptr(counts), _stream()))
-            check(L.ckd_exclusive_scan(_ptr(counts), _ptr(offsets), nb, _stream()))
-        total = int(offsets[-1].item())
+        offsets, total = _csr_offsets(counts, nb)
         idx = torch.empty(total, dtype=torch.int64, device=b.device)
         if nb > 0 and total > 0:
             check(L.ckd_box_fill(tree.handle, _ptr(b), nb, _ptr(offsets), _ptr(idx), _stream()))
@@ -428,7 +461,7 @@ def box_search(tree: KDTree, box):
     """Ids of the points inside one box [xmin, xmax, ymin, ymax, ...] (kdtree.py:82-87)."""
     b = np.array(box, dtype=np.float64, ndmin=1).reshape(-1)
     offsets, idx = box_search_csr(tree, b.reshape(1, -1))
-    with torch.cuda.device(tree.device):
+    with _on(tree.device):
         return _to_host(idx)
 
 
@@ -474,7 +507,7 @@ def box_search_periodic_csr(tree: KDTree, boxes):
             pieces.append([v for lohi in c for v in lohi])
             owner.append(i)
     nb = b.shape[0]
-    with torch.cuda.device(tree.device):
+    with _on(tree.device):
         if not pieces:
             return (torch.zeros(nb + 1, dtype=torch.int64, device=f"cuda:{tree.device}"),
                     torch.empty(0, dtype=torch.int64, device=f"cuda:{tree.device}"))
@@ -495,7 +528,7 @@ def box_search_periodic_csr(tree: KDTree, boxes):
 def save_kdtree(tree, path: str) -> None:
     """Write a built tree (or forest) to ``path``; ``load_kdtree`` restores it without
     rebuilding and with bit-identical results."""
-    with torch.cuda.device(tree.device):
+    with _on(tree.device):
         check(_lib.load().ckd_tree_save(tree.handle, os.fsencode(path)))
 
 
@@ -504,7 +537,7 @@ def load_kdtree(path: str, device=None):
     Returns a KDTree, or a Forest when the file holds several trees."""
     device = torch.cuda.current_device() if device is None else int(device)
     L = _lib.load()
-    with torch.cuda.device(device):
+    with _on(device):
         h = ctypes.c_void_p()
         check(L.ckd_tree_load(os.fsencode(path), ctypes.byref(h)))
         n, d, leaf, per = ctypes.c_int64(), ctypes.c_int(), ctypes.c_int(), ctypes.c_int()

@@ -25,8 +25,8 @@ import torch
 
 from . import _lib
 from ._lib import MLP_FEATURES, MLP_NORM, MLP_PARAMS, CKDArgumentError, check
-from .kdtree import (_PIPE_MIN_ROWS, KDTree, _check_k, _knn_host_pipelined, _ptr, _queries,
-                     _stream, _to_host, knn_search_batch)
+from .kdtree import (_PIPE_MIN_ROWS, KDTree, _all_to_host, _check_k, _knn_host_pipelined, _ptr,
+                     _queries, _stream, knn_search_batch)
 
 __all__ = ["LearnedBound"]
 
@@ -250,7 +250,7 @@ class LearnedBound:
         if isinstance(target, torch.Tensor) and target.is_cuda:
             return dist, idx
         with torch.cuda.device(tree.device):
-            return _to_host(dist), _to_host(idx)
+            return _all_to_host(dist, idx)
 
     def knn_multi_k(self, tree: KDTree, target, ks, sorted=True):
         """Exact kNN with a k per target row and the learned bound, in one call:
@@ -281,7 +281,7 @@ class LearnedBound:
             self.last_fallback = int(nfb.value)
             if isinstance(target, torch.Tensor) and target.is_cuda:
                 return dist, idx
-            return _to_host(dist), _to_host(idx)
+            return _all_to_host(dist, idx)
 
     def knn_batch(self, tree: KDTree, target, k, sorted=True):
         """As ``knn`` with CUDA-tensor results."""

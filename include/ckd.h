@@ -311,6 +311,15 @@ ckd_status ckd_tree_load(const char* path, ckd_tree** out);
 
 /* out_dev[0] = 0, out_dev[i+1] = in_dev[0] + ... + in_dev[i]  (n+1 outputs). */
 ckd_status ckd_exclusive_scan(const int64_t* in_dev, int64_t* out_dev, int64_t n, void* stream);
+/* ckd_exclusive_scan, and the total (out_dev[n]) in host memory when it returns. */
+ckd_status ckd_csr_offsets(const int64_t* counts_dev, int64_t* offsets_dev, int64_t n,
+                           int64_t* total_host, void* stream);
+
+/* *inside_host = 1 when every coordinate of the nq query points lies in [-L/2, L/2] of a
+ * periodic tree or forest (NaN does not), 0 otherwise; 1 for a tree that is not
+ * periodic.  Synchronous: the answer is there when it returns. */
+ckd_status ckd_queries_inside(const ckd_tree* tree, const double* q_dev, int64_t nq,
+                              int* inside_host, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Learned k-th-neighbour distance bound (no counterpart in the reference; it
