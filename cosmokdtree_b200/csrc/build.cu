@@ -147,7 +147,26 @@ __global__ void k_compact_roots(const double* __restrict__ X, const int32_t* __r
   NIDo[w] = t;
 }
 
-// Segmented min/max over the working positions.  Each thread reduces kItems
+// minimum of a 64-bit key over the warp
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+  const unsigned hi = (unsigned)(k >> 32);
+  const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? (unsigned)k : 0xffffffffu);
+  return ((unsigned long long)mh << 32) | ml;
+}
+
+// Whether a tile of working positions is full and lies in one node: a node's positions
+// are contiguous, so equal ids at both ends are enough.  True for most tiles while
+// nodes hold many tiles; the box, flag and scatter passes then do not read the ids,
+// and the first two need no segments (2^24 clustered points, all levels: boxes 2340 ->
+// 1670 us, flags 977 -> 740 us, 28 -> 24 and 12 -> 8 bytes a point).
+__device__ __forceinline__ bool tile_of_one_node(const int32_t* __restrict__ NID, int64_t base,
+                                                 int64_t nw) {
+  return base + kTile <= nw && __ldg(NID + base) == __ldg(NID + base + kTile - 1);
+}
+
+// Segmented min/max over the working positions.  Tiles of one node (all of them while
+// nodes are large) take a plain reduction without reading the ids.  Else each thread reduces kItems
 // consecutive positions in registers; one segmented warp scan per dimension
 // joins the pieces of runs that cross thread boundaries.  Runs that end
 // inside a warp chunk go straight to atomicMin/atomicMax; the first and last
@@ -162,8 +181,46 @@ __global__ void __launch_bounds__(kBT, 5) k_seg_box(const double* __restrict__ X
   __shared__ int32_t rec_id[W][2];
   __shared__ unsigned long long rec_v[W][2][2 * D];
   if (st) nw = st->y;  // working points of this level (device state)
-  if ((int64_t)blockIdx.x * kTile >= nw) return;
+  const int64_t base = (int64_t)blockIdx.x * kTile;
+  if (base >= nw) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (tile_of_one_node(NID, base, nw) && (n & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
+    // whole tile in one node (its positions are contiguous): no ids, no segments;
+    // coordinates in coalesced pairs
+    unsigned long long kmn[D], kmx[D];  // minima of the keys and of their complements
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      const ulonglong2* __restrict__ Xj =
+          reinterpret_cast<const ulonglong2*>(X + (int64_t)j * n + base) + threadIdx.x;
+      kmn[j] = kmx[j] = ~0ull;
+#pragma unroll
+      for (int i = 0; i < kItems / 2; ++i) {
+        const ulonglong2 v = __ldg(Xj + i * kBT);
+        const unsigned long long k0 = dkey_bits(v.x), k1 = dkey_bits(v.y);
+        const unsigned long long mn = k0 < k1 ? k0 : k1, mx = ~(k0 < k1 ? k1 : k0);
+        kmn[j] = mn < kmn[j] ? mn : kmn[j];
+        kmx[j] = mx < kmx[j] ? mx : kmx[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      const unsigned long long mn = warp_min_key(kmn[j]), mx = warp_min_key(kmx[j]);
+      if (lane == 0) {
+        rec_v[w][0][2 * j] = mn;
+        rec_v[w][0][2 * j + 1] = mx;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * D) {
+      unsigned long long v = rec_v[0][0][threadIdx.x];
+#pragma unroll
+      for (int x = 1; x < W; ++x) v = rec_v[x][0][threadIdx.x] < v ? rec_v[x][0][threadIdx.x] : v;
+      unsigned long long* k = &keys[(int64_t)NID[base] * 2 * D + threadIdx.x];
+      if (threadIdx.x & 1) atomicMax(k, ~v);
+      else atomicMin(k, v);
+    }
+    return;
+  }
   const int64_t p0 = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
   // node of every position (-1 past the working set), run breaks inside the thread
   static_assert(kItems == 8, "two int4 / four double2 loads per thread");
@@ -450,7 +507,40 @@ __global__ void __launch_bounds__(kBT) k_flags(const double* __restrict__ X,
     return;
   }
   const int lane = threadIdx.x & 31;
-  const int64_t p0 = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
+  const int64_t base = (int64_t)blockIdx.x * kTile;
+  if (tile_of_one_node(NID, base, nw)) {
+    // one split for the whole tile: 32 consecutive positions a warp and pass, whose
+    // ballot is a word of the bitmap; the node starts or ends here only at the tile's
+    // own ends
+    const int w = threadIdx.x >> 5;
+    const int32_t a1 = __ldg(NID + base);
+    const FlagRec r = frec[a1];
+    const double* __restrict__ xr = X + (int64_t)r.axis * n + base + threadIdx.x;
+    double x[kItems];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) x[i] = __ldg(xr + i * kBT);
+    int32_t sum = 0;
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const unsigned word = __ballot_sync(0xffffffffu, r.md == 0 && x[i] < r.split);
+      if (r.md != 0 && x[i] == r.split)
+        atomicMin(&ext[a1], (int32_t)(base + i * kBT + threadIdx.x));
+      if (lane == 0) flags[(base >> 5) + i * (kBT / 32) + w] = word;
+      sum += __popc(word);
+    }
+    if (lane == 0) tmp[w] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int32_t tot = 0;
+#pragma unroll
+      for (int i = 0; i < kBT / 32; ++i) tot += tmp[i];
+      tile_sum[blockIdx.x] = tot;
+      if (r.wst == base) pstart[a1] = 0;
+      if (r.wst + r.count == base + kTile) pend[a1] = tot;
+    }
+    return;
+  }
+  const int64_t p0 = base + (int64_t)threadIdx.x * kItems;
   int32_t a[kItems];
   const bool full = p0 + kItems <= nw;
   const bool vec = full && (n & 1) == 0 && (reinterpret_cast<uintptr_t>(NID) & 15) == 0 &&
@@ -794,10 +884,12 @@ __global__ void __launch_bounds__(kBT) k_scatter(
   }
   unsigned msk[kItems];
   int32_t av[kItems];
+  const bool one = tile_of_one_node(NID, base, nw);
+  const int32_t one_id = __ldg(NID + base);
 #pragma unroll
   for (int it = 0; it < kItems; ++it) {
     const int64_t p = base + (int64_t)it * kBT + threadIdx.x;
-    av[it] = p < nw ? NID[p] : -1;
+    av[it] = one ? one_id : p < nw ? NID[p] : -1;
     msk[it] = flags[(base >> 5) + it * W + w];  // the flag pass's ballot of these 32 positions
   }
   tile_chunk_prefix(msk, cpre);
@@ -879,14 +971,6 @@ __host__ __device__ constexpr int finish_open(int m, int leaf) { return m / (lea
 __host__ __device__ constexpr size_t finish_smem(int d, int leaf) {
   const size_t m = finish_max(d);
   return m * (8 * d + 4 + 2 * 2) + 2 * (size_t)finish_open((int)m, leaf) * 8;
-}
-
-// minimum of a 64-bit key over the warp
-__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
-  const unsigned hi = (unsigned)(k >> 32);
-  const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? (unsigned)k : 0xffffffffu);
-  return ((unsigned long long)mh << 32) | ml;
 }
 
 // nodes the level passes left: leaves of the list so far with more than `leaf` points
@@ -1218,39 +1302,43 @@ __global__ void k_point_records(const double* __restrict__ Pf, int64_t n, double
   }
 }
 
-// Per node: the record, box and cell at their final place, the box rounded outwards
-// (lo down, hi up: every FP32 gap computed from it is a lower bound of the FP64 gap up
-// to the screen's rounding slack), the cell rounded inwards, a leaf's FP64 centre, and
-// an internal node's child-pair record (both children's outward FP32 boxes, ids,
-// leaf flags and position ranges), so one load serves a whole expansion.
+// The nodes' boxes and cells at their final place, with the FP32 forms: boxes rounded
+// outwards (lo down, hi up: every FP32 gap computed from them is a lower bound of the
+// FP64 gap up to the screen's rounding slack), cells inwards.  One value a thread:
+// with a node a thread its 48-byte strides took 400 us for all node records of 2^24
+// clustered points, against 232 us for this and the next kernel.
+__global__ void k_node_boxes(const double* __restrict__ bbox, const double* __restrict__ bcell,
+                             int64_t count, double* __restrict__ box, double* __restrict__ cell,
+                             float* __restrict__ box32, float* __restrict__ cell32) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  const double x = bbox[i], c = bcell[i];
+  const bool hi = i & 1;
+  box[i] = x;
+  cell[i] = c;
+  box32[i] = hi ? __double2float_ru(x) : __double2float_rd(x);
+  cell32[i] = hi ? __double2float_rd(c) : __double2float_ru(c);
+}
+
+// Per node: the record at its final place, a leaf's FP64 centre, and an internal node's
+// child-pair record (both children's outward FP32 boxes, ids, leaf flags and position
+// ranges), so one load serves a whole expansion.
 template <int D>
 __global__ void k_node_records(const NodeMeta* __restrict__ bmeta, int32_t n_nodes,
-                               const double* __restrict__ bbox, const double* __restrict__ bcell,
-                               NodeMeta* __restrict__ meta, double* __restrict__ box,
-                               double* __restrict__ cell, float* __restrict__ box32,
-                               float4* __restrict__ pair, float* __restrict__ cell32,
-                               double* __restrict__ centre) {
+                               const double* __restrict__ bbox, NodeMeta* __restrict__ meta,
+                               float4* __restrict__ pair, double* __restrict__ centre) {
   constexpr int NV = (D + 3) / 4;
   constexpr int PF = pair_f4(D);
   int32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n_nodes) return;
   const NodeMeta m = bmeta[a];
   meta[a] = m;
-  const int64_t b0 = (int64_t)a * 2 * D;
-  const double2* bx = reinterpret_cast<const double2*>(bbox + b0);
-  const double2* bc = reinterpret_cast<const double2*>(bcell + b0);
+  if (m.left < 0) {
+    const double2* bx = reinterpret_cast<const double2*>(bbox + (int64_t)a * 2 * D);
 #pragma unroll
-  for (int j = 0; j < D; ++j) {
-    const double2 x = bx[j], c = bc[j];
-    reinterpret_cast<double2*>(box + b0)[j] = x;
-    reinterpret_cast<double2*>(cell + b0)[j] = c;
-    reinterpret_cast<float2*>(box32 + b0)[j] =
-        make_float2(__double2float_rd(x.x), __double2float_ru(x.y));
-    reinterpret_cast<float2*>(cell32 + b0)[j] =
-        make_float2(__double2float_ru(c.x), __double2float_rd(c.y));
-    if (m.left < 0) centre[(int64_t)a * D + j] = leaf_centre(x.x, x.y);
+    for (int j = 0; j < D; ++j) centre[(int64_t)a * D + j] = leaf_centre(bx[j].x, bx[j].y);
+    return;
   }
-  if (m.left < 0) return;
   float4* rec = pair + (int64_t)a * PF;
   for (int side = 0; side < 2; ++side) {
     const double2* cx = reinterpret_cast<const double2*>(bbox + (int64_t)(m.left + side) * 2 * D);
@@ -1681,9 +1769,11 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   }
   k_point_records<D><<<(unsigned)cdiv(n, 256), 256, 0, s>>>(t->pts, n, t->pts64, t->pts32);
   CKD_LAUNCH_CHECK();
-  k_node_records<D><<<(unsigned)cdiv(n_nodes, 128), 128, 0, s>>>(
-      B.meta, n_nodes, B.box, B.cell, t->meta, t->box, t->cell, t->box32, t->pair, t->cell32,
-      t->centre);
+  k_node_boxes<<<(unsigned)cdiv((int64_t)n_nodes * 2 * D, 256), 256, 0, s>>>(
+      B.box, B.cell, (int64_t)n_nodes * 2 * D, t->box, t->cell, t->box32, t->cell32);
+  CKD_LAUNCH_CHECK();
+  k_node_records<D><<<(unsigned)cdiv(n_nodes, 128), 128, 0, s>>>(B.meta, n_nodes, B.box, t->meta,
+                                                                 t->pair, t->centre);
   CKD_LAUNCH_CHECK();
   CKD_CUDA(cudaStreamSynchronize(s));
   if (err == 3) return fail(CKD_ERR_TIMEOUT, "build: a tile copy into shared memory timed out");
