@@ -875,6 +875,179 @@ __global__ void __launch_bounds__(128) k_range_warp(
   }
 }
 
+// ---------------------------------------------------- ball, eight lanes per query
+// The same walk with G lanes of a warp per query, for large batches of small balls
+// on evenly filled trees (range_narrow), where rows are of like length: short ranges
+// and few pending nodes leave most lanes of a whole warp idle.  10^5 queries on 2^20
+// uniform points, 5 results each: count 262 -> 160, fill 279 -> 187 us.  Boxes, whose
+// sizes are known on the device only, keep the whole warp.
+template <int G>
+__host__ __device__ constexpr int range_stack(int depth) { return 2 * depth + 4 + 2 * G; }
+template <int G>
+constexpr int kRangeRun = G / 2;  // ranges that wait before they are scanned (count)
+
+template <class QT, bool FILL, int G>
+__global__ void __launch_bounds__(128) k_range_group(
+    TreeView tv, const double* __restrict__ Q, const int32_t* __restrict__ order, int64_t nq,
+    int depth, double r2, int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
+    int64_t* __restrict__ oidx, double* __restrict__ odist, int want_d2) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int NG = 128 / G, KL = kRangeRun<G> + 2 * G;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int scap = range_stack<G>(depth);
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), grp = threadIdx.x / G;
+  const int gsh = lane & ~(G - 1);
+  constexpr unsigned gm = (1u << G) - 1u;
+  const unsigned lt = (1u << gl) - 1u;
+  auto ballot = [&](bool p) -> unsigned { return (__ballot_sync(FULL, p) >> gsh) & gm; };
+  int2* stk = reinterpret_cast<int2*>(rsm) + (size_t)grp * scap;
+  int2* list = reinterpret_cast<int2*>(rsm) + (size_t)NG * scap + grp * KL;
+  const int64_t slot = (int64_t)blockIdx.x * NG + grp;
+  if (slot - grp % (32 / G) >= nq) return;  // a warp without queries leaves together
+  bool valid = slot < nq;
+  const int64_t qi = valid ? (order ? (int64_t)order[slot] : slot) : 0;
+  int64_t cur = FILL ? offsets[qi] : 0;
+  const int64_t cur_end = FILL ? offsets[qi + 1] : 0;
+  if (FILL && cur == cur_end) valid = false;
+  QT qt(tv, Q, qi, r2);
+  int64_t cnt = 0;  // per lane
+  int top = 0, nl = 0;
+  if (valid) {
+    const int2 first = qt.root(0, kBallRoot);
+    top = first.y == kNone ? 0 : 1;
+    if (gl == 0) stk[0] = first;
+  }
+  __syncwarp();
+  // the range of a group that holds flattened index t, from the lanes' inclusive counts
+  auto find = [&](int32_t inc, int32_t t) -> int {
+    int j = 0;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const int32_t v = __shfl_sync(FULL, inc, j + o - 1, G);
+      if (v <= t) j += o;
+    }
+    return j;
+  };
+  while (__any_sync(FULL, top > 0)) {
+    const int n = min(min(top, G), max(1, depth + 2 * G - top));
+    int2 e = make_int2(0, kNone);
+    if (gl < n) e = stk[top - 1 - gl];
+    __syncwarp();
+    top -= n;
+    int lead = 0;  // lanes below hold the ranges that come next (fill)
+    if (FILL) {
+      const unsigned nm = ballot(gl >= n || e.y == 0);
+      lead = nm ? __ffs(nm) - 1 : G;
+    }
+    int2 a = make_int2(0, kNone), b = make_int2(0, kNone);
+    if (gl < n && gl >= lead) {
+      if (e.y == 0) expand(qt, e.x, kBallUnit, a, b);
+      else a = e;
+    }
+    if (!FILL) {
+      if (a.y < 0 && a.y != kNone) {
+        cnt -= a.y;
+        a.y = kNone;
+      }
+      if (b.y < 0 && b.y != kNone) {
+        cnt -= b.y;
+        b.y = kNone;
+      }
+      const unsigned ga = ballot(a.y > 0), gb = ballot(b.y > 0);
+      const int o = nl + __popc(ga & lt) + __popc(gb & lt);
+      if (a.y > 0) list[o] = a;
+      if (b.y > 0) list[o + (a.y > 0 ? 1 : 0)] = b;
+      nl += __popc(ga) + __popc(gb);
+      if (a.y > 0) a.y = kNone;
+      if (b.y > 0) b.y = kNone;
+    }
+    // back onto the stack, the first lane's entries on top, left above right
+    const unsigned ma = ballot(a.y != kNone), mb = ballot(b.y != kNone);
+    const int total = __popc(ma) + __popc(mb);
+    const int above = __popc(ma & lt) + __popc(mb & lt);
+    if (a.y != kNone) stk[top + total - 1 - above] = a;
+    if (b.y != kNone) stk[top + total - 1 - above - (a.y != kNone ? 1 : 0)] = b;
+    top += total;
+    __syncwarp();
+    if (!FILL) {
+      const bool run = nl > 0 && (nl >= kRangeRun<G> || top == 0);
+      if (!__any_sync(FULL, run)) continue;
+      const int nls = run ? nl : 0;
+#pragma unroll 1
+      for (int u0 = 0; __any_sync(FULL, u0 < nls); u0 += G) {
+        const int2 x = u0 + gl < nls ? list[u0 + gl] : make_int2(0, 0);
+        int32_t inc = x.y;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+          const int32_t v = __shfl_up_sync(FULL, inc, o, G);
+          if (gl >= o) inc += v;
+        }
+        const int32_t tot = __shfl_sync(FULL, inc, G - 1, G);
+        const int32_t delta = x.x - (inc - x.y);
+#pragma unroll 2
+        for (int32_t t = gl; __any_sync(FULL, t - gl < tot); t += G) {
+          const int32_t p = __shfl_sync(FULL, delta, find(inc, t), G) + t;
+          double d2;
+          if (t < tot && qt.hit(p, false, d2)) ++cnt;
+        }
+      }
+      if (run) nl = 0;
+      __syncwarp();
+    } else {
+      if (!__any_sync(FULL, lead > 0)) continue;
+      const int32_t ct = gl < lead ? abs(e.y) : 0;
+      int32_t inc = ct;
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) {
+        const int32_t v = __shfl_up_sync(FULL, inc, o, G);
+        if (gl >= o) inc += v;
+      }
+      const int32_t tot = __shfl_sync(FULL, inc, G - 1, G);
+      const int32_t delta = e.x - (inc - ct);
+      const unsigned wholes = ballot(gl < lead && e.y < 0);
+#pragma unroll 2
+      for (int32_t t = gl; __any_sync(FULL, t - gl < tot); t += G) {
+        const int j = find(inc, t);
+        const int32_t p = __shfl_sync(FULL, delta, j, G) + t;
+        bool hit = t < tot;
+        double d2 = 0.0;
+        int32_t id = 0;
+        if (hit) {
+          id = CKD_LDT(&tv.ids[p]);
+          hit = qt.hit(p, (wholes >> j) & 1u, d2);
+        }
+        const unsigned hm = ballot(hit);
+        if (hit) {
+          const int64_t o = cur + __popc(hm & lt);
+          if (o < cur_end) {
+            oidx[o] = id;
+            if (QT::kDist) odist[o] = want_d2 ? d2 : sqrt(d2);
+          }
+        }
+        cur += __popc(hm);
+      }
+      if (cur >= cur_end) top = 0;  // all of the row's results are found
+    }
+  }
+  if (!FILL) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(FULL, cnt, o);
+    if (gl == 0 && valid) counts[qi] = cnt;
+  }
+}
+
+template <class QT, bool FILL>
+ckd_status range_group_launch(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
+                              double r2, int64_t* counts, const int64_t* offsets, int64_t* idx,
+                              double* dist, int want_d2, cudaStream_t s) {
+  constexpr int G = 8, NG = 128 / G;
+  const size_t sm = (size_t)NG * (range_stack<G>(t->depth) + kRangeRun<G> + 2 * G) * sizeof(int2);
+  k_range_group<QT, FILL, G><<<(unsigned)cdiv(nq, NG), 128, sm, s>>>(
+      t->view(), q, order, nq, t->depth, r2, counts, offsets, idx, dist, want_d2);
+  CKD_LAUNCH_CHECK();
+  return CKD_OK;
+}
+
 // rows of the fill split by length: heavy ones (>= kHeavyRow) to `heavy`, the rest
 // to `light`, both in the processing order (`order`, the leaf order when given)
 __global__ void k_split_rows(const int64_t* __restrict__ offsets, const int32_t* __restrict__ order,
@@ -1103,6 +1276,36 @@ __global__ void __launch_bounds__(128) k_box(TreeView tv, const double* __restri
   if (!FILL && valid) counts[bi] = cnt;
 }
 
+// Each row of a fill ordered by (d2, id), and the distances' roots.
+ckd_status sort_rows(const int64_t* offsets, int64_t nq, int64_t* idx, double* dist, int sms,
+                     cudaStream_t s) {
+  Scratch sc(s);
+  int32_t* big = nullptr;
+  int64_t* toff = nullptr;
+  unsigned long long* sel = nullptr;
+  CKD_CUDA(sc.alloc(&big, sizeof(int32_t) * nq));
+  CKD_CUDA(sc.alloc(&toff, sizeof(int64_t) * nq));
+  CKD_CUDA(sc.alloc(&sel, 2 * sizeof(unsigned long long)));
+  CKD_CUDA(cudaMemsetAsync(sel, 0, 2 * sizeof(unsigned long long), s));
+  k_sort_rows<<<(unsigned)cdiv(nq, 128), 128, 0, s>>>(offsets, nq, idx, dist, big, sel, toff);
+  CKD_LAUNCH_CHECK();
+  unsigned long long hs[2] = {0, 0};
+  CKD_CUDA(cudaMemcpyAsync(hs, sel, sizeof(hs), cudaMemcpyDeviceToHost, s));
+  CKD_CUDA(cudaStreamSynchronize(s));
+  if (hs[0] > 0) {
+    int64_t* tidx = nullptr;
+    double* tdist = nullptr;
+    if (hs[1] > 0) {
+      CKD_CUDA(sc.alloc(&tidx, sizeof(int64_t) * hs[1]));
+      CKD_CUDA(sc.alloc(&tdist, sizeof(double) * hs[1]));
+    }
+    const unsigned g = (unsigned)std::min<unsigned long long>(hs[0], (unsigned long long)sms * 8);
+    k_sort_big<<<g, 256, 0, s>>>(offsets, big, sel, toff, idx, dist, tidx, tdist);
+    CKD_LAUNCH_CHECK();
+  }
+  return CKD_OK;
+}
+
 // Batches up to which every query takes a warp of its own.  Beyond, the packet
 // kernel goes first: 32 queries adjacent in leaf order share their nodes, which is
 // faster while the balls are small against their spacing (10^6 queries on 2^20
@@ -1120,6 +1323,23 @@ constexpr int64_t kBallWarpMax = 200000;
 constexpr int kPacketBudget = 512;
 constexpr int64_t kPacketRow = 64;
 bool ball_warp_ok(const ckd_tree* t) { return t->screen_ok && t->depth < kBallReserve - 3; }
+
+// Whether a ball search takes eight lanes per query: small balls (the count of a
+// uniform filling of the tree's extent) in large batches on an even tree.  Measured on
+// uniform points, count + fill, a warp / eight lanes (us): 2^20 points, 5 results a
+// row: 8000 queries 77 / 88, 16000 120 / 100, 100000 541 / 347; 30 results: 32000 256 /
+// 251, 100000 724 / 573 (2^22 points: 304 / 368 and 839 / 806); 290 results and more, and
+// clustered points at any size: the warp.
+bool range_narrow(const ckd_tree* t, int64_t nq, double r) {
+  if (nq < 12000 || tree_uneven(t)) return false;
+  constexpr double kBall[9] = {1.0, 2.0, 3.14159, 4.18879, 4.93480, 5.26379, 5.16771, 4.72477, 4.05871};
+  double hits = (double)t->n * kBall[t->d];
+  for (int j = 0; j < t->d; ++j) {
+    if (!(t->extent[j] > 0.0)) return false;  // unknown (a loaded tree) or flat
+    hits *= r / t->extent[j];
+  }
+  return hits <= (nq >= 100000 ? 64.0 : 16.0);
+}
 
 template <int D, bool PER>
 ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
@@ -1143,6 +1363,14 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
   // kernel's rows before it for large batches and for trees that the warp kernel
   // does not take
   const bool warp = ball_warp_ok(t), packet = !warp || nq > kBallWarpMax;
+  if (warp && !packet && !qroot && range_narrow(t, nq, r)) {
+    if (!fill)
+      return range_group_launch<BallQuery<D, PER>, false>(t, q, order, nq, r2, counts, nullptr,
+                                                          nullptr, nullptr, 0, s);
+    CKD_TRY((range_group_launch<BallQuery<D, PER>, true>(t, q, order, nq, r2, nullptr, offsets, idx,
+                                                         dist, sorted ? 1 : 0, s)));
+    return sorted ? sort_rows(offsets, nq, idx, dist, sms, s) : CKD_OK;
+  }
   int32_t *heavy = nullptr, *light = nullptr;
   unsigned* cnt = nullptr;  // heavy rows, light rows, emission tasks
   CKD_CUDA(sc.alloc(&cnt, 3 * sizeof(unsigned)));
@@ -1208,32 +1436,7 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
                                                           dist, sorted ? 1 : 0);
     CKD_LAUNCH_CHECK();
   }
-  if (fill && sorted) {
-    int32_t* big = nullptr;
-    int64_t* toff = nullptr;
-    unsigned long long* sel = nullptr;
-    CKD_CUDA(sc.alloc(&big, sizeof(int32_t) * nq));
-    CKD_CUDA(sc.alloc(&toff, sizeof(int64_t) * nq));
-    CKD_CUDA(sc.alloc(&sel, 2 * sizeof(unsigned long long)));
-    CKD_CUDA(cudaMemsetAsync(sel, 0, 2 * sizeof(unsigned long long), s));
-    k_sort_rows<<<(unsigned)cdiv(nq, 128), 128, 0, s>>>(offsets, nq, idx, dist, big, sel, toff);
-    CKD_LAUNCH_CHECK();
-    unsigned long long hs[2] = {0, 0};
-    CKD_CUDA(cudaMemcpyAsync(hs, sel, sizeof(hs), cudaMemcpyDeviceToHost, s));
-    CKD_CUDA(cudaStreamSynchronize(s));
-    if (hs[0] > 0) {
-      int64_t* tidx = nullptr;
-      double* tdist = nullptr;
-      if (hs[1] > 0) {
-        CKD_CUDA(sc.alloc(&tidx, sizeof(int64_t) * hs[1]));
-        CKD_CUDA(sc.alloc(&tdist, sizeof(double) * hs[1]));
-      }
-      const unsigned g = (unsigned)std::min<unsigned long long>(hs[0], (unsigned long long)sms * 8);
-      k_sort_big<<<g, 256, 0, s>>>(offsets, big, sel, toff, idx, dist, tidx, tdist);
-      CKD_LAUNCH_CHECK();
-    }
-  }
-  return CKD_OK;
+  return fill && sorted ? sort_rows(offsets, nq, idx, dist, sms, s) : CKD_OK;
 }
 
 // Boxes per call up to which the warp kernel is used on a single tree; beyond, a lane

@@ -1766,6 +1766,7 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
     double b = std::max(std::fabs(rlo[j]), std::fabs(rhi[j])) + (t->periodic ? t->L[j] : 0.0);
     if (!(b < 1e18)) t->screen_ok = false;
     t->slack[j] = (float)(b * (1.0 + 1e-6));
+    t->extent[j] = t->periodic ? t->L[j] : rhi[j] - rlo[j];
   }
   k_point_records<D><<<(unsigned)cdiv(n, 256), 256, 0, s>>>(t->pts, n, t->pts64, t->pts32);
   CKD_LAUNCH_CHECK();

@@ -50,6 +50,45 @@ def test_gpu_ball_warp_matches_oracle(gpu, oracle, name, n, d, periodic, leaf, n
             np.testing.assert_array_equal(np.sort(dist[a:b]), np.sort(odist[a:b]))
 
 
+@pytest.mark.parametrize("sorted_", [False, True])
+@pytest.mark.parametrize("name,d,periodic,leaf,nq,hits", [
+    ("uniform3d", 3, False, 16, 11999, 4.0),   # below the eight lanes' batch
+    ("uniform3d", 3, False, 16, 12001, 4.0),   # eight lanes per query
+    ("uniform3d", 3, False, 1, 12001, 15.9),
+    ("uniform3d", 3, False, 16, 12001, 16.1),  # past their result count
+    ("uniform3d", 3, True, 40, 12003, 10.0),   # across the faces, leaves past a unit
+    ("lattice", 3, False, 16, 12001, 8.0),
+    ("lattice_periodic", 2, True, 16, 12001, 8.0),
+    ("d1", 1, True, 16, 12001, 3.0),
+    ("d5", 5, False, 16, 12001, 2.0),
+    ("uniform3d", 3, False, 16, 100001, 60.0),
+])
+def test_gpu_ball_eight_lanes(gpu, oracle, name, d, periodic, leaf, nq, hits, sorted_):
+    n = 20000
+    P = make_points(name, n, d, periodic)
+    rng = np.random.default_rng(53)
+    Q = np.concatenate([P[rng.integers(0, n, nq // 2)],
+                        rng.random((nq - nq // 2, d)) - (0.5 if periodic else 0.0)])
+    if not periodic:
+        Q[-1] = np.nan
+        Q[-2] = -1e40
+    side = 1.0 if periodic else P.max(0) - P.min(0)
+    ball = [0, 2.0, 3.14159, 4.18879, 0, 5.26379][d]
+    r = float((hits / (n * ball) * np.prod(np.broadcast_to(side, d))) ** (1.0 / d))
+    box = 1.0 if periodic else None
+    t = gpu.kdtree.build_kdtree(P, leaf=leaf, boxsize=box)
+    ooff, oidx, odist = oracle.OracleTree(P, leaf, box).ball_csr(Q, r, sorted=sorted_)
+    off, idx, dist = (x.cpu().numpy() for x in
+                      gpu.kdtree.ball_search_csr(t, Q, r, sorted=sorted_))
+    np.testing.assert_array_equal(off, ooff)
+    if sorted_ or not periodic:
+        np.testing.assert_array_equal(idx, oidx)
+        np.testing.assert_array_equal(dist, odist)
+    else:
+        for a, b in zip(off[:-1][::7], off[1:][::7]):
+            np.testing.assert_array_equal(np.sort(idx[a:b]), np.sort(oidx[a:b]))
+
+
 @pytest.mark.parametrize("name,r", [("uniform3d", 0.01), ("clustered_deep", 0.004)])
 def test_gpu_ball_batches_past_the_warp_rule(gpu, name, r):
     """A batch past the rule (packets first, heavy ones handed over on an uneven tree) gives
