@@ -118,12 +118,27 @@ size_t group_smem(int depth) {  // per block of 4 warps
          (group_stack(G, depth) * 8 + S::kBuf * 12 + S::kList * 12);
 }
 
-template <int D, bool PER, int G, int R>
+// What a bounded search gets besides: every query's squared bound and leaf, and the
+// list of the queries that hold fewer than k points within their bound.
+struct GroupBound {
+  const double* r2;
+  const int32_t* qleaf;
+  int32_t* miss;
+  unsigned* nmiss;
+};
+
+// BOUND: every list starts full of sentinels (r2, INT32_MAX) instead of HUGE, so
+// pruning starts at once, at the lowest ancestor of the query's leaf whose cell strictly
+// contains the ball; every point with d2 <= r2 is still accepted, so a list that ends
+// without a sentinel among its first k is exact.  The others are listed for a rerun and
+// their rows are not written.
+template <int D, bool PER, int G, int R, bool BOUND = false>
 __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __restrict__ Q,
                                                    const int32_t* __restrict__ order, int64_t nq,
                                                    int k, int depth, double* __restrict__ dist,
                                                    int64_t* __restrict__ idx,
-                                                   const int32_t* __restrict__ qroot) {
+                                                   const int32_t* __restrict__ qroot,
+                                                   GroupBound gb = GroupBound{}) {
   using S = GroupShape<G>;
   constexpr int NV = (D + 3) / 4, PF = pair_f4(D), U = S::U, NG = 4 * S::kQ;
   extern __shared__ __align__(16) unsigned char gsm[];
@@ -259,6 +274,38 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
   int nu = 0;  // ranges waiting to be scanned
   int top = 0;
   int32_t next = valid ? (qroot ? qroot[qi] : 0) : -1;  // next seed descent's subtree, -1: none
+  if (BOUND && valid) {
+    const double b = gb.r2[qi];
+    if (b < CKD_HUGE) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        L.d[r] = b;
+        L.i[r] = 0x7fffffff;
+      }
+      bd = b;
+      bid = 0x7fffffff;
+      wd32 = __double2float_ru(b);
+      const float r32 = __fsqrt_ru(wd32);
+      int32_t a = gb.qleaf[qi];
+      while (a >= 0) {
+        const float2* c = reinterpret_cast<const float2*>(tv.cell32 + (int64_t)a * 2 * D);
+        bool inside = true;
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          const float2 lh = CKD_LDT(c + j);
+          inside = inside && __fsub_rd(__fsub_rd(qs.q32[j], r32), qs.dlt[j]) > lh.x &&
+                   __fadd_ru(__fadd_ru(qs.q32[j], r32), qs.dlt[j]) < lh.y;
+        }
+        if (inside) break;
+        a = load_meta(tv.meta, a).parent;
+      }
+      // the subtree waits on the stack, its box untested
+      if (gl == 0) stk[0] = make_uint2((unsigned)(a < 0 ? next : a), kUntested);
+      top = 1;
+      next = -1;
+    }
+  }
+  __syncwarp();
   while (__any_sync(FULL, next >= 0 || top > 0)) {
     const bool act = next >= 0 || top > 0;
     if (next < 0 && top > 0 && bd == CKD_HUGE) next = (int32_t)stk[--top].x;
@@ -408,6 +455,14 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
     if (run) nu = 0;
     __syncwarp();
   }
+  if (BOUND) {  // a sentinel among the first k: fewer than k points within the bound
+    bool left = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) left = left || (r * G + gl < k && L.i[r] == 0x7fffffff);
+    const bool missed = ballot(left) != 0;
+    if (missed && gl == 0) gb.miss[atomicAdd(gb.nmiss, 1u)] = (int32_t)qi;
+    if (missed) return;
+  }
   if (!valid) return;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -451,6 +506,31 @@ ckd_status group_pick(const ckd_tree* t, const double* q, const int32_t* order, 
   return group_launch<D, PER, 32, 4>(t, q, order, nq, k, dist, idx, qroot, s);
 }
 
+template <int D, bool PER, int G, int R>
+ckd_status group_bound_launch(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
+                              int k, double* dist, int64_t* idx, const GroupBound& gb,
+                              cudaStream_t s) {
+  k_knn_group<D, PER, G, R, true><<<(unsigned)cdiv(nq, 4 * GroupShape<G>::kQ), 128,
+                                    group_smem<G>(t->depth), s>>>(
+      t->view(), q, order, nq, k, t->depth, dist, idx, nullptr, gb);
+  CKD_LAUNCH_CHECK();
+  return CKD_OK;
+}
+
+// the bounded search, k <= 64
+template <int D, bool PER>
+ckd_status group_bound_pick(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
+                            int k, double* dist, int64_t* idx, const GroupBound& gb,
+                            cudaStream_t s) {
+  if constexpr (D <= 4) {
+    if (k <= 16) return group_bound_launch<D, PER, 16, 1>(t, q, order, nq, k, dist, idx, gb, s);
+    if (k <= 32) return group_bound_launch<D, PER, 16, 2>(t, q, order, nq, k, dist, idx, gb, s);
+  } else {
+    if (k <= 32) return group_bound_launch<D, PER, 32, 1>(t, q, order, nq, k, dist, idx, gb, s);
+  }
+  return group_bound_launch<D, PER, 32, 2>(t, q, order, nq, k, dist, idx, gb, s);
+}
+
 }  // namespace
 
 // one translation unit instantiates each dimension (knn_group_*.cu)
@@ -460,6 +540,14 @@ ckd_status group_pick(const ckd_tree* t, const double* q, const int32_t* order, 
                              const int32_t* qroot, cudaStream_t s) {                             \
     return t->periodic ? group_pick<DD, true>(t, q, order, nq, k, dist, idx, qroot, s)           \
                        : group_pick<DD, false>(t, q, order, nq, k, dist, idx, qroot, s);         \
+  }                                                                                              \
+  ckd_status knn_group_bound_d##DD(const ckd_tree* t, const double* q, const int32_t* order,     \
+                                   int64_t nq, int k, double* dist, int64_t* idx,                \
+                                   const double* r2, const int32_t* qleaf, int32_t* miss,        \
+                                   unsigned* nmiss, cudaStream_t s) {                            \
+    const GroupBound gb{r2, qleaf, miss, nmiss};                                                 \
+    return t->periodic ? group_bound_pick<DD, true>(t, q, order, nq, k, dist, idx, gb, s)        \
+                       : group_bound_pick<DD, false>(t, q, order, nq, k, dist, idx, gb, s);      \
   }
 
 }  // namespace ckd

@@ -23,7 +23,10 @@ namespace ckd {
 // a group of lanes per query (ckd_knn_group.cuh): sorted rows, k <= 128
 #define CKD_KG(DD)                                                                            \
   ckd_status knn_group_d##DD(const ckd_tree*, const double*, const int32_t*, int64_t, int,    \
-                             double*, int64_t*, const int32_t*, cudaStream_t);
+                             double*, int64_t*, const int32_t*, cudaStream_t);                \
+  ckd_status knn_group_bound_d##DD(const ckd_tree*, const double*, const int32_t*, int64_t,   \
+                                   int, double*, int64_t*, const double*, const int32_t*,     \
+                                   int32_t*, unsigned*, cudaStream_t);
 CKD_KG(1) CKD_KG(2) CKD_KG(3) CKD_KG(4) CKD_KG(5) CKD_KG(6) CKD_KG(7) CKD_KG(8)
 #undef CKD_KG
 
@@ -325,6 +328,18 @@ ckd_status knn_group(const ckd_tree* t, const double* q, const int32_t* order, i
   return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
 }
 
+ckd_status knn_group_bound(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
+                           int k, double* dist, int64_t* idx, const double* r2,
+                           const int32_t* qleaf, int32_t* miss, unsigned* nmiss, cudaStream_t s) {
+  switch (t->d) {
+#define CKD_KG(DD) \
+  case DD: return knn_group_bound_d##DD(t, q, order, nq, k, dist, idx, r2, qleaf, miss, nmiss, s);
+    CKD_KG(1) CKD_KG(2) CKD_KG(3) CKD_KG(4) CKD_KG(5) CKD_KG(6) CKD_KG(7) CKD_KG(8)
+#undef CKD_KG
+  }
+  return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
+}
+
 // Whether the automatic choice takes a group of lanes per query
 // (ckd_knn_group.cuh) instead of the per-lane kernel.  Sorted rows only: an unsorted
 // row is in the order of its kernel's heap.  The lines are where the two cross,
@@ -347,6 +362,17 @@ bool use_knn_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
     return k >= 64 || nq <= (k <= 32 ? 300000 : 500000);
   }
   return k >= 48 || nq <= 32768 + 20000 * (int64_t)k;
+}
+
+// Whether the learned-bound search takes a group of lanes per query for its bounded
+// pass (us a call with ordering, network and reruns, per-lane / groups, 2^22 clustered
+// points): k = 8: 20k queries 475 / 376, 50k 543 / 541, 100k 560 / 790; k = 32: 50k
+// 972 / 710, 100k 1092 / 1090, 300k 2133 / 2559; k = 64: 100k 2484 / 1492, 3M 37532 /
+// 33563; 6-D: k = 8: 100k 2280 / 2102, k = 32: 300k 8838 / 8180.
+bool use_bound_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
+  if (!sorted || learned_kernel() != 3 || knn_variant() != 0 || g_stats_on) return false;
+  if (t->d <= 4) return k > 32 || nq <= 30000 + 2200 * (int64_t)k;
+  return k >= 48 || nq <= 32768 + 10000 * (int64_t)k;
 }
 
 // Kernel choice (ckd_set_knn_variant): 0 automatic, 1 FP64 packet traversal,
@@ -622,7 +648,9 @@ ckd_status knn_learned_impl(const ckd_tree* t, const ckd_mlp* net, const double*
     timing_begin(s);
     st = mlp_radius(t, net, q, order, qleaf, nq, k, r2, s);
   }
-  if (st == CKD_OK) {
+  if (st == CKD_OK && use_bound_group(t, nq, k, sorted)) {
+    st = knn_group_bound(t, q, order, nq, k, dist, idx, r2, qleaf, miss, nmiss, s);
+  } else if (st == CKD_OK) {
     const int nw = std::min(4, knn_warps_per_block());
     const unsigned blocks = (unsigned)cdiv(cdiv(nq, 32), nw);
     size_t sm = (size_t)nw * compact_heap_bytes(k);

@@ -108,3 +108,28 @@ def test_gpu_knn_group_narrow_groups(gpu, oracle, d, leaf, k):
         gd, gi = gpu.kdtree.knn_search(t, q[part], k)
         np.testing.assert_array_equal(gi, oi[part])
         np.testing.assert_array_equal(gd, od[part])
+
+
+@pytest.mark.parametrize("margin", [-2.0, 0.0, 3.0], ids=["tight", "near", "loose"])
+@pytest.mark.parametrize("name,d,periodic,k", [
+    ("uniform3d", 3, False, 1), ("periodic_clustered", 3, True, 16), ("lattice_periodic", 3, True, 17),
+    ("clustered_dup", 3, False, 32), ("uniform3d", 3, False, 33), ("lattice", 2, False, 64),
+    ("d5", 5, True, 20), ("d6", 6, False, 48), ("tiny", 3, False, 30),
+])
+def test_gpu_knn_group_bounded(gpu, oracle, name, d, periodic, k, margin):
+    """The bounded search is exact whatever the bound: a hardly trained network, margins that
+    leave most queries to the rerun or none."""
+    from cosmokdtree_b200.learned import LearnedBound
+    n = 20 if name == "tiny" else 6000
+    P = make_points(name, n, d, periodic)
+    rng = np.random.default_rng(37)
+    Q = np.concatenate([P[rng.integers(0, n, 200)], rng.random((203, d)) - (0.5 if periodic else 0.0)])
+    box = 1.0 if periodic else None
+    t = gpu.kdtree.build_kdtree(P, boxsize=box)
+    net = LearnedBound(seed=3)
+    net.fit(t, P[:min(n, 500)], min(k, n), epochs=2, batch=64)
+    net.set_margin(margin)
+    gd, gi = net.knn(t, Q, k)
+    od, oi = oracle.OracleTree(P, 16, box).knn(Q, k)
+    np.testing.assert_array_equal(gi, oi)
+    np.testing.assert_array_equal(gd, od)
