@@ -4,17 +4,21 @@
 // distance (reference arithmetic) is <= radius^2 (inclusive, :1126, :1175).  The
 // reference's "fully inside" shortcut (:1116-1118, :1332-1366) selects exactly
 // the same points, because a node's max-distance bound is never below the
-// computed distance of a point inside it; the count pass uses it (with the
-// tight box) to skip distance work, on periodic trees too when the box lies
-// within half a box side of the query on every axis (box_maxd2_near).  Traversal is left child first, so the
-// unsorted order of a row is the reference's non-periodic order (left-first DFS,
-// leaf order).  sorted=1 orders each row by (d2, id).
+// computed distance of a point inside it; the searches use it with the tight box
+// to skip distance work, on periodic trees too when the box lies within half a box
+// side of the query on every axis.  An unsorted row is in leaf order, which is the
+// reference's non-periodic order (left-first depth-first walk).  sorted=1 orders each
+// row by (d2, id).
 //
 // Box (cosmokdtree.f90:1220-1328): descend left iff box_lo[axis] < split, right
 // iff box_hi[axis] > split (strict), leaf test lo <= x <= hi on every axis
-// (inclusive), no periodic wrap.  Each lane carries one box; the warp walks the
-// union of the lanes' paths with a per-entry lane mask, left first, so every
-// row comes out in the reference's order.
+// (inclusive), no periodic wrap.  Rows are in leaf order, the reference's.
+//
+// Kernels: k_range_warp (balls and boxes, a warp per query), k_range_group (small
+// balls, eight lanes per query), k_ball (packets of 32 queries: the first pass of very
+// large batches, and trees too deep or coordinates too large for the FP32 tests),
+// k_ball_fill_warp (heavy rows of those trees), k_box_lane (very large batches of
+// boxes), k_box (boxes on trees deeper than its stack).
 #include <algorithm>
 
 #include "ckd_common.cuh"
@@ -804,7 +808,7 @@ __global__ void __launch_bounds__(128) k_range_warp(
       } else if (lead > 0) {
         if (lead == 1) {  // a large whole range: tasks, unless their buffer is full
           const int32_t st = __shfl_sync(FULL, e.x, 0), ct = -__shfl_sync(FULL, e.y, 0);
-          if (ct >= kTaskMin && cur < cur_end) {
+          if (tasks && ct >= kTaskMin && cur < cur_end) {
             const int64_t len = min((int64_t)ct, cur_end - cur);
             const unsigned nt = (unsigned)((len + kTaskChunk - 1) / kTaskChunk);
             unsigned tb = 0;
@@ -1373,8 +1377,10 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
   }
   int32_t *heavy = nullptr, *light = nullptr;
   unsigned* cnt = nullptr;  // heavy rows, light rows, emission tasks
-  CKD_CUDA(sc.alloc(&cnt, 3 * sizeof(unsigned)));
-  if (packet || fill) CKD_CUDA(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), s));
+  if (packet || fill) {
+    CKD_CUDA(sc.alloc(&cnt, 3 * sizeof(unsigned)));
+    CKD_CUDA(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), s));
+  }
   if (packet) {
     if (warp || fill) CKD_CUDA(sc.alloc(&heavy, sizeof(int32_t) * nq));
     if (fill) {
@@ -1465,16 +1471,24 @@ ckd_status box_launch(const ckd_tree* t, const double* boxes, int64_t nb, bool f
     Scratch sc(s);
     const unsigned task_cap =
         (unsigned)std::min<int64_t>(kTaskCap, std::max<int64_t>(1 << 16, nb * 64));
-    EmitTask* tasks = nullptr;  // and their counter behind them
-    CKD_CUDA(sc.alloc(&tasks, sizeof(EmitTask) * (task_cap + 1)));
-    unsigned* ntask = reinterpret_cast<unsigned*>(tasks + task_cap);
-    CKD_CUDA(cudaMemsetAsync(ntask, 0, sizeof(unsigned), s));
+    // tasks and their counter behind them; without room for them the warps copy
+    // whole ranges themselves
+    EmitTask* tasks = nullptr;
+    unsigned* ntask = nullptr;
+    if (sc.alloc(&tasks, sizeof(EmitTask) * (task_cap + 1)) == cudaSuccess) {
+      ntask = reinterpret_cast<unsigned*>(tasks + task_cap);
+      CKD_CUDA(cudaMemsetAsync(ntask, 0, sizeof(unsigned), s));
+    } else {
+      cudaGetLastError();
+    }
     k_range_warp<BoxQuery<D>, true><<<wb, threads, 0, s>>>(tv, boxes, nullptr, nb, 0.0, nullptr,
                                                            offsets, idx, nullptr, 0, tasks, ntask,
                                                            task_cap, broot);
     CKD_LAUNCH_CHECK();
-    k_box_emit<<<(unsigned)sms * 8, 128, 0, s>>>(tv.ids, tasks, ntask, task_cap, idx);
-    CKD_LAUNCH_CHECK();
+    if (tasks) {
+      k_box_emit<<<(unsigned)sms * 8, 128, 0, s>>>(tv.ids, tasks, ntask, task_cap, idx);
+      CKD_LAUNCH_CHECK();
+    }
     return CKD_OK;
   }
   if (t->depth < kBoxLaneStack - 2) {

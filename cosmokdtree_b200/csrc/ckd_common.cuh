@@ -56,13 +56,13 @@ void note_launch();
   } while (0)
 
 // kNN kernel choice (ckd_set_knn_variant): 0 automatic, 1 FP64 packet traversal,
-// 7/8 per-lane compact heap, 9 warp-converged
+// 7/8 per-lane compact heap
 int knn_variant();
 // tuning knobs (see ckd_set_tuning): blocks-per-SM cap (0 = none), warps per block
 int knn_blocks_per_sm();
 int knn_warps_per_block();
 // learned-bound search kernel: 0 bounded per-lane with compact heap (k_knn_lane2),
-// 3 as 0 with child-pair-record descent (default), 4 bounded warp-converged
+// 3 as 0 with child-pair-record descent, groups of lanes where they are faster (default)
 int learned_kernel();
 // query leaf ordering before a search: 0 automatic, 1 always, 2 never
 int query_order_mode();

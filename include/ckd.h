@@ -102,9 +102,11 @@ ckd_status ckd_knn_ordered(const ckd_tree* tree, const double* q_dev, int64_t nq
 /* Number of CUDA kernels this library has launched in this process. */
 int64_t ckd_launch_count(void);
 
-/* Process-wide kNN kernel choice (no reference counterpart): 0 = automatic (8
- * when k <= 64, the coordinates allow the FP32 screen and the tree is shallow
- * enough; 1 otherwise), 1 = FP64 packet
+/* Process-wide kNN kernel choice (no reference counterpart): 0 = automatic (sorted
+ * rows: 32, 16 or 8 lanes of a warp per query for small and middle batches, for
+ * 64 <= k <= 128, and for most k above three dimensions; else 8 when k <= 64; both
+ * when the coordinates allow the FP32 screen and the tree is shallow enough; 1
+ * otherwise), 1 = FP64 packet
  * traversal, 7 = per-lane traversal with 8-byte heap entries (FP32 key +
  * position, exact tie resolution), 8 = 7 expanding nodes from child-pair records.
  * Every variant returns the same exact result. */
@@ -115,12 +117,13 @@ ckd_status ckd_set_knn_variant(int variant);
  * key 1: cap on resident blocks per SM for the per-lane kNN kernel (0 = as many
  * as fit); key 2: warps per block of the per-lane kNN kernel (1..8, default 2,
  * at most 4 used); key 4: search kernel of ckd_knn_learned (0 = bounded per-lane
- * traversal; 3 = 0 with child-pair-record descent, default); key 6: ordering of queries by leaf before kNN and ball
- * searches (0 = automatic, default; 1 = always; 2 = never); key 7: inference of
+ * traversal; 3 = 0 with child-pair-record descent, and groups of lanes per query for
+ * small batches and k > 32, default); key 6: ordering of queries by leaf before kNN and
+ * ball searches (0 = automatic, default; 1 = always; 2 = never); key 7: inference of
  * the learned-bound network (0 = FP32 FMAs; 1 = tensor cores, tcgen05 MMAs on
  * BF16 activations, default); key 8: box search of up to 32768 boxes per call
- * on one tree, and of any number on a forest (1 = a warp per box, frontier
- * expanded a level at a time, default; 0 = a lane per box); key 9: cap in MiB on the device memory the library's pool hands out
+ * on one tree, and of any number on a forest (1 = a warp per box, default; 0 = a
+ * lane per box); key 9: cap in MiB on the device memory the library's pool hands out
  * at any time on the current device (0 = none, default): an allocation past it
  * fails with CKD_ERR_OOM and the call returns everything it had taken; key 10:
  * how long (ms, default 20000) an idle CTA of the persistent forest launch waits

@@ -60,3 +60,22 @@ def test_gpu_box_whole_ranges_as_tasks(gpu):
     assert torch.equal(off, torch.arange(nb + 1, device="cuda") * n)
     assert torch.equal(idx[0].sort().values, torch.arange(n, device="cuda"))
     assert bool((idx == idx[0]).all())
+
+
+def test_gpu_box_fill_without_room_for_tasks(gpu):
+    """With the pool capped at what it holds, the fill copies whole ranges itself."""
+    import torch
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(6)
+    P = torch.from_numpy(rng.random((300000, 3))).cuda()
+    t = gpu.kdtree.build_kdtree(P)
+    B = torch.tensor([[0.1, 0.9] * 3, [-1.0, 2.0] * 3, [0.4, 0.45] * 3], dtype=torch.float64,
+                     device="cuda")
+    want = gpu.kdtree.box_search_csr(t, B)
+    _lib.check(L.ckd_set_tuning(9, 1))  # 1 MiB, less than the tree itself holds
+    try:
+        got = gpu.kdtree.box_search_csr(t, B)
+    finally:
+        _lib.check(L.ckd_set_tuning(9, 0))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
