@@ -98,8 +98,10 @@ SIGNATURES = {
     "ckd_knn_stats": [_int, _pi64],
     "ckd_ball_count": [_vp, _vp, _i64, _dbl, _vp, _vp],
     "ckd_ball_fill": [_vp, _vp, _i64, _dbl, _int, _vp, _vp, _vp, _vp],
+    "ckd_ball_fill_sized": [_vp, _vp, _i64, _dbl, _int, _i64, _vp, _vp, _vp, _vp],
     "ckd_box_count": [_vp, _vp, _i64, _vp, _vp],
     "ckd_box_fill": [_vp, _vp, _i64, _vp, _vp, _vp],
+    "ckd_box_fill_sized": [_vp, _vp, _i64, _i64, _vp, _vp, _vp],
     "ckd_ball_count_host": [_vp, _vp, _i64, _dbl, _vp, _vp],
     "ckd_ball_fill_host": [_vp, _vp, _i64, _dbl, _int, _vp, _vp, _vp, _vp],
     "ckd_box_count_host": [_vp, _vp, _i64, _vp, _vp],
@@ -115,8 +117,10 @@ SIGNATURES = {
     "ckd_forest_knn": [_vp, _vp, _vp, _i64, _int, _int, _vp, _vp, _vp],
     "ckd_forest_box_count": [_vp, _vp, _vp, _i64, _vp, _vp],
     "ckd_forest_box_fill": [_vp, _vp, _vp, _i64, _vp, _vp, _vp],
+    "ckd_forest_box_fill_sized": [_vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp],
     "ckd_forest_ball_count": [_vp, _vp, _vp, _i64, _dbl, _vp, _vp],
     "ckd_forest_ball_fill": [_vp, _vp, _vp, _i64, _dbl, _int, _vp, _vp, _vp, _vp],
+    "ckd_forest_ball_fill_sized": [_vp, _vp, _vp, _i64, _dbl, _int, _i64, _vp, _vp, _vp, _vp],
     "ckd_mlp_create": [ctypes.c_uint64, ctypes.POINTER(_vp)],
     "ckd_mlp_free": [_vp],
     "ckd_mlp_get": [_vp, _vp, _vp, _vp, _vp],

@@ -142,10 +142,10 @@ ckd_status knn_learned(const ckd_tree* t, const ckd_mlp* net, const double* q, i
 ckd_status ball_run(const ckd_tree* t, const double* q, int64_t nq, double r, bool fill, int sorted,
                     int64_t* counts, const int64_t* offsets, int64_t* idx, double* dist,
                     cudaStream_t s,
-                    const int32_t* qroot = nullptr);
+                    const int32_t* qroot = nullptr, int64_t total = -1);
 ckd_status box_run(const ckd_tree* t, const double* boxes, int64_t nb, bool fill, int64_t* counts,
                    const int64_t* offsets, int64_t* idx, cudaStream_t s,
-                   const int32_t* broot = nullptr);
+                   const int32_t* broot = nullptr, int64_t total = -1);
 ckd_status forest_knn(const ckd_tree* t, const double* q, const int32_t* qroot, int64_t nq, int k,
                       int sorted, double* dist, int64_t* idx, cudaStream_t s);
 
@@ -317,7 +317,7 @@ ckd_status ckd_forest_knn(const ckd_tree* t, const double* q, const int64_t* q_o
 
 static ckd_status forest_box(const ckd_tree* t, const double* boxes, const int64_t* b_offsets,
                              int64_t nb, bool fill, int64_t* counts, const int64_t* offsets,
-                             int64_t* idx, void* stream) {
+                             int64_t* idx, void* stream, int64_t total = -1) {
   CKD_TRY(check_forest(t));
   if (nb < 0) return fail(CKD_ERR_BAD_ARG, "negative box count");
   if (nb == 0) return CKD_OK;
@@ -327,7 +327,7 @@ static ckd_status forest_box(const ckd_tree* t, const double* boxes, const int64
   int32_t* broot = nullptr;
   CKD_CUDA(dev_alloc((void**)&broot, sizeof(int32_t) * nb, s));
   ckd_status st = csr_owner(b_offsets, (int32_t)t->n_trees, nb, broot, s);
-  if (st == CKD_OK) st = box_run(t, boxes, nb, fill, counts, offsets, idx, s, broot);
+  if (st == CKD_OK) st = box_run(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
   dev_free(broot, s);
   return st;
 }
@@ -339,12 +339,19 @@ ckd_status ckd_forest_box_count(const ckd_tree* t, const double* boxes, const in
 
 ckd_status ckd_forest_box_fill(const ckd_tree* t, const double* boxes, const int64_t* b_offsets,
                                int64_t nb, const int64_t* offsets, int64_t* idx, void* stream) {
-  return forest_box(t, boxes, b_offsets, nb, true, nullptr, offsets, idx, stream);
+  return ckd_forest_box_fill_sized(t, boxes, b_offsets, nb, -1, offsets, idx, stream);
+}
+
+ckd_status ckd_forest_box_fill_sized(const ckd_tree* t, const double* boxes,
+                                     const int64_t* b_offsets, int64_t nb, int64_t total,
+                                     const int64_t* offsets, int64_t* idx, void* stream) {
+  return forest_box(t, boxes, b_offsets, nb, true, nullptr, offsets, idx, stream, total);
 }
 
 static ckd_status forest_ball(const ckd_tree* t, const double* q, const int64_t* q_offsets,
                               int64_t nq, double radius, bool fill, int sorted, int64_t* counts,
-                              const int64_t* offsets, int64_t* idx, double* dist, void* stream) {
+                              const int64_t* offsets, int64_t* idx, double* dist, void* stream,
+                              int64_t total = -1) {
   CKD_TRY(check_forest(t));
   if (!(radius > 0) || !std::isfinite(radius))
     return fail(CKD_ERR_BAD_ARG, "Radius must be a positive number");
@@ -358,7 +365,7 @@ static ckd_status forest_ball(const ckd_tree* t, const double* q, const int64_t*
   CKD_CUDA(dev_alloc((void**)&qroot, sizeof(int32_t) * nq, s));
   ckd_status st = csr_owner(q_offsets, (int32_t)t->n_trees, nq, qroot, s);
   if (st == CKD_OK)
-    st = ball_run(t, q, nq, radius, fill, sorted, counts, offsets, idx, dist, s, qroot);
+    st = ball_run(t, q, nq, radius, fill, sorted, counts, offsets, idx, dist, s, qroot, total);
   dev_free(qroot, s);
   return st;
 }
@@ -372,8 +379,16 @@ ckd_status ckd_forest_ball_count(const ckd_tree* t, const double* q, const int64
 ckd_status ckd_forest_ball_fill(const ckd_tree* t, const double* q, const int64_t* q_offsets,
                                 int64_t nq, double radius, int sorted, const int64_t* offsets,
                                 int64_t* idx, double* dist, void* stream) {
-  return forest_ball(t, q, q_offsets, nq, radius, true, sorted, nullptr, offsets, idx, dist,
-                     stream);
+  return ckd_forest_ball_fill_sized(t, q, q_offsets, nq, radius, sorted, -1, offsets, idx, dist,
+                                    stream);
+}
+
+ckd_status ckd_forest_ball_fill_sized(const ckd_tree* t, const double* q, const int64_t* q_offsets,
+                                      int64_t nq, double radius, int sorted, int64_t total,
+                                      const int64_t* offsets, int64_t* idx, double* dist,
+                                      void* stream) {
+  return forest_ball(t, q, q_offsets, nq, radius, true, sorted, nullptr, offsets, idx, dist, stream,
+                     total);
 }
 
 ckd_status ckd_pool_usage(int64_t* used, int64_t* reserved) {
@@ -667,6 +682,12 @@ ckd_status ckd_ball_count(const ckd_tree* t, const double* q, int64_t nq, double
 
 ckd_status ckd_ball_fill(const ckd_tree* t, const double* q, int64_t nq, double radius, int sorted,
                          const int64_t* offsets, int64_t* idx, double* dist, void* stream) {
+  return ckd_ball_fill_sized(t, q, nq, radius, sorted, -1, offsets, idx, dist, stream);
+}
+
+ckd_status ckd_ball_fill_sized(const ckd_tree* t, const double* q, int64_t nq, double radius,
+                               int sorted, int64_t total, const int64_t* offsets, int64_t* idx,
+                               double* dist, void* stream) {
   CKD_TRY(check_single(t));
   if (!(radius > 0) || !std::isfinite(radius))
     return fail(CKD_ERR_BAD_ARG, "Radius must be a positive number");
@@ -674,7 +695,7 @@ ckd_status ckd_ball_fill(const ckd_tree* t, const double* q, int64_t nq, double 
   if (nq == 0) return CKD_OK;
   if (!q || !offsets || !idx || !dist) return fail(CKD_ERR_BAD_ARG, "null query or output pointer");
   return ball_run(t, q, nq, radius, true, sorted, nullptr, offsets, idx, dist,
-                  (cudaStream_t)stream);
+                  (cudaStream_t)stream, nullptr, total);
 }
 
 ckd_status ckd_box_count(const ckd_tree* t, const double* boxes, int64_t nb, int64_t* counts,
@@ -688,11 +709,16 @@ ckd_status ckd_box_count(const ckd_tree* t, const double* boxes, int64_t nb, int
 
 ckd_status ckd_box_fill(const ckd_tree* t, const double* boxes, int64_t nb, const int64_t* offsets,
                         int64_t* idx, void* stream) {
+  return ckd_box_fill_sized(t, boxes, nb, -1, offsets, idx, stream);
+}
+
+ckd_status ckd_box_fill_sized(const ckd_tree* t, const double* boxes, int64_t nb, int64_t total,
+                              const int64_t* offsets, int64_t* idx, void* stream) {
   CKD_TRY(check_single(t));
   if (nb < 0) return fail(CKD_ERR_BAD_ARG, "negative box count");
   if (nb == 0) return CKD_OK;
   if (!boxes || !offsets || !idx) return fail(CKD_ERR_BAD_ARG, "null box or output pointer");
-  return box_run(t, boxes, nb, true, nullptr, offsets, idx, (cudaStream_t)stream);
+  return box_run(t, boxes, nb, true, nullptr, offsets, idx, (cudaStream_t)stream, nullptr, total);
 }
 
 // ---------------------------------------------- two-phase CSR on host buffers
@@ -775,7 +801,7 @@ ckd_status ckd_ball_fill_host(const ckd_tree* t, const double* q, int64_t nq, do
   CKD_CUDA(cudaMemcpyAsync(off, offsets_host, sizeof(int64_t) * (nq + 1), cudaMemcpyHostToDevice,
                            sc.s));
   if (total > 0) {
-    CKD_TRY(ball_run(t, dq, nq, radius, true, sorted, nullptr, off, di, dd, sc.s));
+    CKD_TRY(ball_run(t, dq, nq, radius, true, sorted, nullptr, off, di, dd, sc.s, nullptr, total));
     CKD_CUDA(cudaMemcpyAsync(idx_host, di, sizeof(int64_t) * total, cudaMemcpyDeviceToHost, sc.s));
     CKD_CUDA(cudaMemcpyAsync(dist_host, dd, sizeof(double) * total, cudaMemcpyDeviceToHost, sc.s));
   }
@@ -823,7 +849,7 @@ ckd_status ckd_box_fill_host(const ckd_tree* t, const double* boxes, int64_t nb,
   CKD_CUDA(cudaMemcpyAsync(off, offsets_host, sizeof(int64_t) * (nb + 1), cudaMemcpyHostToDevice,
                            sc.s));
   if (total > 0) {
-    CKD_TRY(box_run(t, db, nb, true, nullptr, off, di, sc.s));
+    CKD_TRY(box_run(t, db, nb, true, nullptr, off, di, sc.s, nullptr, total));
     CKD_CUDA(cudaMemcpyAsync(idx_host, di, sizeof(int64_t) * total, cudaMemcpyDeviceToHost, sc.s));
   }
   CKD_CUDA(cudaStreamSynchronize(sc.s));

@@ -519,6 +519,7 @@ struct BallQuery {
     d2 = point_d2_rec<D, PER>(tv, q, p);
     return whole || d2 <= rr;
   }
+  __device__ __forceinline__ void resume(int32_t) {}
   // The subtree that holds the ball, from a root: while the split plane is further
   // than r from the query, only its side of it can hold results.  The points left
   // of a split lie at or below it, those on the right at or above it, and rounding
@@ -598,6 +599,8 @@ struct BoxQuery {
     gl = bl < m.split;
     gr = bh > m.split;
   }
+  // for entries of an earlier walk: paths are checked from the root
+  __device__ __forceinline__ void resume(int32_t node) { top = node; }
   __device__ __forceinline__ int2 root(int32_t node, int32_t unit) {
     NodeMeta m = load_meta(tv.meta, node);
     while (m.left >= 0 && m.count > unit) {
@@ -703,35 +706,137 @@ constexpr int kBallListRun = 16;   // ranges that wait before they are scanned (
 constexpr int32_t kBallUnit = 32;  // subtrees of at most this many points are scanned as a range
 constexpr int32_t kBallRoot = 64;  // and of this many where the descent from the root ends
 
+// What the fill's walk leaves of a long row: its pending entries, in order and refined
+// by breadth-first levels, as parts. A second launch counts their results, a third
+// writes each part behind those before it, a warp per part.  One warp walked the row
+// alone before, and the longest rows were all that ran at the end of a pass (10 % of
+// the warps active): 4001 balls of 20000 results on 2^22 clustered points, fill 0.93 ->
+// 0.67 ms with the recount; 12800 boxes on 200 trees 2.26 -> 0.99.  A budget of 32 or 128
+// steps and 64 entries are within 10 %.  The count pass, which has nothing to tell long
+// rows by, walks them whole; parts shared by the warps of a block only were up to 1.5
+// times slower than whole rows.
+struct Part {
+  int64_t base;    // where the row's first part begins
+  int32_t head;    // the row's first part
+  int32_t qi;      // -1: none
+  int32_t x, y;    // the entry
+  int32_t count;   // its results
+  int32_t pad;
+};
+constexpr int kPartMin = 128;     // entries that a row is refined to, at least, where it can be
+constexpr int kPartBudget = 64;   // steps (32 lanes' work each) before a row is cut
+struct Parts {
+  Part* list;       // null: rows are not cut
+  unsigned* n;
+  unsigned cap;
+  bool run;         // the rows of this launch are parts
+};
+
+// The row's pending entries made parts; false when they do not fit.
+template <class QT>
+__device__ __forceinline__ bool cut_row(const QT& bq, const Parts& parts, int64_t qi, int64_t cur,
+                                       int2*& stk, int2* tmp, int& top) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  if (!parts.list || parts.run || *(volatile unsigned*)parts.n >= parts.cap) return false;
+  bool more = true;
+  while (more && top < kPartMin) {
+    int m = 0;
+    more = false;
+#pragma unroll 1
+    for (int u0 = 0; u0 < top; u0 += 32) {
+      int2 a = make_int2(0, kNone), b = make_int2(0, kNone);
+      const int2 e = u0 + lane < top ? stk[u0 + lane] : make_int2(0, kNone);
+      if (e.y == 0) expand(bq, e.x, kBallUnit, a, b);
+      else a = e;
+      const unsigned ma = __ballot_sync(FULL, a.y != kNone);
+      const unsigned mb = __ballot_sync(FULL, b.y != kNone);
+      const int o = m + __popc(ma & lt) + __popc(mb & lt);  // right below left
+      if (b.y != kNone) tmp[o] = b;
+      if (a.y != kNone) tmp[o + (b.y != kNone ? 1 : 0)] = a;
+      m += __popc(ma) + __popc(mb);
+      more = more || __any_sync(FULL, a.y == 0 || b.y == 0);
+    }
+    __syncwarp();
+    int2* const t = stk;
+    stk = tmp;
+    tmp = t;
+    top = m;
+  }
+  if (top == 0) return true;
+  unsigned pb = 0;
+  if (lane == 0) pb = atomicAdd(parts.n, (unsigned)top);
+  pb = __shfl_sync(FULL, pb, 0);
+  const bool fits = pb + (unsigned)top <= parts.cap;
+  for (int i = lane; i < top && pb + i < parts.cap; i += 32) {
+    Part p;
+    p.base = cur;
+    p.head = (int32_t)pb;
+    p.qi = fits ? (int32_t)qi : -1;
+    p.x = stk[top - 1 - i].x;
+    p.y = stk[top - 1 - i].y;
+    p.count = 0;
+    p.pad = 0;
+    parts.list[pb + i] = p;
+  }
+  __syncwarp();
+  return fits;
+}
+
 template <class QT, bool FILL>
 __global__ void __launch_bounds__(128) k_range_warp(
     TreeView tv, const double* __restrict__ Q, const int32_t* __restrict__ order, int64_t nq,
     double r2, int64_t* __restrict__ counts,
     const int64_t* __restrict__ offsets, int64_t* __restrict__ oidx, double* __restrict__ odist,
     int want_d2, EmitTask* __restrict__ tasks, unsigned* __restrict__ n_tasks, unsigned task_cap,
-    const int32_t* __restrict__ qroot, const unsigned* __restrict__ n_rows = nullptr) {
+    const int32_t* __restrict__ qroot, const unsigned* __restrict__ n_rows = nullptr,
+    const Parts parts = Parts{}) {
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ int2 s_stk[4][kBallStack];
+  __shared__ int2 s_stk[4][FILL ? 2 : 1][kBallStack];
   __shared__ int2 s_list[4][FILL ? 1 : kBallList];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  int2* stk = s_stk[w];
+  int2* stk = s_stk[w][0];
   int2* list = s_list[w];
-  const int64_t nr = n_rows ? (int64_t)*n_rows : nq;
+  const int64_t nr = parts.run ? (int64_t)min(*parts.n, parts.cap) : n_rows ? (int64_t)*n_rows : nq;
   for (int64_t r = (int64_t)blockIdx.x * 4 + w; r < nr; r += (int64_t)gridDim.x * 4) {
-    const int64_t qi = order ? (int64_t)order[r] : r;
-    int64_t cur = FILL ? offsets[qi] : 0;
-    const int64_t cur_end = FILL ? offsets[qi + 1] : 0;
+    int64_t qi, cur = 0, cur_end = 0;
+    int2 first;
+    if (parts.run) {
+      const Part p = parts.list[r];
+      qi = p.qi;
+      if (qi < 0) continue;
+      first = make_int2(p.x, p.y);
+      if (FILL) {
+        for (int64_t i = p.head + lane; i < r; i += 32) cur += parts.list[i].count;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) cur += __shfl_xor_sync(FULL, cur, o);
+        cur += p.base;
+        cur_end = cur + p.count;
+      }
+    } else {
+      qi = order ? (int64_t)order[r] : r;
+      if (FILL) {
+        cur = offsets[qi];
+        cur_end = offsets[qi + 1];
+      }
+    }
     if (FILL && cur == cur_end) continue;
     QT bq(tv, Q, qi, r2);
     int64_t cnt = 0;  // per lane
-    int top = 1, nl = 0;
-    const int2 first = bq.root(qroot ? qroot[qi] : 0, kBallRoot);
+    int top = 1, nl = 0, work = 0;
+    if (parts.run) bq.resume(qroot ? qroot[qi] : 0);
+    else first = bq.root(qroot ? qroot[qi] : 0, kBallRoot);
     if (first.y == kNone) top = 0;
     if (lane == 0) stk[0] = first;
     __syncwarp();
     while (top > 0) {
       if (FILL && cur >= cur_end) break;  // all of the row's results are found
+      if (FILL && ++work > kPartBudget) {
+        work = 0;
+        if (cut_row(bq, parts, qi, cur, stk, s_stk[w][stk == s_stk[w][0] ? 1 : 0], top)) break;
+      }
       const int n = min(min(top, 32), max(1, kBallStack - kBallReserve - top));
       int2 e = make_int2(0, kNone);
       if (lane < n) e = stk[top - 1 - lane];
@@ -842,6 +947,7 @@ __global__ void __launch_bounds__(128) k_range_warp(
         const int32_t tot = __shfl_sync(FULL, inc, 31);
         const int32_t delta = e.x - (inc - ct);
         const unsigned wholes = __ballot_sync(FULL, lane < lead && e.y < 0);
+        work += tot >> 5;
 #pragma unroll 2
         for (int32_t t = lane; t - lane < tot; t += 32) {
           int j = 0;
@@ -873,10 +979,57 @@ __global__ void __launch_bounds__(128) k_range_warp(
     if (!FILL) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(FULL, cnt, o);
-      if (lane == 0) counts[qi] = cnt;
+      if (lane == 0) {
+        if (parts.run) parts.list[r].count = (int32_t)cnt;
+        else counts[qi] = cnt;
+      }
     }
     __syncwarp();
   }
+}
+
+template <class QT>
+ckd_status range_warp_count(const ckd_tree* t, const double* q, const int32_t* rows, int64_t nq,
+                            const unsigned* n_rows, double r2, int64_t* counts,
+                            const int32_t* qroot, int sms, cudaStream_t s) {
+  const unsigned g = (unsigned)std::min<int64_t>(cdiv(nq, 4), (int64_t)sms * 16);
+  k_range_warp<QT, false><<<g, 128, 0, s>>>(t->view(), q, rows, nq, r2, counts, nullptr, nullptr,
+                                            nullptr, 0, nullptr, nullptr, 0, qroot, n_rows,
+                                            Parts{});
+  CKD_LAUNCH_CHECK();
+  return CKD_OK;
+}
+
+// The fill's warps, and those of the parts when its long rows are cut (`n_parts`: a zero).
+template <class QT>
+ckd_status range_warp_fill(const ckd_tree* t, const double* q, const int32_t* rows, int64_t nq,
+                           const unsigned* n_rows, double r2, const int64_t* offsets, int64_t* idx,
+                           double* dist, int want_d2, EmitTask* tasks, unsigned* n_tasks,
+                           unsigned task_cap, const int32_t* qroot, bool cut, unsigned* n_parts,
+                           int sms, cudaStream_t s) {
+  const TreeView tv = t->view();
+  const unsigned g = (unsigned)std::min<int64_t>(cdiv(nq, 4), (int64_t)sms * 16);
+  Scratch sc(s);
+  Parts parts{};
+  parts.n = n_parts;
+  parts.cap = (unsigned)std::min<int64_t>(1 << 20, std::max<int64_t>(1 << 14, nq * 256));
+  if (cut && sc.alloc(&parts.list, sizeof(Part) * parts.cap) != cudaSuccess)
+    cudaGetLastError();  // without room the rows are walked whole
+  k_range_warp<QT, true><<<g, 128, 0, s>>>(tv, q, rows, nq, r2, nullptr, offsets, idx, dist,
+                                           want_d2, tasks, n_tasks, task_cap, qroot, n_rows, parts);
+  CKD_LAUNCH_CHECK();
+  if (!parts.list) return CKD_OK;
+  parts.run = true;
+  const unsigned gp = (unsigned)sms * 16;
+  k_range_warp<QT, false><<<gp, 128, 0, s>>>(tv, q, nullptr, 0, r2, nullptr, nullptr, nullptr,
+                                             nullptr, 0, nullptr, nullptr, 0, qroot, nullptr,
+                                             parts);
+  CKD_LAUNCH_CHECK();
+  k_range_warp<QT, true><<<gp, 128, 0, s>>>(tv, q, nullptr, 0, r2, nullptr, offsets, idx, dist,
+                                            want_d2, tasks, n_tasks, task_cap, qroot, nullptr,
+                                            parts);
+  CKD_LAUNCH_CHECK();
+  return CKD_OK;
 }
 
 // ---------------------------------------------------- ball, eight lanes per query
@@ -1345,10 +1498,24 @@ bool range_narrow(const ckd_tree* t, int64_t nq, double r) {
   return hits <= (nq >= 100000 ? 64.0 : 16.0);
 }
 
+// Whether a fill cuts its long rows: batches with fewer rows than the GPU's resident
+// warps, or few long rows among more (forests), where density is uneven and the caller
+// knows that rows are long on average.  Measured, fill walked whole / cut (us), 2^22
+// clustered points: 300 balls of 9500 results 1220 / 523, 4001 of 730 605 / 289 and of
+// 34800 2415 / 2019; 2^20 points in one cluster: 1000 boxes of 200 171 / 95, of 84000
+// 2057 / 1083; 2^19 clustered, 8000 balls of 960: 390 / 442.  200 trees of 2.5e7 points:
+// 12800 boxes of 2460 results 2257 / 993, 51200 balls of 2130 3782 / 4351; of 1.6e6: 12800
+// balls of 130 190 / 200.  Rows of a few results gain nothing and would pay for two more
+// launches (12 us); on 2^17 points the walks are as short as those.
+bool cut_long_rows(const ckd_tree* t, int64_t nq, int64_t total) {
+  return nq <= (t->n_trees > 1 ? 16384 : 4736) && t->n >= (1 << 19) && total >= nq * 192 &&
+         (t->n_trees > 1 || tree_uneven(t));
+}
+
 template <int D, bool PER>
 ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order, int64_t nq,
                        double r, bool fill, int sorted, int64_t* counts, const int64_t* offsets,
-                       int64_t* idx, double* dist, cudaStream_t s, const int32_t* qroot) {
+                       int64_t* idx, double* dist, cudaStream_t s, const int32_t* qroot, int64_t total) {
   TreeView tv = t->view();
   const int threads = 128, nw = threads / 32;
   int64_t warps = cdiv(nq, 32);
@@ -1376,10 +1543,10 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
     return sorted ? sort_rows(offsets, nq, idx, dist, sms, s) : CKD_OK;
   }
   int32_t *heavy = nullptr, *light = nullptr;
-  unsigned* cnt = nullptr;  // heavy rows, light rows, emission tasks
+  unsigned* cnt = nullptr;  // heavy rows, light rows, emission tasks, parts
   if (packet || fill) {
-    CKD_CUDA(sc.alloc(&cnt, 3 * sizeof(unsigned)));
-    CKD_CUDA(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), s));
+    CKD_CUDA(sc.alloc(&cnt, 4 * sizeof(unsigned)));
+    CKD_CUDA(cudaMemsetAsync(cnt, 0, 4 * sizeof(unsigned), s));
   }
   if (packet) {
     if (warp || fill) CKD_CUDA(sc.alloc(&heavy, sizeof(int32_t) * nq));
@@ -1414,18 +1581,15 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
   EmitTask* tasks = nullptr;
   if (fill) CKD_CUDA(sc.alloc(&tasks, sizeof(EmitTask) * task_cap));
   if (warp) {
-    const unsigned g = (unsigned)std::min<int64_t>(cdiv(nq, nw), (int64_t)sms * 16);
     const int32_t* rows = packet ? heavy : order;
     const unsigned* n_rows = packet ? cnt : nullptr;
     if (fill)
-      k_range_warp<BallQuery<D, PER>, true><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, nullptr, offsets, idx,
-                                                      dist, sorted ? 1 : 0, tasks, cnt + 2,
-                                                      task_cap, qroot, n_rows);
+      CKD_TRY((range_warp_fill<BallQuery<D, PER>>(t, q, rows, nq, n_rows, r2, offsets, idx, dist,
+                                                  sorted ? 1 : 0, tasks, cnt + 2, task_cap, qroot,
+                                                  cut_long_rows(t, nq, total), cnt + 3, sms, s)));
     else
-      k_range_warp<BallQuery<D, PER>, false><<<g, threads, 0, s>>>(tv, q, rows, nq, r2, counts, nullptr,
-                                                       nullptr, nullptr, 0, nullptr, nullptr, 0,
-                                                       qroot, n_rows);
-    CKD_LAUNCH_CHECK();
+      CKD_TRY((range_warp_count<BallQuery<D, PER>>(t, q, rows, nq, n_rows, r2, counts, qroot, sms,
+                                                   s)));
   } else if (fill) {
     const int64_t hblocks = std::min<int64_t>(cdiv(nq, 4), (int64_t)sms * 8);
     const int hstack_len = std::max(kHeavyStack, t->depth + 4);
@@ -1453,38 +1617,33 @@ constexpr int64_t kBoxWarpMax = 32768;
 template <int D>
 ckd_status box_launch(const ckd_tree* t, const double* boxes, int64_t nb, bool fill,
                       int64_t* counts, const int64_t* offsets, int64_t* idx, cudaStream_t s,
-                      const int32_t* broot) {
+                      const int32_t* broot, int64_t total) {
   TreeView tv = t->view();
   const int threads = 128, nw = threads / 32;
   if (t->depth < kBallReserve - 3 && (nb <= kBoxWarpMax || broot) && box_warp_enabled()) {
     int dev = 0, sms = 148;
     CKD_CUDA(cudaGetDevice(&dev));
     CKD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const unsigned wb = (unsigned)std::min<int64_t>(cdiv(nb, nw), (int64_t)sms * 16);
-    if (!fill) {
-      k_range_warp<BoxQuery<D>, false><<<wb, threads, 0, s>>>(tv, boxes, nullptr, nb, 0.0, counts,
-                                                              nullptr, nullptr, nullptr, 0, nullptr,
-                                                              nullptr, 0, broot);
-      CKD_LAUNCH_CHECK();
-      return CKD_OK;
-    }
+    if (!fill)
+      return range_warp_count<BoxQuery<D>>(t, boxes, nullptr, nb, nullptr, 0.0, counts, broot, sms,
+                                           s);
     Scratch sc(s);
     const unsigned task_cap =
         (unsigned)std::min<int64_t>(kTaskCap, std::max<int64_t>(1 << 16, nb * 64));
-    // tasks and their counter behind them; without room for them the warps copy
-    // whole ranges themselves
+    // tasks, their counter and that of the parts behind them; without room for them the
+    // warps copy whole ranges themselves
     EmitTask* tasks = nullptr;
     unsigned* ntask = nullptr;
     if (sc.alloc(&tasks, sizeof(EmitTask) * (task_cap + 1)) == cudaSuccess) {
       ntask = reinterpret_cast<unsigned*>(tasks + task_cap);
-      CKD_CUDA(cudaMemsetAsync(ntask, 0, sizeof(unsigned), s));
+      CKD_CUDA(cudaMemsetAsync(ntask, 0, 2 * sizeof(unsigned), s));
     } else {
       cudaGetLastError();
     }
-    k_range_warp<BoxQuery<D>, true><<<wb, threads, 0, s>>>(tv, boxes, nullptr, nb, 0.0, nullptr,
-                                                           offsets, idx, nullptr, 0, tasks, ntask,
-                                                           task_cap, broot);
-    CKD_LAUNCH_CHECK();
+    CKD_TRY((range_warp_fill<BoxQuery<D>>(t, boxes, nullptr, nb, nullptr, 0.0, offsets, idx, nullptr,
+                                          0, tasks, ntask, task_cap, broot,
+                                          tasks && cut_long_rows(t, nb, total),
+                                          tasks ? ntask + 1 : nullptr, sms, s)));
     if (tasks) {
       k_box_emit<<<(unsigned)sms * 8, 128, 0, s>>>(tv.ids, tasks, ntask, task_cap, idx);
       CKD_LAUNCH_CHECK();
@@ -1535,7 +1694,7 @@ bool want_ball_order(const ckd_tree* t, int64_t nq) {
 
 ckd_status ball_run(const ckd_tree* t, const double* q, int64_t nq, double r, bool fill, int sorted,
                     int64_t* counts, const int64_t* offsets, int64_t* idx, double* dist,
-                    cudaStream_t s, const int32_t* qroot) {
+                    cudaStream_t s, const int32_t* qroot, int64_t total) {
   int32_t* order = nullptr;
   Scratch sc(s);
   if (want_ball_order(t, nq)) {
@@ -1546,9 +1705,9 @@ ckd_status ball_run(const ckd_tree* t, const double* q, int64_t nq, double r, bo
 #define CKD_BALL_CASE(DD)                                                                      \
   case DD:                                                                                     \
     st = t->periodic ? ball_launch<DD, true>(t, q, order, nq, r, fill, sorted, counts, offsets, \
-                                             idx, dist, s, qroot)                              \
+                                             idx, dist, s, qroot, total)                       \
                      : ball_launch<DD, false>(t, q, order, nq, r, fill, sorted, counts,         \
-                                              offsets, idx, dist, s, qroot);                   \
+                                              offsets, idx, dist, s, qroot, total);                   \
     break;
   switch (t->d) {
     CKD_BALL_CASE(1)
@@ -1566,16 +1725,17 @@ ckd_status ball_run(const ckd_tree* t, const double* q, int64_t nq, double r, bo
 }
 
 ckd_status box_run(const ckd_tree* t, const double* boxes, int64_t nb, bool fill, int64_t* counts,
-                   const int64_t* offsets, int64_t* idx, cudaStream_t s, const int32_t* broot) {
+                   const int64_t* offsets, int64_t* idx, cudaStream_t s, const int32_t* broot,
+                   int64_t total) {
   switch (t->d) {
-    case 1: return box_launch<1>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
-    case 2: return box_launch<2>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
-    case 3: return box_launch<3>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
-    case 4: return box_launch<4>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
-    case 5: return box_launch<5>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
-    case 6: return box_launch<6>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
-    case 7: return box_launch<7>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
-    case 8: return box_launch<8>(t, boxes, nb, fill, counts, offsets, idx, s, broot);
+    case 1: return box_launch<1>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
+    case 2: return box_launch<2>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
+    case 3: return box_launch<3>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
+    case 4: return box_launch<4>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
+    case 5: return box_launch<5>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
+    case 6: return box_launch<6>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
+    case 7: return box_launch<7>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
+    case 8: return box_launch<8>(t, boxes, nb, fill, counts, offsets, idx, s, broot, total);
   }
   return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
 }

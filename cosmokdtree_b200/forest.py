@@ -141,8 +141,8 @@ class Forest:
             offsets, total = _csr_offsets(counts, nb)
             idx = torch.empty(total, dtype=torch.int64, device=b.device)
             if nb > 0 and total > 0:
-                check(L.ckd_forest_box_fill(self.handle, _ptr(b), _ptr(bo), nb, _ptr(offsets),
-                                            _ptr(idx), _stream()))
+                check(L.ckd_forest_box_fill_sized(self.handle, _ptr(b), _ptr(bo), nb, total,
+                                                  _ptr(offsets), _ptr(idx), _stream()))
         return offsets, idx
 
     def ball_csr(self, queries, query_offsets, radius, sorted=False):
@@ -164,9 +164,9 @@ class Forest:
             idx = torch.empty(total, dtype=torch.int64, device=q.device)
             dist = torch.empty(total, dtype=torch.float64, device=q.device)
             if nq > 0 and total > 0:
-                check(L.ckd_forest_ball_fill(self.handle, _ptr(q), _ptr(qo), nq, radius,
-                                             int(bool(sorted)), _ptr(offsets), _ptr(idx),
-                                             _ptr(dist), _stream()))
+                check(L.ckd_forest_ball_fill_sized(self.handle, _ptr(q), _ptr(qo), nq, radius,
+                                                   int(bool(sorted)), total, _ptr(offsets),
+                                                   _ptr(idx), _ptr(dist), _stream()))
         return offsets, idx, dist
 
 

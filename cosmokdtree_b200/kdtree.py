@@ -411,8 +411,8 @@ def ball_search_csr(tree: KDTree, target, radius, sorted=False):
         idx = torch.empty(total, dtype=torch.int64, device=q.device)
         dist = torch.empty(total, dtype=torch.float64, device=q.device)
         if nq > 0 and total > 0:
-            check(L.ckd_ball_fill(tree.handle, _ptr(q), nq, radius, int(bool(sorted)),
-                                  _ptr(offsets), _ptr(idx), _ptr(dist), _stream()))
+            check(L.ckd_ball_fill_sized(tree.handle, _ptr(q), nq, radius, int(bool(sorted)), total,
+                                        _ptr(offsets), _ptr(idx), _ptr(dist), _stream()))
     return offsets, idx, dist
 
 
@@ -453,7 +453,8 @@ def box_search_csr(tree: KDTree, boxes):
         offsets, total = _csr_offsets(counts, nb)
         idx = torch.empty(total, dtype=torch.int64, device=b.device)
         if nb > 0 and total > 0:
-            check(L.ckd_box_fill(tree.handle, _ptr(b), nb, _ptr(offsets), _ptr(idx), _stream()))
+            check(L.ckd_box_fill_sized(tree.handle, _ptr(b), nb, total, _ptr(offsets), _ptr(idx),
+                                       _stream()))
     return offsets, idx
 
 

@@ -203,6 +203,13 @@ ckd_status ckd_ball_count(const ckd_tree* tree, const double* q_dev, int64_t nq,
 ckd_status ckd_ball_fill(const ckd_tree* tree, const double* q_dev, int64_t nq, double radius,
                          int sorted, const int64_t* offsets_dev, int64_t* idx_dev,
                          double* dist_dev, void* stream);
+/* The ckd_*_fill_sized forms take the total of the counts (offsets[n]) when the
+ * caller has it, negative otherwise: rows known to be long are shared among warps.
+ * Results are the same. */
+ckd_status ckd_ball_fill_sized(const ckd_tree* tree, const double* q_dev, int64_t nq,
+                               double radius, int sorted, int64_t total,
+                               const int64_t* offsets_dev, int64_t* idx_dev, double* dist_dev,
+                               void* stream);
 
 /* Box search, two-phase CSR protocol.  Boxes are nb x 2d row-major
  * [lo0, hi0, lo1, hi1, ...].  Replaces pybox_search_call_1/2
@@ -212,6 +219,9 @@ ckd_status ckd_box_count(const ckd_tree* tree, const double* boxes_dev, int64_t 
                          int64_t* counts_dev, void* stream);
 ckd_status ckd_box_fill(const ckd_tree* tree, const double* boxes_dev, int64_t nb,
                         const int64_t* offsets_dev, int64_t* idx_dev, void* stream);
+ckd_status ckd_box_fill_sized(const ckd_tree* tree, const double* boxes_dev, int64_t nb,
+                              int64_t total, const int64_t* offsets_dev, int64_t* idx_dev,
+                              void* stream);
 
 /* The same two-phase protocols on host buffers, for callers without device
  * memory of their own (the Fortran module cosmokdtree_gpu, C, other FFIs); the
@@ -295,6 +305,9 @@ ckd_status ckd_forest_box_count(const ckd_tree* forest, const double* boxes_dev,
 ckd_status ckd_forest_box_fill(const ckd_tree* forest, const double* boxes_dev,
                                const int64_t* b_offsets_dev, int64_t nb,
                                const int64_t* offsets_dev, int64_t* idx_dev, void* stream);
+ckd_status ckd_forest_box_fill_sized(const ckd_tree* forest, const double* boxes_dev,
+                                     const int64_t* b_offsets_dev, int64_t nb, int64_t total,
+                                     const int64_t* offsets_dev, int64_t* idx_dev, void* stream);
 /* Ball search over a forest, queries grouped by tree as for ckd_forest_knn;
  * two-phase CSR as ckd_ball_* (ids local to each query's tree). */
 ckd_status ckd_forest_ball_count(const ckd_tree* forest, const double* q_dev,
@@ -304,6 +317,10 @@ ckd_status ckd_forest_ball_fill(const ckd_tree* forest, const double* q_dev,
                                 const int64_t* q_offsets_dev, int64_t nq, double radius,
                                 int sorted, const int64_t* offsets_dev, int64_t* idx_dev,
                                 double* dist_dev, void* stream);
+ckd_status ckd_forest_ball_fill_sized(const ckd_tree* forest, const double* q_dev,
+                                      const int64_t* q_offsets_dev, int64_t nq, double radius,
+                                      int sorted, int64_t total, const int64_t* offsets_dev,
+                                      int64_t* idx_dev, double* dist_dev, void* stream);
 
 /* Save a built tree or forest to a file / load it onto the current device (no
  * counterpart in the reference, which rebuilds on every run).  The file is a raw
