@@ -1520,20 +1520,20 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
   const int threads = 128, nw = threads / 32;
   int64_t warps = cdiv(nq, 32);
   unsigned blocks = (unsigned)cdiv(warps, nw);
+  // rows of the warp kernel (null: all, in processing order), and the packet
+  // kernel's rows before it for large batches and for trees that the warp kernel
+  // does not take
+  const bool warp = ball_warp_ok(t), packet = !warp || nq > kBallWarpMax;
   // a packet stack holds at most one pending sibling per level, plus the roots
   int stack_len = std::max(kStack, t->depth + 4 + (qroot ? 32 : 0));
   Scratch sc(s);
   int32_t* gstack = nullptr;
-  if (stack_len > kStack && !ball_warp_ok(t))
+  if (packet && stack_len > kStack)
     CKD_CUDA(sc.alloc(&gstack, sizeof(int32_t) * 2 * stack_len * (int64_t)blocks * nw));
   double r2 = r * r;  // radius**2 (cosmokdtree.f90:1112)
   int dev = 0, sms = 148;
   CKD_CUDA(cudaGetDevice(&dev));
   CKD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // rows of the warp kernel (null: all, in processing order), and the packet
-  // kernel's rows before it for large batches and for trees that the warp kernel
-  // does not take
-  const bool warp = ball_warp_ok(t), packet = !warp || nq > kBallWarpMax;
   if (warp && !packet && !qroot && range_narrow(t, nq, r)) {
     if (!fill)
       return range_group_launch<BallQuery<D, PER>, false>(t, q, order, nq, r2, counts, nullptr,

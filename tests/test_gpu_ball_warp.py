@@ -113,3 +113,52 @@ def test_gpu_ball_batches_past_the_warp_rule(gpu, name, r):
     take = np.concatenate([np.arange(off[i], off[i + 1]) for i in ids])
     np.testing.assert_array_equal(idx.cpu().numpy()[take], sidx.cpu().numpy())
     np.testing.assert_array_equal(dist.cpu().numpy()[take], sdist.cpu().numpy())
+
+
+def sampled_rows_match(search, batch, sample, ids, nq):
+    """Rows ``ids`` of a large batch equal the same queries searched in small ones."""
+    off, idx, dist = (x.cpu().numpy() for x in search(batch))
+    soff, sidx, sdist = (x.cpu().numpy() for x in search(sample))
+    assert len(off) == nq + 1 and soff[-1] > 0
+    np.testing.assert_array_equal(np.diff(off)[ids], np.diff(soff))
+    take = np.concatenate([np.arange(off[i], off[i + 1]) for i in ids])
+    np.testing.assert_array_equal(idx[take], sidx)
+    np.testing.assert_array_equal(dist[take], sdist)
+
+
+@pytest.mark.parametrize("sorted_", [False, True])
+def test_gpu_ball_packets_on_deep_trees(gpu, sorted_):
+    """Packets of a batch past the warp rule on a tree deeper than their shared stack
+    (96 entries): a cusp at a low corner, whose leftmost paths keep a sibling a level."""
+    rng = np.random.default_rng(61)
+    n, nq = 400001, 200001
+    P = rng.random((n, 3)) * 10.0 ** (-10 * rng.random((n, 1)))
+    t = gpu.kdtree.build_kdtree(P)
+    assert 96 <= t.depth < 127
+    near = np.argsort((P * P).sum(1))[:nq]  # the deepest leaves are all among them
+    Q = P[near]
+    ids = np.concatenate([np.arange(2000), rng.integers(2000, nq, 2000)])
+    sampled_rows_match(lambda q: gpu.kdtree.ball_search_csr(t, q, 1e-11, sorted=sorted_),
+                       Q, Q[ids], ids, nq)
+
+
+def test_gpu_ball_packets_on_deep_forests(gpu):
+    """The same in a forest, where the packets hold several roots besides."""
+    rng = np.random.default_rng(67)
+    trees, m, per = 20001, 110, 10
+    P = 0.5 ** np.arange(m)[None, :, None] * (1 + 0.1 * rng.random((trees, m, 3)))
+    poff = np.arange(trees + 1) * m
+    f = gpu.build_forest(P.reshape(-1, 3), poff, leaf=1)
+    assert 96 <= f.depth < 127
+    Q = P[:, m - per:]  # next to the corner of each tree
+    pick = np.arange(0, trees, 97)
+    ids = (pick[:, None] * per + np.arange(per)).ravel()
+
+    def search(q):
+        return f.ball_csr(q.reshape(-1, 3), qoff[len(q)], 1e-31)
+
+    qoff = {trees: np.arange(trees + 1) * per}
+    few = np.zeros(trees + 1, np.int64)
+    few[pick + 1] = per
+    qoff[len(pick)] = np.cumsum(few)
+    sampled_rows_match(search, Q, Q[pick], ids, trees * per)
