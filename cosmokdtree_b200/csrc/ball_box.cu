@@ -723,7 +723,10 @@ struct Part {
   int32_t count;   // its results
   int32_t pad;
 };
-constexpr int kPartMin = 128;     // entries that a row is refined to, at least, where it can be
+constexpr int kPartMin = 96;      // entries that a row is refined to, at least, where it can be
+// a level at most doubles the entries, and a row that finds no room for its parts is
+// walked on from what it was refined to: one-at-a-time descents still have their room
+static_assert(2 * (kPartMin - 1) <= kBallStack - kBallReserve, "refined rows and the stack");
 constexpr int kPartBudget = 64;   // steps (32 lanes' work each) before a row is cut
 struct Parts {
   Part* list;       // null: rows are not cut

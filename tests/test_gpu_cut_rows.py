@@ -85,3 +85,34 @@ def test_gpu_cut_rows_of_a_forest(gpu):
     o, idx = f.box_csr(B, qoff.cpu().numpy())
     assert int(o[-1]) >= 192 * len(q)
     assert torch.equal(idx, whole(L, _lib, f.handle, B, o, None, 0, qoff)[0])
+
+
+@pytest.fixture(scope="module")
+def core_forest(gpu):
+    """Two deep trees, each with 8192 targets about its dense core: the 16384 rows of thousands
+    of results want more parts (96 and more a row) than their list holds (2^20)."""
+    from cosmokdtree_b200 import forest
+    m, per = 300000, 8192
+    P, Q = [], []
+    for seed in (5, 6):
+        rng = np.random.default_rng(seed)
+        x = rng.normal(size=(m, 3))
+        x *= 0.4 * rng.random((m, 1)) ** 2 / np.linalg.norm(x, axis=1, keepdims=True)
+        P.append(x)
+        Q.append(x[np.argsort((x * x).sum(1))[20000:20000 + per]])
+    f = forest.build_forest(np.concatenate(P), [0, m, 2 * m], leaf=1)
+    assert 66 < f.depth < 127
+    return f, np.concatenate(Q), [0, per, 2 * per]
+
+
+def test_gpu_cut_rows_boxes_past_the_part_list(gpu, core_forest):
+    import torch
+    from cosmokdtree_b200 import _lib
+    f, q, qoff = core_forest
+    Q = torch.from_numpy(q).cuda()
+    B = torch.stack([Q - 0.003, Q + 0.003], 2).reshape(-1, 6).contiguous()
+    o, idx = f.box_csr(B, qoff)
+    assert int((o[1:] - o[:-1]).min()) >= 4096  # every row is long enough to be cut
+    want, _ = whole(_lib.load(), _lib, f.handle, B, o, None, 0,
+                    torch.tensor(qoff, device="cuda"))
+    assert torch.equal(idx, want)
