@@ -742,7 +742,11 @@ __device__ __forceinline__ bool cut_row(const QT& bq, const Parts& parts, int64_
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  if (!parts.list || parts.run || *(volatile unsigned*)parts.n >= parts.cap) return false;
+  if (!parts.list || parts.run) return false;
+  // read by one lane: other warps add to it, and the warp has to agree
+  unsigned used = 0;
+  if (lane == 0) used = *(volatile unsigned*)parts.n;
+  if (__shfl_sync(FULL, used, 0) >= parts.cap) return false;
   bool more = true;
   while (more && top < kPartMin) {
     int m = 0;

@@ -116,3 +116,17 @@ def test_gpu_cut_rows_boxes_past_the_part_list(gpu, core_forest):
     want, _ = whole(_lib.load(), _lib, f.handle, B, o, None, 0,
                     torch.tensor(qoff, device="cuda"))
     assert torch.equal(idx, want)
+
+
+@pytest.mark.parametrize("sorted_", [0, 1])
+def test_gpu_cut_rows_balls_past_the_part_list(gpu, core_forest, sorted_):
+    """Warps that find the list full while others fill it walk their rows on."""
+    import torch
+    from cosmokdtree_b200 import _lib
+    f, q, qoff = core_forest
+    Q = torch.from_numpy(q).cuda()
+    o, idx, dist = f.ball_csr(Q, qoff, 0.003, sorted=bool(sorted_))
+    assert int((o[1:] - o[:-1]).min()) >= 4096
+    wi, wd = whole(_lib.load(), _lib, f.handle, Q, o, 0.003, sorted_,
+                   torch.tensor(qoff, device="cuda"))
+    assert torch.equal(idx, wi) and torch.equal(dist, wd)
