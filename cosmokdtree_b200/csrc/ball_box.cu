@@ -820,7 +820,8 @@ __global__ void __launch_bounds__(128) k_range_warp(
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cur += __shfl_xor_sync(FULL, cur, o);
         cur += p.base;
-        cur_end = cur + p.count;
+        // no further than the row, whose length is the caller's
+        cur_end = min(cur + p.count, offsets[qi + 1]);
       }
     } else {
       qi = order ? (int64_t)order[r] : r;
@@ -829,7 +830,7 @@ __global__ void __launch_bounds__(128) k_range_warp(
         cur_end = offsets[qi + 1];
       }
     }
-    if (FILL && cur == cur_end) continue;
+    if (FILL && cur >= cur_end) continue;
     QT bq(tv, Q, qi, r2);
     int64_t cnt = 0;  // per lane
     int top = 1, nl = 0, work = 0;

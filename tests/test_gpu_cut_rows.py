@@ -130,3 +130,24 @@ def test_gpu_cut_rows_balls_past_the_part_list(gpu, core_forest, sorted_):
     wi, wd = whole(_lib.load(), _lib, f.handle, Q, o, 0.003, sorted_,
                    torch.tensor(qoff, device="cuda"))
     assert torch.equal(idx, wi) and torch.equal(dist, wd)
+
+
+def test_gpu_cut_rows_end_where_the_offsets_say(gpu):
+    """A fill with a larger radius than the count's truncates its rows, cut or whole."""
+    import torch
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    P = torch.from_numpy(cluster(1 << 19, 3, 3)).cuda()
+    Q = P[(P * P).sum(1).argsort()[1000:1300]].contiguous()
+    t = gpu.kdtree.build_kdtree(P)
+    off, _, _ = gpu.kdtree.ball_search_csr(t, Q, 0.004)
+    total, guard = int(off[-1]), 1 << 24
+    assert total >= 192 * 300
+    want, wd = whole(L, _lib, t.handle, Q, off, 0.005, 0)
+    idx = torch.full((total + guard,), -7, dtype=torch.int64, device="cuda")
+    dist = torch.full((total + guard,), -7.0, dtype=torch.float64, device="cuda")
+    ptr = lambda x: ctypes.c_void_p(x.data_ptr())
+    _lib.check(L.ckd_ball_fill_sized(t.handle, ptr(Q), 300, 0.005, 0, total, ptr(off), ptr(idx),
+                                     ptr(dist), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert bool((idx[total:] == -7).all()) and bool((dist[total:] == -7.0).all())
+    assert torch.equal(idx[:total], want) and torch.equal(dist[:total], wd)
