@@ -42,6 +42,7 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned kUntested = 0xffffffffu;  // stack entry whose box has not been tested
+constexpr float kFarQuery = 1e25f;
 constexpr int32_t kUnit = 16;     // subtrees of at most this many points are scanned as a range
 
 // (d, id) lexicographic order
@@ -169,7 +170,9 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
 #pragma unroll
   for (int j = 0; j < D; ++j) {
     q[j] = valid ? Q[qi * D + j] : 0.0;
-    qs.q32[j] = __double2float_rn(q[j]);
+    // clamped so that its gaps stay numbers: a query out there is further than HUGE from
+    // every point (coordinates are below 1e18 here); NaN, which no point is near, likewise
+    qs.q32[j] = fminf(fmaxf(__double2float_rn(q[j]), -kFarQuery), kFarQuery);
     qs.dlt[j] = kTwoM21 * (fabsf(qs.q32[j]) + tv.slack[j]) * 1.0001f;
     xl[j] = __fadd_ru(qs.q32[j], qs.dlt[j]);
     xh[j] = __fsub_rd(qs.q32[j], qs.dlt[j]);
@@ -308,11 +311,16 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
   __syncwarp();
   while (__any_sync(FULL, next >= 0 || top > 0)) {
     const bool act = next >= 0 || top > 0;
-    if (next < 0 && top > 0 && bd == CKD_HUGE) next = (int32_t)stk[--top].x;
+    if (next < 0 && top > 0 && bd == CKD_HUGE) {
+      // dropped when all of it is further than HUGE: a query far from every point would
+      // read the whole tree (64 such of 2^20 points, k = 100: 16 ms)
+      next = (int32_t)stk[--top].x;
+      if (!(node_lb(next) <= wd32)) next = -1;
+    }
     __syncwarp();
     int32_t c0 = -1, c1 = -1, st0 = 0, ct0 = 0, st1 = 0, ct1 = 0;
     float l0 = 0.0f, l1 = 0.0f;
-    if (act && bd == CKD_HUGE) {
+    if (next >= 0) {
       // fewer than k found yet: descent from the nearest waiting subtree (at first
       // the root) along the query's side of the splits to a range
       NodeMeta m = load_meta(tv.meta, next);
@@ -332,7 +340,7 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
         st0 = m.start;
         ct0 = m.count;
       }
-    } else if (act) {
+    } else if (act && bd < CKD_HUGE) {
       // up to G waiting subtrees at once, a lane each
       const int n = min(min(top, G), max(1, depth + 2 * G - top));
       int32_t c = -1;

@@ -133,3 +133,38 @@ def test_gpu_knn_group_bounded(gpu, oracle, name, d, periodic, k, margin):
     od, oi = oracle.OracleTree(P, 16, box).knn(Q, k)
     np.testing.assert_array_equal(gi, oi)
     np.testing.assert_array_equal(gd, od)
+
+
+@pytest.mark.parametrize("k", [1, 16, 100])
+def test_gpu_knn_group_far_queries(gpu, oracle, k):
+    """A query further than the largest distance from every point finds nothing, and does not
+    read the tree for it: it takes no longer than ten queries among the points (the whole tree
+    of 2^20 would take thousands of times as long)."""
+    import time
+    import torch
+    rng = np.random.default_rng(43)
+    P = rng.random((1 << 20, 3))
+    t = gpu.kdtree.build_kdtree(P)
+    far = np.array([2e19, -1e20, 1e30, -1e60, 1e200, np.inf, -np.inf, np.nan])
+    Q = np.full((64, 3), 0.5)
+    Q[np.arange(64), rng.integers(0, 3, 64)] = np.resize(far, 64)
+    near = torch.from_numpy(rng.random((64, 3))).cuda()
+    Q = torch.from_numpy(Q).cuda()
+
+    def clock(q):
+        best = np.inf
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            r = gpu.kdtree.knn_search_batch(t, q, k)
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t0)
+        return best, r
+
+    tn, _ = clock(near)
+    tf, (d, i) = clock(Q)
+    od, oi = oracle.OracleTree(P[:1000], 16, None).knn(Q.cpu().numpy(), k)
+    np.testing.assert_array_equal(i.cpu().numpy(), oi)
+    np.testing.assert_array_equal(d.cpu().numpy(), od)
+    assert (oi == -2).all()
+    assert tf < 10 * tn
