@@ -966,6 +966,7 @@ __global__ void __launch_bounds__(kBT) k_scatter(
 // 128 or 512 threads, small subtrees queued for warps that need no barrier.
 constexpr int kFinT = 256;
 constexpr int kFinBlock = 512;
+constexpr int64_t kFinGrowMax = (int64_t)4 << 30;  // bytes of the largest node arrays taken at once
 __host__ __device__ constexpr int finish_max(int d) { return d <= 3 ? 2048 : 1024; }
 __host__ __device__ constexpr int finish_open(int m, int leaf) { return m / (leaf + 1) + 1; }
 __host__ __device__ constexpr size_t finish_smem(int d, int leaf) {
@@ -981,14 +982,19 @@ __global__ void k_finish_list(const NodeMeta* __restrict__ meta, int32_t n_nodes
   if (meta[a].left < 0 && meta[a].count > leaf) list[atomicAdd(n_list, 1)] = a;
 }
 
-// ctr: {node count, deepest level + 1, error (1 node capacity, 2 depth), next list entry}
+// ctr: {node count, deepest level + 1, depth error, next list entry, length of the list,
+// length of redo}.  A subtree whose nodes no longer fit (node_cap) puts its points back and
+// goes to `redo`, for a launch with more room.  The node ids that it had taken stay its
+// own: log holds, per level, the first (at the subtree's positions, the last of which says
+// how many), and the next launch (`resume`) takes them again.
 template <int D>
 __global__ void __launch_bounds__(kFinT) k_finish(const int32_t* __restrict__ list,
                                                   const int32_t* __restrict__ n_list,
                                                   NodeMeta* meta, double* cell, double* box,
                                                   double* Pf, int32_t* If, int64_t n, int leaf,
                                                   int32_t node_cap, int32_t max_levels,
-                                                  int32_t* ctr) {
+                                                  int32_t* ctr, int32_t* redo, int32_t* log,
+                                                  bool resume) {
   constexpr int M = finish_max(D), W = kFinT / 32, NP = M / kFinT;
   static_assert(NP * W <= 64, "one warp scans the chunk counts");
   extern __shared__ __align__(16) unsigned char fsm[];
@@ -999,19 +1005,31 @@ __global__ void __launch_bounds__(kFinT) k_finish(const int32_t* __restrict__ li
   int2* open = reinterpret_cast<int2*>(perm0 + 2 * M);                   // [2][lcap] {node, start | count << 16}
   __shared__ unsigned long long red[W][2 * D];
   __shared__ int32_t cpre[65];
-  __shared__ int32_t s_job, s_base, s_next, s_ext;
+  __shared__ int32_t s_job, s_full, s_base, s_next, s_ext;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
   const int32_t jobs = *n_list;
   int deepest = 0;
   for (;;) {
-    if (tid == 0) s_job = atomicAdd(&ctr[3], 1);
+    if (tid == 0) {
+      s_job = atomicAdd(&ctr[3], 1);
+      s_full = *(volatile int32_t*)&ctr[0] >= node_cap;
+    }
     __syncthreads();
     const int32_t job = s_job;
     if (job >= jobs) break;
     const int32_t root = list[job];
     const int32_t g0 = meta[root].start, c0 = meta[root].count;
     int depth = meta[root].depth;
+    const int known = resume ? log[g0 + c0 - 1] : 0;  // levels whose ids were taken before
+    if (known == 0 && s_full) {
+      if (tid == 0) {
+        log[g0 + c0 - 1] = 0;
+        redo[atomicAdd(&ctr[5], 1)] = root;
+      }
+      __syncthreads();  // s_job and s_full serve the next subtree
+      continue;
+    }
     for (int i = tid; i < c0; i += kFinT) {
 #pragma unroll
       for (int j = 0; j < D; ++j) X[j * M + i] = dkey(Pf[(int64_t)j * n + g0 + i]);
@@ -1021,21 +1039,35 @@ __global__ void __launch_bounds__(kFinT) k_finish(const int32_t* __restrict__ li
     if (tid == 0) open[0] = make_int2(root, c0 << 16);
     int m = 1, cur = 0;
     bool ok = true;
-    while (m > 0) {
+    for (int level = 0; m > 0; ++level) {
       const uint16_t* pa = perm0 + (cur ? M : 0);
       uint16_t* pb = perm0 + (cur ? 0 : M);
       const int2* oa = open + (cur ? lcap : 0);
       int2* ob = open + (cur ? 0 : lcap);
       if (tid == 0) {
-        s_base = atomicAdd(&ctr[0], 2 * m);
+        s_base = level < known ? log[g0 + level] : atomicAdd(&ctr[0], 2 * m);
+        log[g0 + level] = s_base;
         s_next = 0;
       }
       __syncthreads();  // also: the points, the open list and the permutation are in place
       const int32_t base = s_base;
-      if (depth >= max_levels || base > node_cap - 2 * m) {
-        if (tid == 0) atomicMax(&ctr[2], depth >= max_levels ? 2 : 1);
+      if (depth >= max_levels) {
+        if (tid == 0) ctr[2] = 1;
         ok = false;
         break;  // the same for the whole block
+      }
+      if (base > node_cap - 2 * m) {
+        for (int i = tid; i < c0; i += kFinT) {
+#pragma unroll
+          for (int j = 0; j < D; ++j) Pf[(int64_t)j * n + g0 + i] = dkey_inv(X[j * M + i]);
+          If[g0 + i] = I[i];
+        }
+        if (tid == 0) {
+          log[g0 + c0 - 1] = level + 1;
+          redo[atomicAdd(&ctr[5], 1)] = root;
+        }
+        ok = false;
+        break;
       }
       // the children of open node e (node a, local start s, count c), split as told,
       // with nl points on the left: records and the next open list
@@ -1454,12 +1486,8 @@ void free_bufs(BuildBufs& B, cudaStream_t s) {
   B = BuildBufs();
 }
 
-// node_cap: capacity of the node arrays for the subtrees finished in shared memory;
-// 0 takes four nodes per full leaf.  When the tree needs more, *again is set and the
-// caller builds once more with the largest count a tree can have.
 template <int D>
-ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t s,
-                      int64_t node_cap, bool* again) {
+ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t s) {
   const int64_t n = t->n;
   // the level passes end at nodes that a block finishes in shared memory
   const int tree_leaf = t->leaf;
@@ -1477,13 +1505,12 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
   const int64_t ntiles = cdiv(n, kTile);
   const int32_t T = (int32_t)t->n_trees;
   const int64_t max_open = n / (leaf + 1) + 2 + T;
-  B.tcap = node_cap > 0 ? node_cap
-                        : (int64_t)T + std::min<int64_t>(2 * n, 4 * (n / tree_leaf) + 64);
+  B.tcap = (int64_t)T + std::min<int64_t>(2 * n, 4 * (n / tree_leaf) + 64);  // grown on need
   B.cap = (int64_t)T + 4 * (n / leaf) + 64;
   B.tcap = std::max(B.tcap, B.cap);
   int64_t* off_dev = nullptr;
   double* Ldev = nullptr;
-  int32_t *flist = nullptr, *fctr = nullptr;  // nodes to finish; k_finish's counters, list length
+  int32_t *flist = nullptr, *fctr = nullptr;  // nodes to finish (two lists); k_finish's counters
   for (int pass = 0; pass < 2; ++pass) {
     Carve c(B.arena);
     for (int b = 0; b < 2; ++b) {
@@ -1713,10 +1740,12 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
 
   if (finish) {
     int32_t* const ctr = fctr;
-    CKD_CUDA(sc.alloc(&flist, sizeof(int32_t) * n_nodes));
-    int32_t h[5] = {n_nodes, depth_levels, 0, 0, 0};
+    CKD_CUDA(sc.alloc(&flist, sizeof(int32_t) * 2 * n_nodes));
+    int32_t *list = flist, *redo = flist + n_nodes;
+    int32_t* const log = B.I[0];  // free after the levels
+    int32_t h[6] = {n_nodes, depth_levels, 0, 0, 0, 0};
     CKD_CUDA(cudaMemcpyAsync(ctr, h, sizeof(h), cudaMemcpyHostToDevice, s));
-    k_finish_list<<<(unsigned)cdiv(n_nodes, 256), 256, 0, s>>>(B.meta, n_nodes, tree_leaf, flist,
+    k_finish_list<<<(unsigned)cdiv(n_nodes, 256), 256, 0, s>>>(B.meta, n_nodes, tree_leaf, list,
                                                                ctr + 4);
     CKD_LAUNCH_CHECK();
     int dev = 0, sms = 148, per_sm = 1;
@@ -1726,18 +1755,39 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
     CKD_CUDA(cudaFuncSetAttribute(k_finish<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sm));
     CKD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_finish<D>, kFinT, sm));
-    const int64_t g = std::min<int64_t>(n_nodes, (int64_t)sms * std::max(1, per_sm));
-    k_finish<D><<<(unsigned)g, kFinT, sm, s>>>(
-        flist, ctr + 4, B.meta, B.cell, B.box, t->pts, t->ids, n, tree_leaf,
-        (int32_t)std::min<int64_t>(B.tcap, INT32_MAX), kMaxLevels, ctr);
-    CKD_LAUNCH_CHECK();
-    CKD_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CKD_CUDA(cudaStreamSynchronize(s));
-    if (h[2] == 2)
-      return fail(CKD_ERR_DEPTH, "tree depth exceeds the build's level cap (8192 levels)");
-    if (h[2] == 1) {
-      *again = true;
-      return CKD_OK;
+    int64_t jobs = n_nodes;
+    for (bool resume = false;; resume = true) {
+      const int64_t g = std::min<int64_t>(jobs, (int64_t)sms * std::max(1, per_sm));
+      k_finish<D><<<(unsigned)g, kFinT, sm, s>>>(
+          list, ctr + 4, B.meta, B.cell, B.box, t->pts, t->ids, n, tree_leaf,
+          (int32_t)std::min<int64_t>(B.tcap, INT32_MAX), kMaxLevels, ctr, redo, log, resume);
+      CKD_LAUNCH_CHECK();
+      CKD_CUDA(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
+      CKD_CUDA(cudaStreamSynchronize(s));
+      if (h[2])
+        return fail(CKD_ERR_DEPTH, "tree depth exceeds the build's level cap (8192 levels)");
+      if (h[5] == 0) break;
+      // More nodes than planned (many equal points, steep clusters): the arrays grow and
+      // only the subtrees that found no room are finished again.  At once to the most
+      // nodes that a tree can have while these arrays stay small: every launch that runs out
+      // of room again costs its deepest subtree's levels (2^22 points of many copies, 27
+      // times the planned nodes: 22.8 ms when the tree was built twice, 36.1 when the
+      // arrays doubled five times).
+      const int64_t most = T + 2 * n;
+      ckd_status st = CKD_ERR_OOM;
+      if (most * (int64_t)(sizeof(NodeMeta) + 4 * D * sizeof(double)) <= kFinGrowMax)
+        st = ensure_tree_cap(B, most, s);
+      if (st == CKD_ERR_OOM) {
+        cudaGetLastError();
+        st = ensure_tree_cap(B, std::max<int64_t>(h[0], B.tcap + 1), s);
+      }
+      CKD_TRY(st);
+      jobs = h[5];
+      h[3] = 0;
+      h[4] = h[5];
+      h[5] = 0;
+      CKD_CUDA(cudaMemcpyAsync(ctr, h, sizeof(h), cudaMemcpyHostToDevice, s));
+      std::swap(list, redo);
     }
     n_nodes = h[0];
     depth_levels = std::max(depth_levels, (int)h[1]);
@@ -1787,28 +1837,13 @@ ckd_status build_impl(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t 
 }  // namespace
 
 ckd_status build_dispatch(ckd_tree* t, const void* pts_dev, int dtype, cudaStream_t s) {
-  bool again = false;
-  int64_t cap = 0;
-  for (;;) {
-    ckd_status st = CKD_OK;
-    switch (t->d) {
+  switch (t->d) {
 #define CKD_BD(DD) \
-  case DD: st = build_impl<DD>(t, pts_dev, dtype, s, cap, &again); break;
-      CKD_BD(1) CKD_BD(2) CKD_BD(3) CKD_BD(4) CKD_BD(5) CKD_BD(6) CKD_BD(7) CKD_BD(8)
+  case DD: return build_impl<DD>(t, pts_dev, dtype, s);
+    CKD_BD(1) CKD_BD(2) CKD_BD(3) CKD_BD(4) CKD_BD(5) CKD_BD(6) CKD_BD(7) CKD_BD(8)
 #undef CKD_BD
-      default: return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
-    }
-    if (st != CKD_OK || !again) return st;
-    // more nodes than planned: once more with room for every tree of these points
-    again = false;
-    cap = t->n_trees + 2 * t->n;
-    dev_free(t->block[0], s);
-    t->block[0] = nullptr;
-    t->pts = nullptr;
-    t->ids = nullptr;
-    t->pts32 = nullptr;
-    t->pts64 = nullptr;
   }
+  return fail(CKD_ERR_BAD_DIM, "dimensionality must be 1..8");
 }
 
 }  // namespace ckd

@@ -78,3 +78,55 @@ def test_gpu_finish_forest(gpu, oracle):
         od, oi = oracle.OracleTree(P, 16, 1.0).knn(P[:20], 6)
         np.testing.assert_array_equal(i[qoff[t]:qoff[t + 1]].cpu().numpy(), oi)
         np.testing.assert_array_equal(d[qoff[t]:qoff[t + 1]].cpu().numpy(), od)
+
+
+@pytest.mark.parametrize("kind,n,d,leaf", [
+    ("copies", 2000, 3, 16),      # one subtree, no levels before it
+    ("copies", 60000, 3, 16),     # many subtrees, some of which find room
+    ("copies", 60000, 2, 64),     # room several times too small
+    ("copies", 40000, 5, 3),
+    ("half", 60001, 3, 16),
+    ("clumps", 60000, 3, 256),
+    ("clumps", 60000, 6, 64),
+])
+def test_gpu_finish_grows_and_resumes(gpu, oracle, kind, n, d, leaf):
+    """Subtrees that found no room for their nodes are finished again, not the whole tree."""
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(71)
+    U = rng.random((n, d))
+    if kind == "copies":
+        P = np.repeat(U[:n // 100], 100, 0)[rng.permutation(n)]
+    elif kind == "half":
+        P = np.where(np.arange(n)[:, None] % 2, U, U[np.arange(n) // 400 * 400])
+    else:
+        P = U[rng.integers(0, 40, n)] + 10.0 ** rng.uniform(-9, -1, (n, 1)) * rng.normal(size=(n, d))
+
+    def launches(pts):
+        before = L.ckd_launch_count()
+        gpu.kdtree.build_kdtree(pts, leaf=leaf)
+        return L.ckd_launch_count() - before
+
+    t = same_tree(gpu, oracle, P, leaf, None)
+    assert t.n_nodes > 4 * (n // leaf) + 65  # more than planned
+    if n == 2000:
+        assert launches(P) < 2 * launches(U) - 3  # the even tree's, and k_finish again
+    d_, i_ = gpu.kdtree.knn_search(t, P[:50], 5)
+    od, oi = oracle.OracleTree(P, leaf, None).knn(P[:50], 5)
+    np.testing.assert_array_equal(i_, oi)
+    np.testing.assert_array_equal(d_, od)
+
+
+def test_gpu_finish_grows_and_resumes_in_a_forest(gpu, oracle):
+    rng = np.random.default_rng(73)
+    parts = [rng.random((n, 3)) for n in (700, 3000, 1, 9000, 50)]
+    parts += [np.repeat(rng.random((n // 50, 3)), 50, 0) for n in (3000, 20000, 1000)]
+    f = gpu.build_forest(parts, leaf=16)
+    assert f.n_nodes == sum(oracle.OracleTree(P, 16, None).n_nodes for P in parts)
+    q = np.concatenate([P[:20] for P in parts])
+    qoff = np.cumsum([0] + [min(20, len(P)) for P in parts])
+    d, i = f.knn(q, qoff, 6)
+    for t, P in enumerate(parts):
+        od, oi = oracle.OracleTree(P, 16, None).knn(P[:20], 6)
+        np.testing.assert_array_equal(i[qoff[t]:qoff[t + 1]].cpu().numpy(), oi)
+        np.testing.assert_array_equal(d[qoff[t]:qoff[t + 1]].cpu().numpy(), od)
