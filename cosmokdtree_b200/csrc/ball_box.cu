@@ -1500,7 +1500,7 @@ bool range_narrow(const ckd_tree* t, int64_t nq, double r) {
   constexpr double kBall[9] = {1.0, 2.0, 3.14159, 4.18879, 4.93480, 5.26379, 5.16771, 4.72477, 4.05871};
   double hits = (double)t->n * kBall[t->d];
   for (int j = 0; j < t->d; ++j) {
-    if (!(t->extent[j] > 0.0)) return false;  // unknown (a loaded tree) or flat
+    if (!(t->extent[j] > 0.0)) return false;  // unknown or flat
     hits *= r / t->extent[j];
   }
   return hits <= (nq >= 100000 ? 64.0 : 16.0);

@@ -263,7 +263,8 @@ struct ckd_tree {
   float4* pts32 = nullptr;
   double4* pts64 = nullptr;
   float slack[CKD_MAX_D] = {0};
-  // sides of the points' extent (periodic: of the box); 0 when not known (loaded trees)
+  // sides of the points' extent (periodic: of the box); 0 when not known (trees of a forest
+  // plan)
   double extent[CKD_MAX_D] = {0};
   bool screen_ok = false;  // FP32 screen usable (coordinates well inside FP32 range)
   float4* pair = nullptr;

@@ -6,6 +6,8 @@
 // of fixed-size scalars, the tree offsets (n_trees + 1 int64), then each array as
 // (int64 byte count, bytes) in a fixed order.  No counterpart in the reference,
 // which rebuilds its tree on every run.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -145,6 +147,17 @@ ckd_status ckd_tree_load(const char* path, ckd_tree** out) {
       st = fail(CKD_ERR_BAD_ARG, std::string(path) + ": truncated");
       break;
     }
+    if (a.dev == (void**)&t->box)  // the extent, as the build has it
+      for (int j = 0; j < t->d; ++j) {
+        double lo = INFINITY, hi = -INFINITY;
+        for (int64_t r = 0; r < std::min<int64_t>(t->n_trees, t->n_nodes); ++r) {
+          double b[2];
+          std::memcpy(b, buf.data() + sizeof(b) * (r * t->d + j), sizeof(b));
+          lo = std::min(lo, b[0]);
+          hi = std::max(hi, b[1]);
+        }
+        t->extent[j] = t->periodic ? t->L[j] : hi - lo;
+      }
     cudaError_t e = dev_alloc(a.dev, a.bytes, 0);  // legacy stream: ordered before the copy
     if (e == cudaSuccess) e = cudaMemcpy(*a.dev, buf.data(), a.bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) st = cuda_fail(e, "uploading a saved tree");

@@ -162,3 +162,26 @@ def test_gpu_ball_packets_on_deep_forests(gpu):
     few[pick + 1] = per
     qoff[len(pick)] = np.cumsum(few)
     sampled_rows_match(search, Q, Q[pick], ids, trees * per)
+
+
+@pytest.mark.parametrize("periodic", [False, True])
+def test_gpu_ball_kernels_of_a_loaded_tree(gpu, tmp_path, periodic):
+    """A tree read back from its file is searched by the kernels that the built one is: the
+    same rows in as many launches (eight lanes a query need one fewer than a warp)."""
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(79)
+    P = rng.random((20000, 3)) - 0.5
+    t = gpu.kdtree.build_kdtree(P, boxsize=1.0 if periodic else None)
+    gpu.kdtree.save_kdtree(t, str(tmp_path / "tree"))
+    u = gpu.kdtree.load_kdtree(str(tmp_path / "tree"))
+
+    def run(tree):
+        before = L.ckd_launch_count()
+        out = [x.cpu().numpy() for x in gpu.kdtree.ball_search_csr(tree, P[:12001], 0.03)]
+        return out, L.ckd_launch_count() - before
+
+    (a, na), (b, nb) = run(t), run(u)
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
+    assert na == nb
