@@ -61,7 +61,7 @@ struct BuildBufs {
   // one block holds every buffer below; only arrays that had to grow leave it
   char* arena = nullptr;
   size_t arena_bytes = 0;
-  bool owns(const void* p) const {
+  bool outside(const void* p) const {
     return p && !(static_cast<const char*>(p) >= arena && static_cast<const char*>(p) < arena + arena_bytes);
   }
   double* X[2] = {nullptr, nullptr};
@@ -1441,7 +1441,7 @@ cudaError_t grow(const BuildBufs& B, T** p, int64_t old_n, int64_t new_n, cudaSt
       dev_free(q, s);
       return e;
     }
-    if (B.owns(*p)) dev_free(*p, s);
+    if (B.outside(*p)) dev_free(*p, s);
   }
   *p = q;
   return cudaSuccess;
@@ -1481,7 +1481,7 @@ void free_bufs(BuildBufs& B, cudaStream_t s) {
   void* ps[] = {B.meta, B.cell,  B.box, B.keys,  B.ext,  B.mode, B.pstart,
                 B.pend, B.nleft, B.pbase, B.wst, B.frec, B.srec};
   for (void* p : ps)
-    if (B.owns(p)) dev_free(p, s);
+    if (B.outside(p)) dev_free(p, s);
   if (B.arena) dev_free(B.arena, s);
   B = BuildBufs();
 }
