@@ -877,14 +877,55 @@ __global__ void k_outside(const double* __restrict__ q, int64_t n, TreeView tv, 
   if (bad) *outside = 1;
 }
 
-// one pinned word per host thread for results that the caller waits for
-cudaError_t pinned_word(int64_t** out) {
-  static thread_local int64_t* p = nullptr;
-  cudaError_t e = cudaSuccess;
-  if (!p) e = cudaHostAlloc((void**)&p, sizeof(int64_t), cudaHostAllocPortable | cudaHostAllocMapped);
-  *out = p;
-  return e;
-}
+// A pinned word for a result that the calling thread waits for, taken for one call: out of
+// a block that the process keeps (kWords calls at once), or one of its own when all are
+// taken.
+class PinnedWord {
+ public:
+  PinnedWord() {
+    std::lock_guard<std::mutex> lock(mu());
+    if (!block())
+      err_ = cudaHostAlloc((void**)&block(), kWords * kStride * sizeof(int64_t), kFlags);
+    if (err_ == cudaSuccess && free_words()) {
+      slot_ = __builtin_ctzll(free_words());
+      free_words() &= free_words() - 1;
+      p_ = block() + slot_ * kStride;
+    } else if (err_ == cudaSuccess) {
+      err_ = cudaHostAlloc((void**)&p_, sizeof(int64_t), kFlags);
+    }
+  }
+  ~PinnedWord() {
+    if (slot_ >= 0) {
+      std::lock_guard<std::mutex> lock(mu());
+      free_words() |= 1ull << slot_;
+    } else if (p_) {
+      cudaFreeHost(p_);
+    }
+  }
+  PinnedWord(const PinnedWord&) = delete;
+  PinnedWord& operator=(const PinnedWord&) = delete;
+  cudaError_t error() const { return err_; }
+  int64_t* get() const { return p_; }
+
+ private:
+  static constexpr unsigned kFlags = cudaHostAllocPortable | cudaHostAllocMapped;
+  static constexpr int kWords = 64, kStride = 8;  // a cache line each
+  static std::mutex& mu() {
+    static std::mutex m;
+    return m;
+  }
+  static int64_t*& block() {
+    static int64_t* b = nullptr;
+    return b;
+  }
+  static uint64_t& free_words() {
+    static uint64_t f = ~0ull;
+    return f;
+  }
+  int64_t* p_ = nullptr;
+  int slot_ = -1;
+  cudaError_t err_ = cudaSuccess;
+};
 
 }  // namespace
 
@@ -895,8 +936,9 @@ ckd_status ckd_csr_offsets(const int64_t* counts, int64_t* offsets, int64_t n, i
   if (n < 0 || !offsets || !total || (n > 0 && !counts))
     return fail(CKD_ERR_BAD_ARG, "bad scan arguments");
   cudaStream_t s = (cudaStream_t)stream;
-  int64_t* w = nullptr;
-  CKD_CUDA(pinned_word(&w));
+  PinnedWord word;
+  CKD_CUDA(word.error());
+  int64_t* const w = word.get();
   CKD_TRY(scan_i64(counts, offsets, n, s));
   CKD_CUDA(cudaMemcpyAsync(w, offsets + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   CKD_CUDA(cudaStreamSynchronize(s));
@@ -913,8 +955,9 @@ ckd_status ckd_queries_inside(const ckd_tree* t, const double* q, int64_t nq, in
   *inside = 1;
   if (!t->periodic || nq == 0) return CKD_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  int64_t* w = nullptr;
-  CKD_CUDA(pinned_word(&w));
+  PinnedWord word;
+  CKD_CUDA(word.error());
+  int64_t* const w = word.get();
   *w = 0;
   const int64_t n = nq * t->d;
   k_outside<<<(unsigned)std::min<int64_t>(cdiv(n, 256), 148 * 8), 256, 0, s>>>(

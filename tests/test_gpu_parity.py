@@ -468,3 +468,73 @@ def test_gpu_knn_host_pipeline(gpu):
     np.testing.assert_array_equal(d, dd.cpu().numpy())
     with pytest.raises(AssertionError):
         kd.knn_search(t, np.full((1 << 20, 3), 0.75), 4)  # outside the periodic box
+
+
+def test_gpu_threads_wait_for_their_own_totals(gpu):
+    """More threads at once than the library keeps pinned words for (64): each gets the total and
+    the rows of its own call, on its own stream, and its own answer of the range check."""
+    import threading
+    import torch
+    rng = np.random.default_rng(83)
+    P = torch.from_numpy(rng.random((30000, 3)) - 0.5).cuda()
+    t = gpu.kdtree.build_kdtree(P, boxsize=1.0)
+    n = 80
+    radii = np.linspace(0.01, 0.04, n)
+    want = [gpu.kdtree.ball_search_csr(t, P[:200], r) for r in radii]
+    torch.cuda.synchronize()
+    got, bad = [None] * n, []
+    gate = threading.Barrier(n)
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                gate.wait()
+                for _ in range(5):
+                    got[i] = gpu.kdtree.ball_search_csr(t, P[:200], radii[i])
+                out = P[:5].clone()
+                out[i % 5, i % 3] = 0.75
+                with pytest.raises(AssertionError):
+                    gpu.kdtree.ball_search_csr(t, out, radii[i])
+                torch.cuda.current_stream().synchronize()
+        except BaseException as e:
+            bad.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(n)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not bad
+    for a, b in zip(got, want):
+        for x, y in zip(a, b):
+            assert torch.equal(x, y)
+
+
+def test_gpu_threads_leave_no_pinned_memory(gpu):
+    """Threads that come and go keep nothing: 3000 calls from threads of their own grow the
+    process by less than 2 MB (2 kB each, with a pinned word a thread)."""
+    import ctypes
+    import re
+    import threading
+    import torch
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    counts = torch.ones(100, dtype=torch.int64, device="cuda")
+    offsets = torch.empty(101, dtype=torch.int64, device="cuda")
+
+    def one():
+        total = ctypes.c_int64()
+        _lib.check(L.ckd_csr_offsets(ctypes.c_void_p(counts.data_ptr()),
+                                     ctypes.c_void_p(offsets.data_ptr()), 100,
+                                     ctypes.byref(total), None))
+        assert total.value == 100
+
+    def resident(n):
+        for _ in range(n):
+            th = threading.Thread(target=one)
+            th.start()
+            th.join()
+        return int(re.search(r"VmRSS:\s+(\d+)", open("/proc/self/status").read())[1])
+
+    before = resident(500)
+    assert resident(3000) - before < 2048
