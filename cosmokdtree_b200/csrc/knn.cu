@@ -9,6 +9,7 @@
 // (cosmokdtree.f90:517-518).  Distances are FP64, separately rounded, so results
 // are bit-identical to the CPU restatement.
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "ckd_common.cuh"
@@ -353,26 +354,59 @@ ckd_status knn_group_bound(const ckd_tree* t, const double* q, const int32_t* or
 
 // Whether the automatic choice takes a group of lanes per query
 // (ckd_knn_group.cuh) instead of the per-lane kernel.  Sorted rows only: an unsorted
-// row is in the order of its kernel's heap.  The lines are where the two cross,
-// measured on 2^20 uniform, 2^22 clustered and 2^22 6-D points (us a call, per-lane /
-// groups):
-//   k = 8: 150k queries 406 / 375, 200k 427 / 471 (uniform), 857 / 831 (clustered)
-//   k = 16: 50k 316 / 206, 100k 359 / 376 (uniform), 300k 1389 / 1375 (clustered)
-//   k = 32: 300k 1287 / 1319 (uniform), 2148 / 1935, 500k 2915 / 2992 (clustered)
-//   k = 48: 400k 3146 / 2947, 1M 6594 / 7224 (uniform)
-//   k = 64: 100k 2723 / 1232, 1M 14376 / 9726 (clustered): always groups
-//   k = 16, 6-D: 200k 4505 / 3687, 400k 7089 / 7344;  k >= 48, 6-D: always groups
-//   k = 100: 30k 16414 / 810 (against the packet kernel in the output rows)
+// row is in the order of its kernel's heap.  A lane per query takes about as long for
+// 1000 queries as for 50000, the groups' time grows with the batch from a few thousand on.
+// Where they cross depends, besides k, on what fills a lane's time: small trees stay in the
+// caches (lower lines), short leaves and uneven density leave lanes waiting (higher
+// lines).  The lines are fitted to both kernels' times on 100 trees of 3000 to 4 M points,
+// 1-D to 8-D, leaf 1 to 128, uniform, clustered, lattices and forests, batches of 15000 to
+// 10^6 from the points or uniform (20600 pairs of times, a slower choice counted three
+// times); where they are taken, the groups are the slower kernel by more than 5 % in 2 %
+// of them.  With one line for all trees and leaves it was 15 %, by a factor of two at
+// worst.  Us, per-lane / groups, 3-D points, leaf 16: 2^20 uniform, k = 8: 75k queries 250 /
+// 214, 110k 276 / 292; k = 32: 75k 531 / 421, 110k 563 / 585; leaf 64, k = 8: 110k 260 / 417;
+// 2^22 clustered, k = 16: 110k 723 / 554, 200k 991 / 846; 6-D 2^22, leaf 32, k = 8: 110k
+// 2388 / 2297, 200k 3707 / 4013, k = 32: 200k 9834 / 6233.
 bool use_knn_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
   if (!sorted || k > 128 || !t->screen_ok || t->depth >= kLaneStack - 1 || knn_variant() != 0 ||
       g_stats_on)
     return false;
-  if (t->d <= 4) {
-    if (k <= 8) return nq <= 180000;
-    if (k <= 16) return nq <= (tree_uneven(t) ? 180000 : 90000);
-    return k >= 64 || nq <= (k <= 32 ? 300000 : 500000);
-  }
-  return k >= 48 || nq <= 32768 + 20000 * (int64_t)k;
+  if (k > kSmemK || (k == kSmemK && t->d > 2) || (k >= 48 && t->d > 4)) return true;
+  // thousands of queries at 2^18 points and leaf 16, the exponents of the points (between
+  // 2^13 and 2^22) and of 16 / leaf, and the factor for uneven trees
+  struct Line {
+    double base, size, leaf, uneven;
+  };
+  Line l;
+  if (t->d <= 2)
+    l = k == 1    ? Line{250, 0.2, 0, 0.8}
+        : k <= 8  ? Line{150, 0.23, 0, 1.1}
+        : k <= 16 ? Line{94, 0.2, 0, 1.6}
+        : k <= 32 ? Line{90, 0.3, 0, 1.6}
+        : k < 48  ? Line{100, 0.25, 0, 1.2}
+        : k < 56  ? Line{250, 0.4, 0, 1}
+                  : Line{600, 0.3, 0, 1};
+  else if (t->d <= 4)
+    l = k == 1    ? Line{220, 0.1, 0.15, 0.36}
+        : k <= 8  ? Line{80, 0.15, 0.42, 1}
+        : k <= 16 ? Line{85, 0.17, 0.45, 1.3}
+        : k <= 32 ? Line{125, 0.19, 0.5, 1.5}
+        : k < 48  ? Line{350, 0.4, 0, 1.2}
+                  : Line{800, 0.36, 0, 0.65};
+  else
+    l = k == 1    ? Line{25, 0.15, 0.2, 2}
+        : k <= 8  ? Line{75, 0.17, 0.3, 1.15}
+        : k <= 16 ? Line{105, 0.24, 0.6, 1.5}
+        : k <= 32 ? Line{165, 0.3, 0.5, 1.8}
+                  : Line{300, 0.14, 0.5, 1.2};
+  const double size = std::min(std::max((double)t->n, 8192.0), 4194304.0);
+  double line = 1000.0 * l.base * std::pow(size / 262144.0, l.size) *
+                std::pow(16.0 / t->leaf, l.leaf) * (tree_uneven(t) ? l.uneven : 1.0);
+  // many equal points, which leave leaves of a point or two: the nearest few of a
+  // query tie and every subtree at distance zero is read (2^18 points in 2^13 places, k = 1:
+  // 90k queries 119 / 203)
+  if (k < 8 && (double)t->n_leaves * t->leaf > 4.0 * (double)t->n) line = std::min(line, 35000.0);
+  return (double)nq <= line;
 }
 
 // Whether the learned-bound search takes a group of lanes per query for its bounded

@@ -168,3 +168,45 @@ def test_gpu_knn_group_far_queries(gpu, oracle, k):
     np.testing.assert_array_equal(d.cpu().numpy(), od)
     assert (oi == -2).all()
     assert tf < 10 * tn
+
+
+@pytest.mark.parametrize("kind,n,d,leaf,nq,k", [
+    ("uniform", 1 << 20, 3, 64, 180000, 8),    # long leaves
+    ("copies", 1 << 18, 3, 16, 180000, 1),     # 32 points in every place
+    ("uniform", 1 << 18, 2, 16, 300000, 24),
+    ("uniform", 30000, 5, 16, 180000, 8),      # a small tree
+    ("clustered", 1 << 16, 2, 16, 150000, 4),
+])
+def test_gpu_knn_choice_is_no_slower_than_a_lane_per_query(gpu, kind, n, d, leaf, nq, k):
+    """Calls that the groups were slower at (1.3 to 2 times a lane per query when they were
+    given these) take no longer than the per-lane kernel, and give its rows."""
+    import time
+    import torch
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    P = torch.rand(n, d, generator=g, device="cuda", dtype=torch.float64)
+    if kind == "copies":
+        P = P[:n // 32].repeat(32, 1)
+    elif kind == "clustered":
+        P = P[:64][torch.arange(n, device="cuda") % 64] + \
+            10 ** (-1 - 4 * P[:, :1]) * torch.randn(n, d, generator=g, device="cuda",
+                                                    dtype=torch.float64)
+    Q = P[torch.arange(nq, device="cuda") * 7919 % n].contiguous()
+    t = gpu.kdtree.build_kdtree(P, leaf=leaf)
+    best, rows = {0: np.inf, 8: np.inf}, {}
+    try:
+        for i in range(12):
+            for v in best:
+                _lib.check(L.ckd_set_knn_variant(v))
+                torch.cuda.synchronize()
+                t0 = time.perf_counter()
+                rows[v] = gpu.kdtree.knn_search_batch(t, Q, k)
+                torch.cuda.synchronize()
+                if i > 1:
+                    best[v] = min(best[v], time.perf_counter() - t0)
+    finally:
+        _lib.check(L.ckd_set_knn_variant(0))
+    assert torch.equal(rows[0][0], rows[8][0]) and torch.equal(rows[0][1], rows[8][1])
+    assert best[0] < 1.15 * best[8]
