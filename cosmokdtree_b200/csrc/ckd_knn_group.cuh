@@ -130,7 +130,10 @@ struct GroupBound {
 
 // BOUND: every list starts full of sentinels (r2, INT32_MAX) instead of HUGE, so
 // pruning starts at once, at the lowest ancestor of the query's leaf whose cell strictly
-// contains the ball; every point with d2 <= r2 is still accepted, so a list that ends
+// contains the ball, from where the same descent gives the nearest range first (a loose
+// bound alone, as in voids, prunes little until k are found: 500k queries of 2^22 points
+// of one cluster, half of them outside it, k = 64: 39.4 -> 30.9 ms, of 2^22 clustered points
+// 5.8 -> 5.2, 6-D 10 % less); every point with d2 <= r2 is still accepted, so a list that ends
 // without a sentinel among its first k is exact.  The others are listed for a rerun and
 // their rows are not written.
 template <int D, bool PER, int G, int R, bool BOUND = false>
@@ -302,10 +305,7 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
         if (inside) break;
         a = load_meta(tv.meta, a).parent;
       }
-      // the subtree waits on the stack, its box untested
-      if (gl == 0) stk[0] = make_uint2((unsigned)(a < 0 ? next : a), kUntested);
-      top = 1;
-      next = -1;
+      if (a >= 0) next = a;  // the descent starts there
     }
   }
   __syncwarp();
@@ -320,7 +320,8 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
     __syncwarp();
     int32_t c0 = -1, c1 = -1, st0 = 0, ct0 = 0, st1 = 0, ct1 = 0;
     float l0 = 0.0f, l1 = 0.0f;
-    if (next >= 0) {
+    const bool seeded = next >= 0;
+    if (seeded) {
       // fewer than k found yet: descent from the nearest waiting subtree (at first
       // the root) along the query's side of the splits to a range
       NodeMeta m = load_meta(tv.meta, next);
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
     // Scan the listed ranges, flattened over the query's lanes, when enough wait,
     // while fewer than k are known, and at the end; what then waits for a merge is
     // merged too in the last two cases.
-    const bool force = bd == CKD_HUGE || top == 0;
+    const bool force = seeded || bd == CKD_HUGE || top == 0;
     const bool run = force || nu >= S::kRun;
     if (!__any_sync(FULL, run && (nu > 0 || nb > 0))) continue;
     const int nus = run ? nu : 0;

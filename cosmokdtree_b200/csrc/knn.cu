@@ -412,12 +412,17 @@ bool use_knn_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
 // Whether the learned-bound search takes a group of lanes per query for its bounded
 // pass (us a call with ordering, network and reruns, per-lane / groups, 2^22 clustered
 // points): k = 8: 20k queries 475 / 376, 50k 543 / 541, 100k 560 / 790; k = 32: 50k
-// 972 / 710, 100k 1092 / 1090, 300k 2133 / 2559; k = 64: 100k 2484 / 1492, 3M 37532 /
-// 33563; 6-D: k = 8: 100k 2280 / 2102, k = 32: 300k 8838 / 8180.
+// 972 / 710, 100k 1092 / 1090, 300k 2133 / 2559; 6-D: k = 8: 100k 2280 / 2102, k = 32: 300k
+// 8838 / 8180.  For 33 <= k <= 64 the lists have room for 64, so the line rises with k (k = 33:
+// 300k 3321 / 2699, 500k 4175 / 4253; k = 40: 500k 5223 / 4490, 1M 7920 / 8532; k = 48: 1M
+// 10150 / 8989; k = 64: 1M 15242 / 9886).  Targets in the void about a single cluster cross
+// earlier (k = 33: 200k 8748 / 10296; k = 64: 300k 15620 / 18857), which the lines below
+// k = 56 make room for.
 bool use_bound_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
   if (!sorted || learned_kernel() != 3 || knn_variant() != 0 || g_stats_on) return false;
-  if (t->d <= 4) return k > 32 || nq <= 30000 + 2200 * (int64_t)k;
-  return k >= 48 || nq <= 32768 + 10000 * (int64_t)k;
+  if (t->d > 4) return k >= 48 || nq <= 32768 + 10000 * (int64_t)k;
+  if (k <= 32) return nq <= 30000 + 2200 * (int64_t)k;
+  return k >= 56 || nq <= (k <= 36 ? 150000 : k <= 44 ? 250000 : 450000);
 }
 
 // Kernel choice (ckd_set_knn_variant): 0 automatic, 1 FP64 packet traversal,

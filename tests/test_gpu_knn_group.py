@@ -210,3 +210,40 @@ def test_gpu_knn_choice_is_no_slower_than_a_lane_per_query(gpu, kind, n, d, leaf
         _lib.check(L.ckd_set_knn_variant(0))
     assert torch.equal(rows[0][0], rows[8][0]) and torch.equal(rows[0][1], rows[8][1])
     assert best[0] < 1.15 * best[8]
+
+
+@pytest.mark.parametrize("k,nq", [(33, 400000), (40, 500000), (48, 1000000)])
+def test_gpu_learned_choice_is_no_slower_than_a_lane_per_query(gpu, k, nq):
+    """Large learned batches about one cluster, where groups took twice as long as a lane per
+    query for their bounded pass: no slower than that, the same rows."""
+    import time
+    import torch
+    from cosmokdtree_b200 import _lib
+    from cosmokdtree_b200.learned import LearnedBound
+    L = _lib.load()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    n = 1 << 18
+    x = torch.randn(n, 3, generator=g, device="cuda", dtype=torch.float64)
+    P = x / x.norm(dim=1, keepdim=True) * 0.25 * \
+        torch.rand(n, 1, generator=g, device="cuda", dtype=torch.float64) ** 2
+    Q = torch.rand(nq, 3, generator=g, device="cuda", dtype=torch.float64) - 0.5
+    Q[::2] = P[torch.arange((nq + 1) // 2, device="cuda") * 7919 % n]
+    t = gpu.kdtree.build_kdtree(P, boxsize=1.0)
+    net = LearnedBound(seed=1)
+    net.fit(t, Q[:8000].contiguous(), k, epochs=4, batch=1024)
+    best, rows = {3: np.inf, 0: np.inf}, {}
+    try:
+        for i in range(8):
+            for v in best:
+                _lib.check(L.ckd_set_tuning(4, v))
+                torch.cuda.synchronize()
+                t0 = time.perf_counter()
+                rows[v] = net.knn(t, Q, k)
+                torch.cuda.synchronize()
+                if i > 1:
+                    best[v] = min(best[v], time.perf_counter() - t0)
+    finally:
+        _lib.check(L.ckd_set_tuning(4, 3))
+    assert torch.equal(rows[0][0], rows[3][0]) and torch.equal(rows[0][1], rows[3][1])
+    assert best[3] < 1.2 * best[0]
