@@ -1481,12 +1481,35 @@ ckd_status sort_rows(const int64_t* offsets, int64_t nq, int64_t* idx, double* d
 // clustered points, 950 results each, count with / without handing over: 2^20
 // queries 8.3 / 12.4 ms, 2^22 queries 27.4 / 23.4 ms); on an even tree it shares
 // enough to go on (10^6 queries on 2^20 uniform points, 2700 results each: 13.3
-// against 16.5 ms).  The fill gives it
-// rows of fewer than kPacketRow results only (3 x 10^5 rows of 287 results: 13.4 ms
-// as packets, 2.2 as warps; of 30 results: 1.09 and 1.05).
-constexpr int64_t kBallWarpMax = 200000;
+// against 16.5 ms).  Even trees that the caches hold change over earlier (10^4 uniform
+// points, 20 results each, packets / warps, us: 90k queries 504 / 481, 199k 597 / 730).
+// The fill gives the packets rows of fewer than 64 results only (3 x 10^5 rows of 287:
+// 13.4 ms as packets, 2.2 as warps; of 30: 1.09 and 1.05), on even trees with rows of up
+// to kPacketMean on average those of fewer than kHeavyRow: 32 neighbours' balls share most
+// of their nodes there, and packets thinned out by the longer of like rows lose by it (3 x
+// 10^5 queries of 2^20 uniform points, count and fill, the line at 256 / at 64, ms: 60
+// results 2.40 / 3.35, 80 2.64 / 4.02, 130 3.31 / 4.30, 160 3.83 / 4.20, 200 5.02 / 4.61).
 constexpr int kPacketBudget = 512;
-constexpr int64_t kPacketRow = 64;
+constexpr double kPacketMean = 150.0;
+// results a ball holds on average where the points fill their extent evenly; infinite on
+// an uneven tree or where the extent is not known
+double even_hits(const ckd_tree* t, double r) {
+  constexpr double kBall[9] = {1.0, 2.0, 3.14159, 4.18879, 4.93480, 5.26379, 5.16771, 4.72477, 4.05871};
+  if (tree_uneven(t)) return INFINITY;
+  double hits = (double)t->n * kBall[t->d];
+  for (int j = 0; j < t->d; ++j) {
+    if (!(t->extent[j] > 0.0)) return INFINITY;  // unknown or flat
+    hits *= r / t->extent[j];
+  }
+  return hits;
+}
+int64_t ball_warp_max(const ckd_tree* t, double r) {
+  return t->n < 32768 && even_hits(t, r) < kPacketMean ? 100000 : 200000;
+}
+int64_t packet_row(const ckd_tree* t, int64_t nq, double r, int64_t total) {
+  const double mean = total >= 0 && !tree_uneven(t) ? (double)total / (double)nq : even_hits(t, r);
+  return mean < kPacketMean ? kHeavyRow : 64;
+}
 bool ball_warp_ok(const ckd_tree* t) { return t->screen_ok && t->depth < kBallReserve - 3; }
 
 // Whether a ball search takes eight lanes per query: small balls (the count of a
@@ -1496,14 +1519,7 @@ bool ball_warp_ok(const ckd_tree* t) { return t->screen_ok && t->depth < kBallRe
 // 251, 100000 724 / 573 (2^22 points: 304 / 368 and 839 / 806); 290 results and more, and
 // clustered points at any size: the warp.
 bool range_narrow(const ckd_tree* t, int64_t nq, double r) {
-  if (nq < 12000 || tree_uneven(t)) return false;
-  constexpr double kBall[9] = {1.0, 2.0, 3.14159, 4.18879, 4.93480, 5.26379, 5.16771, 4.72477, 4.05871};
-  double hits = (double)t->n * kBall[t->d];
-  for (int j = 0; j < t->d; ++j) {
-    if (!(t->extent[j] > 0.0)) return false;  // unknown or flat
-    hits *= r / t->extent[j];
-  }
-  return hits <= (nq >= 100000 ? 64.0 : 16.0);
+  return nq >= 12000 && even_hits(t, r) <= (nq >= 100000 ? 64.0 : 16.0);
 }
 
 // Whether a fill cuts its long rows: batches with fewer rows than the GPU's resident
@@ -1531,7 +1547,7 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
   // rows of the warp kernel (null: all, in processing order), and the packet
   // kernel's rows before it for large batches and for trees that the warp kernel
   // does not take
-  const bool warp = ball_warp_ok(t), packet = !warp || nq > kBallWarpMax;
+  const bool warp = ball_warp_ok(t), packet = !warp || nq > ball_warp_max(t, r);
   // a packet stack holds at most one pending sibling per level, plus the roots
   int stack_len = std::max(kStack, t->depth + 4 + (qroot ? 32 : 0));
   Scratch sc(s);
@@ -1561,7 +1577,7 @@ ckd_status ball_launch(const ckd_tree* t, const double* q, const int32_t* order,
     if (fill) {
       CKD_CUDA(sc.alloc(&light, sizeof(int32_t) * nq));
       k_split_rows<<<(unsigned)cdiv(nq, 256), 256, 0, s>>>(
-          offsets, order, nq, warp ? kPacketRow : kHeavyRow, heavy, cnt, light, cnt + 1);
+          offsets, order, nq, warp ? packet_row(t, nq, r, total) : kHeavyRow, heavy, cnt, light, cnt + 1);
       CKD_LAUNCH_CHECK();
     }
     int32_t* bail = warp && tree_uneven(t) && nq * 2 <= t->n ? heavy : nullptr;
@@ -1695,8 +1711,8 @@ ckd_status query_order_roots(const ckd_tree* t, const double* q, int64_t nq, int
 // through the caches, where density is uneven and rows are long (10^5 queries on 2^22 clustered points, 218 results
 // each: count + fill 1473 ordered, 1920 us in the caller's order; on 2^20 uniform
 // points 611 against 533, the ordering included).
-bool want_ball_order(const ckd_tree* t, int64_t nq) {
-  if (query_order_mode() != 0 || nq > kBallWarpMax || !ball_warp_ok(t)) return want_order(t, nq);
+bool want_ball_order(const ckd_tree* t, int64_t nq, double r) {
+  if (query_order_mode() != 0 || nq > ball_warp_max(t, r) || !ball_warp_ok(t)) return want_order(t, nq);
   return nq >= 50000 && tree_uneven(t) && want_order(t, nq);
 }
 
@@ -1705,7 +1721,7 @@ ckd_status ball_run(const ckd_tree* t, const double* q, int64_t nq, double r, bo
                     cudaStream_t s, const int32_t* qroot, int64_t total) {
   int32_t* order = nullptr;
   Scratch sc(s);
-  if (want_ball_order(t, nq)) {
+  if (want_ball_order(t, nq, r)) {
     CKD_CUDA(sc.alloc(&order, sizeof(int32_t) * nq));
     CKD_TRY(query_order_roots(t, q, nq, order, qroot, s));
   }

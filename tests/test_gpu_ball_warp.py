@@ -185,3 +185,54 @@ def test_gpu_ball_kernels_of_a_loaded_tree(gpu, tmp_path, periodic):
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
     assert na == nb
+
+
+@pytest.mark.parametrize("n,nq,hits", [
+    (1 << 18, 200001, 130), (1 << 18, 200001, 220), (10000, 100001, 20), (10000, 100001, 200)])
+def test_gpu_ball_rows_on_both_sides_of_the_packets_line(gpu, n, nq, hits):
+    """Even trees: short and long rows in one batch, on both sides of the mean that decides, and
+    the line of small trees, against the same queries in small batches."""
+    rng = np.random.default_rng(89)
+    P = rng.random((n, 3))
+    t = gpu.kdtree.build_kdtree(P)
+    Q = P[rng.integers(0, n, nq)]
+    r = float((hits / (n * 4.18879)) ** (1 / 3))
+    ids = rng.integers(0, nq, 3000)
+    sampled_rows_match(lambda q: gpu.kdtree.ball_search_csr(t, q, r), Q, Q[ids], ids, nq)
+
+
+def test_gpu_ball_packets_fill_the_short_rows_of_even_trees(gpu):
+    """3 x 10^5 rows of some 80 results on an even tree: the fill takes at most twice as long as
+    the count (1.4 times with packets; a warp a row took 2.7 times)."""
+    import ctypes
+    import torch
+    from cosmokdtree_b200 import _lib
+    L = _lib.load()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    n, nq = 1 << 20, 300000
+    P = torch.rand(n, 3, generator=g, device="cuda", dtype=torch.float64)
+    Q = P[torch.arange(nq, device="cuda") * 7919 % n].contiguous()
+    r = float((80 / (n * 4.18879)) ** (1 / 3))
+    t = gpu.kdtree.build_kdtree(P)
+    off, idx, dist = gpu.kdtree.ball_search_csr(t, Q, r)
+    counts = torch.empty(nq, dtype=torch.int64, device="cuda")
+    ptr = lambda x: ctypes.c_void_p(x.data_ptr())
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def clock(f):
+        best = np.inf
+        for _ in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            _lib.check(f())
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    tc = clock(lambda: L.ckd_ball_count(t.handle, ptr(Q), nq, r, ptr(counts), s))
+    tf = clock(lambda: L.ckd_ball_fill_sized(t.handle, ptr(Q), nq, r, 0, int(off[-1]), ptr(off),
+                                             ptr(idx), ptr(dist), s))
+    print("count %.3f fill %.3f ms" % (tc, tf))
+    assert tf < 2.0 * tc
