@@ -42,7 +42,6 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned kUntested = 0xffffffffu;  // stack entry whose box has not been tested
-constexpr float kFarQuery = 1e25f;
 constexpr int32_t kUnit = 16;     // subtrees of at most this many points are scanned as a range
 
 // (d, id) lexicographic order
@@ -173,9 +172,7 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
 #pragma unroll
   for (int j = 0; j < D; ++j) {
     q[j] = valid ? Q[qi * D + j] : 0.0;
-    // clamped so that its gaps stay numbers: a query out there is further than HUGE from
-    // every point (coordinates are below 1e18 here); NaN, which no point is near, likewise
-    qs.q32[j] = fminf(fmaxf(__double2float_rn(q[j]), -kFarQuery), kFarQuery);
+    qs.q32[j] = __double2float_rn(q[j]);
     qs.dlt[j] = kTwoM21 * (fabsf(qs.q32[j]) + tv.slack[j]) * 1.0001f;
     xl[j] = __fadd_ru(qs.q32[j], qs.dlt[j]);
     xh[j] = __fsub_rd(qs.q32[j], qs.dlt[j]);
@@ -280,7 +277,20 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
   int nu = 0;  // ranges waiting to be scanned
   int top = 0;
   int32_t next = valid ? (qroot ? qroot[qi] : 0) : -1;  // next seed descent's subtree, -1: none
+  // A query further than HUGE from every point, or not finite, finds nothing: by the largest
+  // coordinate of each axis, or it would read the whole tree (64 such of 2^20 points, k = 100:
+  // 16 ms).
+  {
+    float far = 0.0f;
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      const float a = fabsf(qs.q32[j]), g = 0.5f * fmaxf(a - tv.slack[j], 0.0f);
+      far = a <= FLT_MAX ? fmaf(g, g, far) : CUDART_INF_F;
+    }
+    if (!(far * kShrink <= 0.25f * FLT_MAX)) next = -1;
+  }
   if (BOUND && valid) {
+    const bool near = next >= 0;
     const double b = gb.r2[qi];
     if (b < CKD_HUGE) {
 #pragma unroll
@@ -305,18 +315,13 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
         if (inside) break;
         a = load_meta(tv.meta, a).parent;
       }
-      if (a >= 0) next = a;  // the descent starts there
+      if (a >= 0 && near) next = a;  // the descent starts there
     }
   }
   __syncwarp();
   while (__any_sync(FULL, next >= 0 || top > 0)) {
     const bool act = next >= 0 || top > 0;
-    if (next < 0 && top > 0 && bd == CKD_HUGE) {
-      // dropped when all of it is further than HUGE: a query far from every point would
-      // read the whole tree (64 such of 2^20 points, k = 100: 16 ms)
-      next = (int32_t)stk[--top].x;
-      if (!(node_lb(next) <= wd32)) next = -1;
-    }
+    if (next < 0 && top > 0 && bd == CKD_HUGE) next = (int32_t)stk[--top].x;
     __syncwarp();
     int32_t c0 = -1, c1 = -1, st0 = 0, ct0 = 0, st1 = 0, ct1 = 0;
     float l0 = 0.0f, l1 = 0.0f;
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
         st0 = m.start;
         ct0 = m.count;
       }
-    } else if (act && bd < CKD_HUGE) {
+    } else if (act) {
       // up to G waiting subtrees at once, a lane each
       const int n = min(min(top, G), max(1, depth + 2 * G - top));
       int32_t c = -1;
