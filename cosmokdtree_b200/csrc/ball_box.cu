@@ -699,8 +699,9 @@ __device__ __forceinline__ void expand(const QT& qt, int32_t node, int32_t unit,
 // results each: 0.39 -> 0.26 and 0.44 -> 0.28 ms.  Now bound by issue: about 3000
 // warp instructions a query of the latter.  A lane per query (tried for small
 // balls, 100k queries) was no faster, waiting on its dependent loads.
-constexpr int kBallStack = 320;
+constexpr int kBallStack = 384;
 constexpr int kBallReserve = 130;  // room for one-at-a-time descents (tree depth < 127)
+constexpr int kBallWide = 190;     // entries up to which several are expanded at once
 constexpr int kBallList = 128;
 constexpr int kBallListRun = 16;   // ranges that wait before they are scanned (count)
 constexpr int32_t kBallUnit = 32;  // subtrees of at most this many points are scanned as a range
@@ -723,10 +724,12 @@ struct Part {
   int32_t count;   // its results
   int32_t pad;
 };
-constexpr int kPartMin = 96;      // entries that a row is refined to, at least, where it can be
-// a level at most doubles the entries, and a row that finds no room for its parts is
-// walked on from what it was refined to: one-at-a-time descents still have their room
-static_assert(2 * (kPartMin - 1) <= kBallStack - kBallReserve, "refined rows and the stack");
+constexpr int kPartMin = 128;     // entries that a row is refined to, at least, where it can be
+// A level at most doubles the entries, and a row that finds no room for its parts is
+// walked on from what it was refined to: one-at-a-time descents still have their room.
+// (96 entries and a stack of 320: 4001 clustered balls 1249 -> 1293 us a call.)
+static_assert(kBallWide + kBallReserve <= kBallStack &&
+              2 * (kPartMin - 1) + kBallReserve <= kBallStack, "walks and refined rows fit");
 constexpr int kPartBudget = 64;   // steps (32 lanes' work each) before a row is cut
 struct Parts {
   Part* list;       // null: rows are not cut
@@ -845,7 +848,7 @@ __global__ void __launch_bounds__(128) k_range_warp(
         work = 0;
         if (cut_row(bq, parts, qi, cur, stk, s_stk[w][stk == s_stk[w][0] ? 1 : 0], top)) break;
       }
-      const int n = min(min(top, 32), max(1, kBallStack - kBallReserve - top));
+      const int n = min(min(top, 32), max(1, kBallWide - top));
       int2 e = make_int2(0, kNone);
       if (lane < n) e = stk[top - 1 - lane];
       __syncwarp();
