@@ -389,7 +389,7 @@ bool use_knn_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
   else if (t->d <= 4)
     l = k == 1    ? Line{220, 0.1, 0.15, 0.36}
         : k <= 8  ? Line{80, 0.15, 0.42, 1}
-        : k <= 16 ? Line{85, 0.17, 0.45, 1.3}
+        : k <= 16 ? Line{75, 0.17, 0.45, 1.45}
         : k <= 32 ? Line{125, 0.19, 0.5, 1.5}
         : k < 48  ? Line{350, 0.4, 0, 1.2}
                   : Line{800, 0.36, 0, 0.65};
