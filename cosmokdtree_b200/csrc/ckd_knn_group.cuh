@@ -273,24 +273,25 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
       wf = inside;
     }
   };
+  // Whether the query is further than HUGE from every point, by the largest coordinate of
+  // each axis, or not finite: it finds nothing, and would read the whole tree for it (64
+  // such of 2^20 points, k = 100: 16 ms).  Asked for only when the first range has
+  // left fewer than k, off the path that every query takes, of values that the walk holds.
+  // Not on periodic trees, whose queries lie in the box.
+  auto beyond = [&]() -> bool {
+    float s2 = 0.0f;
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      const float b = tv.slack[j], g = 0.5f * fmaxf(fmaxf(-b - xl[j], xh[j] - b), 0.0f);
+      s2 = xl[j] - xh[j] <= FLT_MAX ? fmaf(g, g, s2) : CUDART_INF_F;
+    }
+    return !(s2 * kShrink <= 0.25f * FLT_MAX);
+  };
   const int32_t seed = max(2 * G, 4 * k);
   int nu = 0;  // ranges waiting to be scanned
   int top = 0;
   int32_t next = valid ? (qroot ? qroot[qi] : 0) : -1;  // next seed descent's subtree, -1: none
-  // A query further than HUGE from every point, or not finite, finds nothing: by the largest
-  // coordinate of each axis, or it would read the whole tree (64 such of 2^20 points, k = 100:
-  // 16 ms).
-  {
-    float far = 0.0f;
-#pragma unroll
-    for (int j = 0; j < D; ++j) {
-      const float a = fabsf(qs.q32[j]), g = 0.5f * fmaxf(a - tv.slack[j], 0.0f);
-      far = a <= FLT_MAX ? fmaf(g, g, far) : CUDART_INF_F;
-    }
-    if (!(far * kShrink <= 0.25f * FLT_MAX)) next = -1;
-  }
   if (BOUND && valid) {
-    const bool near = next >= 0;
     const double b = gb.r2[qi];
     if (b < CKD_HUGE) {
 #pragma unroll
@@ -315,13 +316,19 @@ __global__ void __launch_bounds__(128) k_knn_group(TreeView tv, const double* __
         if (inside) break;
         a = load_meta(tv.meta, a).parent;
       }
-      if (a >= 0 && near) next = a;  // the descent starts there
+      if (a >= 0) next = a;  // the descent starts there
     }
   }
   __syncwarp();
   while (__any_sync(FULL, next >= 0 || top > 0)) {
     const bool act = next >= 0 || top > 0;
-    if (next < 0 && top > 0 && bd == CKD_HUGE) next = (int32_t)stk[--top].x;
+    if (next < 0 && top > 0 && bd == CKD_HUGE) {
+      next = (int32_t)stk[--top].x;
+      if (!PER && beyond()) {
+        next = -1;
+        top = 0;
+      }
+    }
     __syncwarp();
     int32_t c0 = -1, c1 = -1, st0 = 0, ct0 = 0, st1 = 0, ct1 = 0;
     float l0 = 0.0f, l1 = 0.0f;

@@ -371,7 +371,7 @@ bool use_knn_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
   if (!sorted || k > 128 || !t->screen_ok || t->depth >= kLaneStack - 1 || knn_variant() != 0 ||
       g_stats_on)
     return false;
-  if (k > kSmemK || (k == kSmemK && t->d > 2) || (k >= 48 && t->d > 4)) return true;
+  if (nq <= 4000 || k > kSmemK || (k == kSmemK && t->d > 2) || (k >= 48 && t->d > 4)) return true;
   // thousands of queries at 2^18 points and leaf 16, the exponents of the points (between
   // 2^13 and 2^22) and of 16 / leaf, and the factor for uneven trees
   struct Line {
