@@ -632,34 +632,38 @@ def workload_config(name, world=1):
             "l2": "inputs larger than L2 (tree ~0.6 GB, outputs 8.6 GB per step)"}
 
 
-# DRAM bytes per working point and level of the build's three large kernels (k_seg_box,
-# k_flags, k_scatter), from one ncu capture of each at a mid-depth level of the 16.7M-point
-# clustered build (322.5 + 143.1 + 673.0 MB over ~11.3M working points)
-BUILD_DRAM_BYTES_PER_POINT_LEVEL = 100.8
-BUILD_TRAFFIC_NOTE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_seg_box, k_flags "
-                      "and k_scatter at one mid-depth level, per working point, scaled by the "
-                      "tree's point-levels (the per-level box, flag and scatter passes each "
-                      "read the working set)")
+# DRAM bytes (read + write) of a whole build's kernels per algorithmic byte (build_roofline),
+# from one ncu capture of every launch of the 16.7M-point clustered build
+BUILD_DRAM_PER_ALG_BYTE = 36.39e9 / 21.59e9
+BUILD_TRAFFIC_NOTE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum over all launches of the "
+                      "16.7M-point clustered build, per algorithmic byte")
+
+
+def finish_points(d):
+    """Nodes of at most this many points are built in shared memory by one block."""
+    return 2048 if d <= 3 else 1024
 
 
 def build_roofline(tree, n, d, ms):
-    """Build roofline from the algorithmic bytes of a level-synchronous build: the
-    input read once (N·D·8), every point read and written once per level above its
-    leaf (Σ_p depth(p)·2·(D·8 + 4)), and the leaf-ordered write (N·(D·8 + 4))."""
+    """Build roofline from the bytes that the build cannot do without as it is laid out: the
+    input read (N·D·8) and written as rows with ids (N·(D·8 + 4)); every point read and
+    written once per level of a node that is too large to be finished in shared memory, and
+    once more by the block that finishes its subtree (2·(D·8 + 4) each time)."""
     ex = tree.export()
-    left, right, count, axis = ex["left"], ex["right"], ex["count"], ex["axis"]
-    depth = np.zeros(len(left), dtype=np.int64)
-    internal = np.nonzero(left >= 0)[0]
-    for _ in range(int(tree.depth) + 1):  # preorder parents precede children
-        depth[left[internal]] = depth[internal] + 1
-        depth[right[internal]] = depth[internal] + 1
-    leaves = axis < 0
-    point_levels = int((depth[leaves] * count[leaves]).sum())
+    left, count = ex["left"], ex["count"]
+    inner = left >= 0
+    small = finish_points(d)
+    point_levels = int(count[inner & (count > small)].sum())
+    # subtrees finished: their roots are small and have no small parent
+    parent_small = np.zeros(len(left), dtype=bool)
+    for side in ("left", "right"):
+        parent_small[ex[side][inner]] = count[inner] <= small
+    finished = int(count[inner & (count <= small) & ~parent_small].sum())
     rec = d * 8 + 4
-    alg = n * d * 8 + point_levels * 2 * rec + n * rec
+    alg = n * d * 8 + n * rec + (point_levels + finished) * 2 * rec
     peak, kind = measured_peaks()
     a = alg / (ms / 1e3) / 1e9
-    traffic = BUILD_DRAM_BYTES_PER_POINT_LEVEL * point_levels if d == 3 else None
+    traffic = BUILD_DRAM_PER_ALG_BYTE * alg if d == 3 else None
     return {"bound": "hbm", "achieved": a, "peak": peak, "unit": "GB/s", "frac": a / peak,
             "traffic": traffic, "traffic_note": BUILD_TRAFFIC_NOTE if traffic else None,
             "alg_bytes": alg, "point_levels_per_point": point_levels / n,

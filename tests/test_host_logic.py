@@ -35,3 +35,25 @@ def test_wrap_pieces_inside_box_unchanged():
     assert _wrap_pieces(-0.2, 0.3, 1.0) == [(-0.2, 0.3)]
     assert _wrap_pieces(0.4, 0.7, 1.0)[0][0] == 0.4
     assert _wrap_pieces(-3.0, 5.0, 1.0) == [(-0.5, 0.5)]
+
+
+def test_build_roofline_counts_only_passes_over_memory(oracle):
+    """Points of subtrees that are finished in shared memory are read and written once for all
+    of their levels, not once a level."""
+    import bench
+    rng = np.random.default_rng(97)
+    for d, n, leaf in ((3, 30000, 16), (4, 5000, 8), (3, 1500, 16), (3, 9000, 3000)):
+        t = oracle.OracleTree(rng.random((n, d)) ** 3, leaf, None)
+        ex = t.export()
+        small = bench.finish_points(d)
+
+        def passes(a):  # point passes over memory of the subtree of a node
+            if ex["left"][a] < 0:
+                return 0
+            if ex["count"][a] <= small:
+                return int(ex["count"][a])
+            return int(ex["count"][a]) + passes(ex["left"][a]) + passes(ex["right"][a])
+
+        rec = d * 8 + 4
+        r = bench.build_roofline(t, n, d, 1.0)
+        assert r["alg_bytes"] == n * d * 8 + n * rec + passes(0) * 2 * rec
