@@ -19,11 +19,12 @@
 //
 // Bound by instruction issue (70-76 % of slots at G = 8 and 16) and, for small batches,
 // by dependent loads.  Measured (us a call, before -> now): one query of 2^20 points,
-// k = 16: 54 -> 24 (a lane before); 30k queries of 10^6 clustered points, k = 100:
-// 9470 -> 640 (heaps in the output rows before); 200k queries of 2^22 6-D points, k = 64:
-// 16060 -> 6400; 100k queries of 2^22 clustered points, k = 32: 1199 -> 847.  The whole
-// warp for each of the last ones takes 947: fewer lanes a query waste less on short
-// ranges and few pending nodes, at the price of waiting for three neighbours.
+// k = 16: 54 -> 16 (a lane before; part of it the shorter way through the host); 30k queries
+// of 10^6 clustered points, k = 100: 9470 -> 549 (heaps in the output rows before); 200k
+// queries of 2^22 6-D points, k = 64: 16060 -> 6370; 100k queries of 2^22 clustered points,
+// k = 32: 1199 -> 847.  The whole warp for each of the last ones takes 947: fewer lanes a
+// query waste less on short ranges and few pending nodes, at the price of waiting for
+// three neighbours.
 // Dropped: following single children inside a lane (10 to 30 % slower), an FP32
 // screen of the points before the FP64 records (no gain).
 //

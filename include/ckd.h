@@ -103,9 +103,9 @@ ckd_status ckd_knn_ordered(const ckd_tree* tree, const double* q_dev, int64_t nq
 int64_t ckd_launch_count(void);
 
 /* Process-wide kNN kernel choice (no reference counterpart): 0 = automatic (sorted
- * rows: 32, 16 or 8 lanes of a warp per query for small and middle batches, for
- * 64 <= k <= 128, and for most k above three dimensions; else 8 when k <= 64; both
- * when the coordinates allow the FP32 screen and the tree is shallow enough; 1
+ * rows: 32, 16 or 8 lanes of a warp per query where that is faster: up to a batch that
+ * rises with the points and falls with the leaf size, always for 64 < k <= 128; else 8
+ * when k <= 64; both when the coordinates allow the FP32 screen and the tree is shallow enough; 1
  * otherwise), 1 = FP64 packet
  * traversal, 7 = per-lane traversal with 8-byte heap entries (FP32 key +
  * position, exact tie resolution), 8 = 7 expanding nodes from child-pair records.
@@ -117,8 +117,8 @@ ckd_status ckd_set_knn_variant(int variant);
  * key 1: cap on resident blocks per SM for the per-lane kNN kernel (0 = as many
  * as fit); key 2: warps per block of the per-lane kNN kernel (1..8, default 2,
  * at most 4 used); key 4: search kernel of ckd_knn_learned (0 = bounded per-lane
- * traversal; 3 = 0 with child-pair-record descent, and groups of lanes per query for
- * small batches and k > 32, default); key 6: ordering of queries by leaf before kNN and
+ * traversal; 3 = 0 with child-pair-record descent, and groups of lanes per query up to
+ * batches that rise with k, default); key 6: ordering of queries by leaf before kNN and
  * ball searches (0 = automatic, default; 1 = always; 2 = never); key 7: inference of
  * the learned-bound network (0 = FP32 FMAs; 1 = tensor cores, tcgen05 MMAs on
  * BF16 activations, default); key 8: box search of up to 32768 boxes per call
