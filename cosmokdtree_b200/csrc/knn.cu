@@ -379,13 +379,14 @@ bool use_knn_group(const ckd_tree* t, int64_t nq, int k, int sorted) {
   };
   Line l;
   if (t->d <= 2)
-    l = k == 1    ? Line{250, 0.2, 0, 0.8}
-        : k <= 8  ? Line{150, 0.23, 0, 1.1}
-        : k <= 16 ? Line{94, 0.2, 0, 1.6}
-        : k <= 32 ? Line{90, 0.3, 0, 1.6}
-        : k < 48  ? Line{100, 0.25, 0, 1.2}
-        : k < 56  ? Line{250, 0.4, 0, 1}
-                  : Line{600, 0.3, 0, 1};
+    l = k == 1                ? Line{250, 0.2, 0, 0.8}
+        : k <= 8 && t->d == 1 ? Line{220, 0.2, 0, 1.1}
+        : k <= 8              ? Line{110, 0.25, 0, 1.2}
+        : k <= 16             ? Line{94, 0.2, 0, 1.6}
+        : k <= 32             ? Line{90, 0.3, 0, 1.6}
+        : k < 48              ? Line{90, 0.25, 0, 1.2}
+        : k < 56              ? Line{150, 0.4, 0, 1}
+                              : Line{600, 0.3, 0, 1};
   else if (t->d <= 4)
     l = k == 1    ? Line{220, 0.1, 0.15, 0.36}
         : k <= 8  ? Line{80, 0.15, 0.42, 1}
